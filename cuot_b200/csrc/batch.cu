@@ -12,10 +12,9 @@
 //     of rows of every instance, both roles of a row from one index
 //     computation (the two roles share the public LPN seed).
 //   SOT branch: the persistent PPRF launches over the SOT sender and then
-//     receiver trees; then per transform size, largest first: blocks into the
-//     encode's layout, transform passes that span every instance of that
-//     size (each with its own A_hat), back to blocks, and the receivers'
-//     choice-bit encodes.
+//     receiver trees; then per transform size, largest first: the dual LPNs
+//     of every instance of that size (each with its own A_hat), in passes that
+//     span several instances, and the receivers' choice-bit encodes.
 // cfg.schedule: CUOT_BATCH_SERIAL (default) runs every launch in one chain
 // on the caller's stream, each role's PPRF as one persistent launch over the
 // trees of both branches; CUOT_BATCH_FORK_FERRET runs the Ferret branch on a
@@ -161,10 +160,12 @@ int batch_setup_device() {
 
 struct SotClass {
   int e;
+  int kind = 0;                   // transform (qc_kind when the batch is made)
   int batch = 1;                  // planes per transform pass group of this size
   std::vector<int> items;         // item indices of this size
-  uint8_t *planes = nullptr;      // 2 * items * 16n bytes (jobs: item x role)
+  void *planes = nullptr;         // layout buffer of the jobs (item x role)
   void *Y = nullptr;              // this size's intermediate: qc_y_bytes(batch)
+  std::vector<cuot_block *> io;     // per job: the role's blocks
   std::vector<const void *> ahats;  // per job
 };
 
@@ -338,16 +339,7 @@ int enqueue_lane(cuot_batch *b, const std::vector<int> &lane, cudaStream_t st) {
     SotClass &c = b->classes[ci];
     const uint64_t n = 1ull << c.e;
     const int njobs = int(c.items.size()) * 2;
-    for (int j = 0; j < njobs; j++) {
-      const cuot_batch_item &it = b->items[c.items[j / 2]];
-      CUOT_TRY(qc_job_to_layout(ctx, c.e, j % 2 ? it.w_d : it.v_d, c.planes + uint64_t(j) * n * 16, st));
-    }
-    CUOT_TRY(qc_encode_jobs(ctx, c.e, reinterpret_cast<uint64_t *>(c.planes), njobs, c.ahats.data(), c.Y,
-                            c.batch, st));
-    for (int j = 0; j < njobs; j++) {
-      const cuot_batch_item &it = b->items[c.items[j / 2]];
-      CUOT_TRY(qc_job_from_layout(ctx, c.e, c.planes + uint64_t(j) * n * 16, j % 2 ? it.w_d : it.v_d, st));
-    }
+    CUOT_TRY(qc_encode_jobs(ctx, c.kind, c.e, c.io.data(), njobs, c.ahats.data(), c.planes, c.Y, c.batch, st));
     for (int i : c.items) {
       const cuot_batch_item &it = b->items[i];
       CUOT_TRY(cuot_qc_encode_sparse(ctx, it.a_d, it.punct_d, int(it.t), n, it.cbits_d, st));
@@ -581,14 +573,15 @@ int cuot_batch_create(cuot_ctx *ctx, const cuot_batch_item *items, int count,
   for (size_t ci = 0; ci < b->classes.size(); ci++) {
     SotClass &c = b->classes[ci];
     const uint64_t n = 1ull << c.e;
-    if ((st = qc_prepare(ctx, c.e))) return cleanup(st);
-    if ((st = balloc(b, &c.planes, 2 * c.items.size() * n * 16))) return cleanup(st);
+    c.kind = qc_kind(ctx, c.e);
+    if ((st = qc_prepare(ctx, c.kind, c.e))) return cleanup(st);
+    if ((st = balloc(b, &c.planes, qc_layout_bytes(c.kind, c.e, int(2 * c.items.size()))))) return cleanup(st);
     int pb = b->cfg.qc_planes_per_pass > 0 ? b->cfg.qc_planes_per_pass
                                            : qc_default_batch(n, int(256 * c.items.size()));
     pb = std::min(pb, int(256 * c.items.size()));
     c.batch = pb;
-    if ((st = balloc(b, &c.Y, qc_y_bytes(ctx, c.e, pb)))) return cleanup(st);
-    const int key = qc_lane(ctx, c.e);
+    if ((st = balloc(b, &c.Y, qc_y_bytes(ctx, c.kind, c.e, pb)))) return cleanup(st);
+    const int key = qc_lane(c.kind, c.e);
     auto l = lane_of.find(key);
     if (l == lane_of.end()) {
       lane_of[key] = int(b->lanes.size());
@@ -597,10 +590,11 @@ int cuot_batch_create(cuot_ctx *ctx, const cuot_batch_item *items, int count,
       b->lanes[l->second].push_back(int(ci));
     }
     for (int i : c.items) {
-      if ((st = balloc(b, &b->item_ahat[i], qc_ahat_bytes(ctx, c.e)))) return cleanup(st);
-      if ((st = qc_build_ahat(ctx, c.e, items[i].a_d, c.Y, b->item_ahat[i], nullptr))) return cleanup(st);
-      c.ahats.push_back(b->item_ahat[i]);  // sender job
-      c.ahats.push_back(b->item_ahat[i]);  // receiver job
+      if ((st = balloc(b, &b->item_ahat[i], qc_ahat_bytes(c.kind, c.e)))) return cleanup(st);
+      if ((st = qc_build_ahat(ctx, c.kind, c.e, items[i].a_d, c.Y, b->item_ahat[i], nullptr))) return cleanup(st);
+      c.ahats.insert(c.ahats.end(), 2, b->item_ahat[i]);  // sender and receiver job
+      c.io.push_back(items[i].v_d);
+      c.io.push_back(items[i].w_d);
       if ((st = cuot_qc_plan_create(ctx, items[i].a_d, n, nullptr, &b->plans[i]))) return cleanup(st);
     }
   }

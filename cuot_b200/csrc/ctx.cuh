@@ -42,22 +42,24 @@ void qc_free_ctx_tables(cuot_ctx *ctx);
 // Scratch bytes of the one-shot dual LPN (cuot_sot_dual_lpn, or with r2
 // cuot_sot_dual_lpn_r2) of n = 2^e on ctx (qc.cu).
 uint64_t qc_one_shot_dual_bytes(const cuot_ctx *ctx, int e, bool r2);
-// QC helpers used by the batched engine (qc.cu).  The backend (NTT or FFT)
-// of an n = 2^e encode follows the context's CUOT_TUNE_QC_BACKEND; A_hat
-// and intermediate sizes depend on it.
-int qc_prepare(cuot_ctx *ctx, int e);
-uint64_t qc_ahat_bytes(const cuot_ctx *ctx, int e);
+// QC helpers used by the batched engine (qc.cu).  A size's transform follows
+// the context's tuning when the batch is made (qc_kind); the sizes and calls
+// below take that value, since tuning may change before the batch runs.
+int qc_kind(const cuot_ctx *ctx, int e);
+int qc_prepare(cuot_ctx *ctx, int kind, int e);
+uint64_t qc_ahat_bytes(int kind, int e);
 // Encodes of two sizes with the same lane share per-size FFT state (the
 // tables' second stream, events and plane-parity words) and must not run at
 // the same time; different lanes may.
-int qc_lane(const cuot_ctx *ctx, int e);
-uint64_t qc_y_bytes(const cuot_ctx *ctx, int e, int batch);
-int qc_build_ahat(cuot_ctx *ctx, int e, const uint64_t *a_d, void *Y, void *ahat, cudaStream_t st);
-int qc_encode_jobs(cuot_ctx *ctx, int e, uint64_t *planes, int njobs, const void *const *ahats,
-                   void *Y, int batch, cudaStream_t st);
-// n = 2^e blocks into a job's encode layout (16n bytes) and back.
-int qc_job_to_layout(const cuot_ctx *ctx, int e, const cuot_block *in, void *job, cudaStream_t st);
-int qc_job_from_layout(const cuot_ctx *ctx, int e, const void *job, cuot_block *out, cudaStream_t st);
+int qc_lane(int kind, int e);
+uint64_t qc_y_bytes(const cuot_ctx *ctx, int kind, int e, int batch);
+int qc_build_ahat(cuot_ctx *ctx, int kind, int e, const uint64_t *a_d, void *Y, void *ahat, cudaStream_t st);
+// Bytes of the layout buffer that qc_encode_jobs needs for njobs jobs.
+uint64_t qc_layout_bytes(int kind, int e, int njobs);
+// io[j] <- a_j * io[j] blockwise (n = 2^e blocks each), ahats[j] the A_hat of
+// a_j (host arrays).  layout: qc_layout_bytes; Y: qc_y_bytes(batch).
+int qc_encode_jobs(cuot_ctx *ctx, int kind, int e, cuot_block *const *io, int njobs, const void *const *ahats,
+                   void *layout, void *Y, int batch, cudaStream_t st);
 int qc_default_batch(uint64_t n, int nplanes);
 // FP64 FFT backend of the QC encode (qc_fft.cu): n = 2^e, 10 <= e <= kQcfMaxE.
 constexpr int kQcfMaxE = 22;
@@ -108,6 +110,21 @@ int qck_build_ahat(const QcfTables *leaf, int e, const uint64_t *a_d, void *bits
 // leaf FFT passes' intermediate for `batch` planes.
 int qck_dual_lpn(const QcfTables *leaf, int e, const void *ahat, const cuot_block *in, const cuot_block *xor_in,
                  cuot_block *out, void *scratch, void *Y, int batch, cudaStream_t st);
+// Ternary-transform dual LPN (qc_tern.cu): n = 2^e, kTernMinE <= e <= kTernMaxE.
+struct TernJob {
+  const cuot_block *in, *xor_in;  // n blocks; XORed into the result, or null
+  cuot_block *out;                // may be `in` or `xor_in`
+  const void *ahat;
+};
+bool tern_supported(int e);
+uint64_t tern_ahat_bytes(int e);   // leaf constants of `a`
+uint64_t tern_build_bytes(int e);  // scratch of tern_build_ahat
+uint64_t tern_job_bytes(int e);    // scratch per job of a launch
+int tern_build_ahat(int e, const uint64_t *a_d, void *scratch, void *ahat, cudaStream_t st);
+// Up to kTernMaxJobs dual LPNs of one size side by side; scratch holds
+// tern_job_bytes(e) for each.
+constexpr int kTernMaxJobs = 16;
+int tern_dual(int e, const TernJob *jobs, int njobs, void *scratch, cudaStream_t st);
 int transpose_launch(const void *in, uint64_t rows, uint64_t row_bytes, uint64_t col_lo,
                      uint64_t col_hi, void *out, cudaStream_t st);
 }  // namespace cuot

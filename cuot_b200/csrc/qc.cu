@@ -815,20 +815,26 @@ static int default_batch(uint64_t n, int nplanes) {
 }
 
 // ---- backend selection -------------------------------------------------------
-// Transform of the dual LPN of n = 2^e: the fp64 FFT (qc_fft.cu) up to 2^22,
-// GF(2) Karatsuba over it (qc_kara.cu) for 2^23 and 2^24, the NTT above and
-// whenever the context asks for it.  Plane encodes (cuot_qc_encode and
+// Transform of the dual LPN of n = 2^e: the ternary transform (qc_tern.cu)
+// for 2^16 .. 2^22, the fp64 FFT (qc_fft.cu) for other n up to 2^22 (below
+// 2^16 the ternary transform's six launches cost more: 42 against 35 us at
+// 2^14, 53 against 47 at 2^15, but 61 against 65 at 2^16 and 425 against 727
+// at 2^20) and whenever the context asks for it or records its margin, GF(2)
+// Karatsuba over it (qc_kara.cu) for 2^23 and 2^24, the NTT above and whenever
+// the context asks for it.  Plane encodes (cuot_qc_encode and
 // cuot_qc_plan_encode) take the FFT or the NTT.
-enum QcKind { kQcNtt = 0, kQcFft = 1, kQcKara = 2 };
+enum QcKind { kQcNtt = 0, kQcFft = 1, kQcKara = 2, kQcTern = 3 };
 
 static QcKind dual_kind(const cuot_ctx *ctx, int e) {
   if (ctx->qc_backend == 1) return kQcNtt;
+  if (ctx->qc_backend == 0 && !ctx->qcf_margin && tern_supported(e)) return kQcTern;
   if (qcf_supported(e)) return kQcFft;
   if (qck_supported(e)) return kQcKara;
   return kQcNtt;
 }
 
-static QcKind plane_kind(const cuot_ctx *ctx, int e) { return dual_kind(ctx, e) == kQcFft ? kQcFft : kQcNtt; }
+static bool planes_by_fft(QcKind k) { return k == kQcFft || k == kQcTern; }
+static QcKind plane_kind(const cuot_ctx *ctx, int e) { return planes_by_fft(dual_kind(ctx, e)) ? kQcFft : kQcNtt; }
 
 // Intermediate bytes of a pass over `batch` planes: 4 bytes per plane and
 // coefficient for both transforms (the FFT packs 4 planes in 16 bytes, in
@@ -844,10 +850,15 @@ static int leaf_batch(const cuot_ctx *ctx) {
   return ctx->qc_planes_per_pass > 0 ? ctx->qc_planes_per_pass : default_batch(1ull << kQcfMaxE, 128);
 }
 
-// Bytes of A_hat: NTT n Shoup pairs; FFT n complex doubles; Karatsuba the
-// 3^L leaf transforms, followed (with_planes) by the NTT's for plane encodes.
+// The ternary transform's constants, padded so that an FFT A_hat can follow.
+static uint64_t tern_ahat_span(int e) { return (tern_ahat_bytes(e) + 255) & ~255ull; }
+
+// Bytes of A_hat: NTT n Shoup pairs; FFT n complex doubles; ternary its leaf
+// constants; Karatsuba the 3^L leaf transforms.  With planes the last two are
+// followed by the FFT's / the NTT's A_hat for plane encodes.
 static uint64_t ahat_bytes(QcKind k, int e, bool with_planes) {
   if (k == kQcFft) return qcf_ahat_bytes(e);
+  if (k == kQcTern) return tern_ahat_span(e) + (with_planes ? qcf_ahat_bytes(e) : 0);
   if (k == kQcKara) return qck_ahat_bytes(e) + (with_planes ? 8ull << e : 0);
   return 8ull << e;
 }
@@ -855,6 +866,7 @@ static uint64_t ahat_bytes(QcKind k, int e, bool with_planes) {
 // Scratch of the A_hat build.
 static uint64_t ahat_scratch_bytes(QcKind k, int e) {
   if (k == kQcFft) return 16ull << e;
+  if (k == kQcTern) return tern_build_bytes(e) > (16ull << e) ? tern_build_bytes(e) : 16ull << e;
   if (k == kQcKara) {
     const uint64_t kb = qck_bits_scratch_bytes(e) + (16ull << kQcfMaxE);
     return kb > (4ull << e) ? kb : (4ull << e);
@@ -864,8 +876,9 @@ static uint64_t ahat_scratch_bytes(QcKind k, int e) {
 
 // Scratch of a dual LPN (rate 1, or rate 1/2 with r2): the planes / tile
 // words (and the 2n-bit planes of the rate-1/2 form) or the Karatsuba
-// split blocks, then the pass intermediate.
+// split blocks, then the pass intermediate; the ternary transform's values.
 static uint64_t dual_scratch_bytes(const cuot_ctx *ctx, QcKind k, int e, int batch, bool r2) {
+  if (k == kQcTern) return tern_job_bytes(e);
   if (k == kQcKara) return qck_scratch_bytes(e) + y_bytes(true, kQcfMaxE, leaf_batch(ctx));
   return ((r2 ? 32ull : 16ull) << e) + y_bytes(k == kQcFft, e, batch);
 }
@@ -877,14 +890,16 @@ static uint64_t dual_y_offset(QcKind k, int e, bool r2) {
 struct QcEngine {
   QcKind kind;
   QcTables *t;   // NTT tables (NTT, and Karatsuba plans' plane encodes)
-  QcfTables *f;  // FFT tables (FFT: of n; Karatsuba: of the 2^22 leaves)
+  QcfTables *f;  // FFT tables (FFT, and ternary plans' plane encodes: of n; Karatsuba: of the 2^22 leaves)
 };
 
-static int engine(cuot_ctx *ctx, int e, QcKind kind, QcEngine *g) {
+// planes: the plane encodes of a plan are wanted too.
+static int engine(cuot_ctx *ctx, int e, QcKind kind, bool planes, QcEngine *g) {
   g->kind = kind;
   g->t = nullptr;
   g->f = nullptr;
-  if (kind == kQcFft) return qcf_get_tables(ctx, e, &g->f);
+  if (kind == kQcTern && !planes) return CUOT_OK;  // the ternary transform needs no tables
+  if (planes_by_fft(kind)) return qcf_get_tables(ctx, e, &g->f);
   if (kind == kQcKara) CUOT_TRY(qcf_get_tables(ctx, kQcfMaxE, &g->f));
   CUOT_TRY(get_tables(ctx, e, &g->t));
   return set_attrs(g->t);
@@ -902,6 +917,11 @@ static QcfAhatTab single_tab(const void *ahat) {
 static int eng_ahat(const QcEngine &g, int e, const uint64_t *a_d, void *scr, void *ahat, bool with_planes,
                     cudaStream_t st) {
   if (g.kind == kQcFft) return qcf_build_ahat(g.f, a_d, scr, ahat, st);
+  if (g.kind == kQcTern) {
+    CUOT_TRY(tern_build_ahat(e, a_d, scr, ahat, st));
+    if (!with_planes) return CUOT_OK;
+    return qcf_build_ahat(g.f, a_d, scr, static_cast<uint8_t *>(ahat) + tern_ahat_span(e), st);
+  }
   if (g.kind == kQcKara) {
     const uint64_t bb = qck_bits_scratch_bytes(e);
     CUOT_TRY(qck_build_ahat(g.f, e, a_d, scr, static_cast<uint8_t *>(scr) + bb, ahat, st));
@@ -912,11 +932,13 @@ static int eng_ahat(const QcEngine &g, int e, const uint64_t *a_d, void *scr, vo
 }
 
 // Planes p < nplanes: in + p * stride -> out + p * stride (64-bit words),
-// written or XORed into (accumulate).  A Karatsuba plan encodes planes with
-// the NTT A_hat stored after its leaves.
+// written or XORed into (accumulate).  A ternary (Karatsuba) plan encodes
+// planes with the FFT (NTT) A_hat stored after its constants (leaves).
 static int eng_encode(const QcEngine &g, int e, const void *ahat, const uint64_t *in, uint64_t *out, uint64_t stride,
                       int accumulate, int nplanes, void *Y, int batch, cudaStream_t st) {
-  if (g.kind == kQcFft) return qcf_encode(g.f, single_tab(ahat), in, out, stride, accumulate, nplanes, Y, batch, st);
+  if (g.kind == kQcTern) ahat = static_cast<const uint8_t *>(ahat) + tern_ahat_span(e);
+  if (planes_by_fft(g.kind))
+    return qcf_encode(g.f, single_tab(ahat), in, out, stride, accumulate, nplanes, Y, batch, st);
   if (g.kind == kQcKara) ahat = static_cast<const uint8_t *>(ahat) + qck_ahat_bytes(e);
   return encode_planes_strided(g.t, static_cast<const uint2 *>(ahat), in, out, stride, accumulate, nplanes,
                                static_cast<uint32_t *>(Y), batch, st);
@@ -928,9 +950,13 @@ static int eng_encode(const QcEngine &g, int e, const void *ahat, const uint64_t
 static int eng_dual(cuot_ctx *ctx, const QcEngine &g, int e, const void *ahat, const cuot_block *in, cuot_block *out,
                     bool r2, uint8_t *scr, int batch, cudaStream_t st) {
   const uint64_t n = 1ull << e;
-  void *Y = scr + dual_y_offset(g.kind, e, r2);
   const cuot_block *src = r2 ? in + n : in;
   const cuot_block *xor_in = r2 ? in : nullptr;
+  if (g.kind == kQcTern) {
+    const TernJob job{src, xor_in, out, ahat};
+    return tern_dual(e, &job, 1, scr, st);
+  }
+  void *Y = scr + dual_y_offset(g.kind, e, r2);
   if (g.kind == kQcKara) return qck_dual_lpn(g.f, e, ahat, src, xor_in, out, scr, Y, leaf_batch(ctx), st);
   if (g.kind == kQcFft) {
     uint32_t *tiles = reinterpret_cast<uint32_t *>(scr);
@@ -951,82 +977,72 @@ static int eng_dual(cuot_ctx *ctx, const QcEngine &g, int e, const void *ahat, c
 }
 
 // ---- helpers for the batched engine (batch.cu) ----------------------------
-int qc_prepare(cuot_ctx *ctx, int e) {
+int qc_kind(const cuot_ctx *ctx, int e) { return dual_kind(ctx, e); }
+
+int qc_prepare(cuot_ctx *ctx, int kind, int e) {
   QcEngine g;
-  return engine(ctx, e, dual_kind(ctx, e), &g);
+  return engine(ctx, e, QcKind(kind), false, &g);
 }
 
-uint64_t qc_ahat_bytes(const cuot_ctx *ctx, int e) { return ahat_bytes(dual_kind(ctx, e), e, false); }
+uint64_t qc_ahat_bytes(int kind, int e) { return ahat_bytes(QcKind(kind), e, false); }
 
-int qc_lane(const cuot_ctx *ctx, int e) {
-  const QcKind k = dual_kind(ctx, e);
-  if (k == kQcFft) return e;
-  if (k == kQcKara) return kQcfMaxE;  // its leaves run on the 2^22 FFT tables
-  return 64 + e;                      // NTT tables hold no per-call state
+int qc_lane(int kind, int e) {
+  if (kind == kQcFft) return e;
+  if (kind == kQcKara) return kQcfMaxE;  // its leaves run on the 2^22 FFT tables
+  return 64 + e;                         // the NTT and the ternary transform keep no per-call state in the context
 }
 
-uint64_t qc_y_bytes(const cuot_ctx *ctx, int e, int batch) {
-  const QcKind k = dual_kind(ctx, e);
-  const uint64_t y = k == kQcKara ? dual_scratch_bytes(ctx, k, e, batch, false) : y_bytes(k == kQcFft, e, batch);
+uint64_t qc_layout_bytes(int kind, int e, int njobs) {
+  return kind == kQcFft || kind == kQcNtt ? uint64_t(njobs) * 16 << e : 0;
+}
+
+// Dual LPNs per launch of the ternary transform for a batch of `batch`
+// planes: as many as leave its values (tern_job_bytes each) in L2.
+static int tern_jobs_per_launch(int e, int batch) {
+  const uint64_t fit = (80ull << 20) / tern_job_bytes(e);
+  uint64_t jobs = uint64_t(batch > 128 ? batch / 128 : 1);
+  if (jobs > kTernMaxJobs) jobs = kTernMaxJobs;
+  return int(jobs < fit ? jobs : fit < 1 ? 1 : fit);
+}
+
+uint64_t qc_y_bytes(const cuot_ctx *ctx, int kind, int e, int batch) {
+  const QcKind k = QcKind(kind);
+  const uint64_t y = k == kQcKara   ? dual_scratch_bytes(ctx, k, e, batch, false)
+                     : k == kQcTern ? tern_jobs_per_launch(e, batch) * tern_job_bytes(e)
+                                    : y_bytes(k == kQcFft, e, batch);
   const uint64_t a = ahat_scratch_bytes(k, e);
   return y > a ? y : a;
 }
 
-int qc_build_ahat(cuot_ctx *ctx, int e, const uint64_t *a_d, void *Y, void *ahat, cudaStream_t st) {
+int qc_build_ahat(cuot_ctx *ctx, int kind, int e, const uint64_t *a_d, void *Y, void *ahat, cudaStream_t st) {
   QcEngine g;
-  CUOT_TRY(engine(ctx, e, dual_kind(ctx, e), &g));
+  CUOT_TRY(engine(ctx, e, QcKind(kind), false, &g));
   return eng_ahat(g, e, a_d, Y, ahat, false, st);
 }
 
-int qc_job_to_layout(const cuot_ctx *ctx, int e, const cuot_block *in, void *job, cudaStream_t st) {
-  const QcKind k = dual_kind(ctx, e);
-  if (k == kQcFft) return qcf_gather(e, in, static_cast<uint32_t *>(job), st);
-  if (k == kQcKara) {
-    if (cudaMemcpyAsync(job, in, 16ull << e, cudaMemcpyDeviceToDevice, st) != cudaSuccess) return launch_status(0);
-    return CUOT_OK;
-  }
-  return transpose_launch(in, 1ull << e, 16, 0, 128, job, st);
-}
-
-int qc_job_from_layout(const cuot_ctx *ctx, int e, const void *job, cuot_block *out, cudaStream_t st) {
-  const QcKind k = dual_kind(ctx, e);
-  if (k == kQcFft) return qcf_scatter(e, static_cast<const uint32_t *>(job), nullptr, out, st);
-  if (k == kQcKara) {
-    if (cudaMemcpyAsync(out, job, 16ull << e, cudaMemcpyDeviceToDevice, st) != cudaSuccess) return launch_status(0);
-    return CUOT_OK;
-  }
-  return transpose_launch(job, 128, (1ull << e) / 8, 0, 1ull << e, out, st);
-}
-
-// Encodes `njobs` consecutive jobs (16n bytes each: 128 planes, the FFT's
-// tile layout, or the blocks themselves for Karatsuba) in place; job j uses
-// ahats[j] (host array of device pointers).  Y holds qc_y_bytes(batch).
-int qc_encode_jobs(cuot_ctx *ctx, int e, uint64_t *planes, int njobs, const void *const *ahats, void *Y,
-                   int batch, cudaStream_t st) {
-  QcEngine g;
-  CUOT_TRY(engine(ctx, e, dual_kind(ctx, e), &g));
+static int encode_jobs_fft(const QcEngine &g, int e, cuot_block *const *io, int njobs, const void *const *ahats,
+                           uint32_t *tiles, void *Y, int batch, cudaStream_t st) {
   const uint64_t n = 1ull << e;
-  if (g.kind == kQcKara) {
-    for (int j = 0; j < njobs; j++) {
-      cuot_block *blk = reinterpret_cast<cuot_block *>(planes) + uint64_t(j) * n;
-      CUOT_TRY(eng_dual(ctx, g, e, ahats[j], blk, blk, false, static_cast<uint8_t *>(Y), batch, st));
-    }
-    return CUOT_OK;
+  for (int j = 0; j < njobs; j++) CUOT_TRY(qcf_gather(e, io[j], tiles + uint64_t(j) * n * 4, st));
+  int bt = batch < 4 ? 1 : batch / 4;
+  if (bt > 32 * 15) bt = 32 * 15;  // a launch may span at most 16 jobs
+  for (int t0 = 0; t0 < 32 * njobs; t0 += bt) {
+    const int ntr = 32 * njobs - t0 < bt ? 32 * njobs - t0 : bt;
+    QcfAhatTab tab{};
+    tab.per = 32;
+    tab.first = t0 % 32;
+    for (int j = 0; j < 16 && t0 / 32 + j < njobs; j++) tab.p[j] = ahats[t0 / 32 + j];
+    CUOT_TRY(qcf_encode_tiles(g.f, tab, tiles + uint64_t(t0) * (n / 8), ntr, Y, 4 * ntr, st));
   }
-  if (g.kind == kQcFft) {
-    int bt = batch < 4 ? 1 : batch / 4;
-    if (bt > 32 * 15) bt = 32 * 15;  // a launch may span at most 16 jobs
-    uint32_t *tiles = reinterpret_cast<uint32_t *>(planes);
-    for (int t0 = 0; t0 < 32 * njobs; t0 += bt) {
-      const int ntr = 32 * njobs - t0 < bt ? 32 * njobs - t0 : bt;
-      QcfAhatTab tab{};
-      tab.per = 32;
-      tab.first = t0 % 32;
-      for (int j = 0; j < 16 && t0 / 32 + j < njobs; j++) tab.p[j] = ahats[t0 / 32 + j];
-      CUOT_TRY(qcf_encode_tiles(g.f, tab, tiles + uint64_t(t0) * (n / 8), ntr, Y, 4 * ntr, st));
-    }
-    return CUOT_OK;
-  }
+  for (int j = 0; j < njobs; j++) CUOT_TRY(qcf_scatter(e, tiles + uint64_t(j) * n * 4, nullptr, io[j], st));
+  return CUOT_OK;
+}
+
+static int encode_jobs_ntt(const QcEngine &g, int e, cuot_block *const *io, int njobs, const void *const *ahats,
+                           uint64_t *planes, void *Y, int batch, cudaStream_t st) {
+  const uint64_t n = 1ull << e;
+  for (int j = 0; j < njobs; j++)
+    CUOT_TRY(transpose_launch(io[j], n, 16, 0, 128, planes + uint64_t(j) * n * 2, st));
   const int nplanes = 128 * njobs;
   // a launch may span at most kAhatTab jobs
   if (batch > 128 * (kAhatTab - 1)) batch = 128 * (kAhatTab - 1);
@@ -1046,7 +1062,34 @@ int qc_encode_jobs(cuot_ctx *ctx, int e, uint64_t *planes, int njobs, const void
                    n / 8);
     launches += 3;
   }
-  return launch_status(launches);
+  CUOT_TRY(launch_status(launches));
+  for (int j = 0; j < njobs; j++)
+    CUOT_TRY(transpose_launch(planes + uint64_t(j) * n * 2, 128, n / 8, 0, n, io[j], st));
+  return CUOT_OK;
+}
+
+int qc_encode_jobs(cuot_ctx *ctx, int kind, int e, cuot_block *const *io, int njobs, const void *const *ahats,
+                   void *layout, void *Y, int batch, cudaStream_t st) {
+  QcEngine g;
+  CUOT_TRY(engine(ctx, e, QcKind(kind), false, &g));
+  if (g.kind == kQcTern) {
+    const int per = tern_jobs_per_launch(e, batch);
+    for (int j0 = 0; j0 < njobs; j0 += per) {
+      TernJob jobs[kTernMaxJobs];
+      const int nj = njobs - j0 < per ? njobs - j0 : per;
+      for (int j = 0; j < nj; j++) jobs[j] = TernJob{io[j0 + j], nullptr, io[j0 + j], ahats[j0 + j]};
+      CUOT_TRY(tern_dual(e, jobs, nj, Y, st));
+    }
+    return CUOT_OK;
+  }
+  if (g.kind == kQcKara) {
+    for (int j = 0; j < njobs; j++)
+      CUOT_TRY(eng_dual(ctx, g, e, ahats[j], io[j], io[j], false, static_cast<uint8_t *>(Y), batch, st));
+    return CUOT_OK;
+  }
+  if (g.kind == kQcFft)
+    return encode_jobs_fft(g, e, io, njobs, ahats, static_cast<uint32_t *>(layout), Y, batch, st);
+  return encode_jobs_ntt(g, e, io, njobs, ahats, static_cast<uint64_t *>(layout), Y, batch, st);
 }
 
 int qc_default_batch(uint64_t n, int nplanes) { return default_batch(n, nplanes); }
@@ -1109,7 +1152,7 @@ int cuot_qc_plan_create(cuot_ctx *ctx, const uint64_t *a_d, uint64_t n, void *st
   DeviceGuard dg(ctx);
   cuot_qc_plan *pl = new cuot_qc_plan{ctx, e, n, dual_kind(ctx, e), nullptr, 0};
   QcEngine g;
-  int st = engine(ctx, e, pl->kind, &g);
+  int st = engine(ctx, e, pl->kind, true, &g);
   if (st == CUOT_OK) st = dev_alloc(&pl->ahat, ahat_bytes(pl->kind, e, true));
   void *scr = nullptr;
   if (st == CUOT_OK) st = scratch(ctx, ahat_scratch_bytes(pl->kind, e), &scr);
@@ -1143,10 +1186,10 @@ int cuot_qc_plan_encode(cuot_qc_plan *pl, uint64_t *planes_io_d, int nplanes, vo
   cuot_ctx *ctx = pl->ctx;
   DeviceGuard dg(ctx);
   QcEngine g;
-  CUOT_TRY(engine(ctx, pl->e, pl->kind, &g));
+  CUOT_TRY(engine(ctx, pl->e, pl->kind, true, &g));
   const int batch = pl->batch < nplanes ? pl->batch : nplanes;
   void *scr;
-  CUOT_TRY(scratch(ctx, y_bytes(pl->kind == kQcFft, pl->e, batch), &scr));
+  CUOT_TRY(scratch(ctx, y_bytes(planes_by_fft(pl->kind), pl->e, batch), &scr));
   return eng_encode(g, pl->e, pl->ahat, planes_io_d, planes_io_d, pl->n / 64, 0, nplanes, scr, batch,
                     static_cast<cudaStream_t>(stream));
 }
@@ -1156,7 +1199,7 @@ int cuot_qc_plan_dual_lpn(cuot_qc_plan *pl, cuot_block *io_d, void *stream) {
   cuot_ctx *ctx = pl->ctx;
   DeviceGuard dg(ctx);
   QcEngine g;
-  CUOT_TRY(engine(ctx, pl->e, pl->kind, &g));
+  CUOT_TRY(engine(ctx, pl->e, pl->kind, false, &g));
   const int batch = pl->batch < 128 ? pl->batch : 128;
   void *scr;
   CUOT_TRY(scratch(ctx, dual_scratch_bytes(ctx, pl->kind, pl->e, batch, false), &scr));
@@ -1169,7 +1212,7 @@ int cuot_qc_plan_dual_lpn_r2(cuot_qc_plan *pl, const cuot_block *in_d, cuot_bloc
   cuot_ctx *ctx = pl->ctx;
   DeviceGuard dg(ctx);
   QcEngine g;
-  CUOT_TRY(engine(ctx, pl->e, pl->kind, &g));
+  CUOT_TRY(engine(ctx, pl->e, pl->kind, false, &g));
   const int batch = pl->batch < 128 ? pl->batch : 128;
   void *scr;
   CUOT_TRY(scratch(ctx, dual_scratch_bytes(ctx, pl->kind, pl->e, batch, true), &scr));
@@ -1185,7 +1228,7 @@ int cuot_qc_encode(cuot_ctx *ctx, const uint64_t *a_d, uint64_t *planes_io_d, ui
   DeviceGuard dg(ctx);
   QcEngine g;
   const QcKind kind = plane_kind(ctx, e);
-  CUOT_TRY(engine(ctx, e, kind, &g));
+  CUOT_TRY(engine(ctx, e, kind, false, &g));
   int batch = ctx->qc_planes_per_pass > 0 ? ctx->qc_planes_per_pass : default_batch(n, nplanes);
   if (batch > nplanes) batch = nplanes;
   const uint64_t ab = ahat_bytes(kind, e, false);
@@ -1206,7 +1249,7 @@ static int one_shot_dual(cuot_ctx *ctx, const uint64_t *a_d, const cuot_block *i
   DeviceGuard dg(ctx);
   QcEngine g;
   const QcKind kind = dual_kind(ctx, e);
-  CUOT_TRY(engine(ctx, e, kind, &g));
+  CUOT_TRY(engine(ctx, e, kind, false, &g));
   const int batch = one_shot_batch(ctx, n);
   const uint64_t ab = ahat_bytes(kind, e, false);
   void *scr;

@@ -1,0 +1,470 @@
+// qc_tern.cu -- exact quasi-cyclic dual LPN of n = 2^e blocks, 16 <= e <= 22,
+// by the ternary transform of qc_tern.cuh: out = a * in mod (x^n - 1) for all
+// 128 bit planes at once, with blocks read and written as they are (a block
+// is the 128 planes' bits of one coefficient, so no bit transpose is needed)
+// and XORs only.
+//
+// Kernels of one dual LPN, between two buffers of P points x L pairs of words
+// per 32 planes ([word group][point][part][coefficient]):
+//   tern_pass27            pieces of the input -> first pass of every coset
+//   tern_pass27 / pass9    the other forward passes
+//   tern_inner             per point and 32 planes: the product in R_L, in
+//                          shared memory (in place)
+//   tern_pass27 / pass9    inverse passes
+//   tern_final             pieces -> coefficients mod x^n - 1 (XORed with xor_in)
+// Measured on B200, one dual LPN through a plan, the fp64 FFT path against this:
+// n = 2^16 65 / 61 us, 2^17 102 / 90, 2^18 184 / 122, 2^19 371 / 215, 2^20 727
+// / 425, 2^21 1542 / 1118, 2^22 3346 / 2288.
+#include "ctx.cuh"
+#include "qc_tern.cuh"
+
+namespace cuot {
+namespace {
+
+struct TernJobs {
+  const uint32_t *in[kTernMaxJobs];
+  const uint32_t *xor_in[kTernMaxJobs];
+  uint32_t *out[kTernMaxJobs];
+  const uint32_t *consts[kTernMaxJobs];
+};
+
+// sigma of every node of every pass and size (host: for nothing but the upload).
+__constant__ TernSigmas c_sigmas = tern_sigmas();
+
+// What a pass reads and writes: src != dst, or the pieces of jobs.in first.
+struct PassArgs {
+  int e, pass;
+  int W;  // word groups: 4, or 1 for the bits of `a`
+  const uint32_t *src;
+  uint32_t *dst;
+  uint64_t job_words;
+  TernJobs jobs;
+};
+enum PassKind { kFirst, kFirstBits, kForward, kInverse, kLastInverse };
+constexpr bool pass_first(PassKind k) { return k == kFirst || k == kFirstBits; }
+constexpr bool pass_inverse(PassKind k) { return k == kInverse || k == kLastInverse; }
+
+// Rotation table of a pass in shared memory, and the one of its rotated stores.
+template <int L, PassKind KIND>
+__device__ __forceinline__ void fill_tables(RotEntry *load, RotEntry *store) {
+  for (int i = threadIdx.x; i < kRotEntries; i += blockDim.x) {
+    load[i] = pass_first(KIND) ? rot_entry_first(L, i) : rot_entry(L, i, false);
+    if (KIND == kLastInverse) store[i] = rot_entry(L, i, true);
+  }
+}
+
+// The pieces (children) k0 + dk k (k < N) of a butterfly, blocks i0 + 3c (c < 3)
+// of residue r.  All words are loaded before the first is touched: the masks
+// of the rotations are looked up again afterwards, since holding them would
+// halve the loads in flight.
+template <int L, int RAD, int N, PassKind KIND>
+__device__ __forceinline__ void load_slots(const PassArgs &a, const Butterfly &b, const uint16_t *sigmas,
+                                           const uint32_t *src, const RotEntry *tab, int k0, int dk, int i0, int r,
+                                           int w, G4 (&f)[N][3]) {
+  int ti[N];
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    const int slot = k0 + dk * k;
+    const RotBase rb =
+        rot_base<L>(pass_inverse(KIND) ? inv_rotation<L>(b, sigmas, slot) : fwd_rotation<RAD>(b, slot), r);
+    ti[k] = rb.i + i0;
+    if constexpr (pass_first(KIND)) {
+      const int at = (b.piece + slot * b.step) * L + rb.off;
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        const int j = at + tab[ti[k] + 3 * c].x;
+        uint32_t x = 0;
+        if (j < (1 << a.e)) x = KIND == kFirstBits ? __ldg(&src[j >> 5]) >> (j & 31) : __ldg(&src[j * 4 + w]);
+        f[k][c].a = x;
+      }
+    } else {
+      const uint32_t *p = src + (b.first + slot * b.step) * tern_element(L) + rb.off;
+#pragma unroll
+      for (int c = 0; c < 3; c++) f[k][c] = load_raw(p, tab[ti[k] + 3 * c]);
+    }
+  }
+  asm volatile("" ::: "memory");  // or the compiler keeps the masks of the first lookup
+#pragma unroll
+  for (int k = 0; k < N; k++)
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const RotEntry t = tab[ti[k] + 3 * c];
+      if constexpr (pass_first(KIND)) {
+        const uint32_t x = KIND == kFirstBits ? 0u - (f[k][c].a & 1u) : f[k][c].a;
+        f[k][c] = G4{x & t.m1, x & t.m2};
+      } else {
+        f[k][c] = load_fix(t, f[k][c]);
+      }
+    }
+}
+
+// A thread's word group w and residue r from its index over both.  The first
+// pass reads whole blocks (word groups fastest), the others contiguous words.
+struct Lane {
+  int w, r;
+  bool on;
+};
+template <int L, PassKind KIND>
+__device__ __forceinline__ Lane lane_of(int id, int W) {
+  constexpr int B = tern_block(L);
+  const Lane l = pass_first(KIND) ? Lane{id % W, id / W, false} : Lane{id / B, id % B, false};
+  return Lane{l.w, l.r, l.w < W && l.r < L / 9};
+}
+
+// Radix 27: butterfly blockIdx.x, 32 (word group, residue) indices per
+// CTA (blockIdx.y), job blockIdx.z.  Nine warps: a warp first takes the 9-point
+// DFTs over k1 of one k2 and one coefficient class i0, then the three-point
+// ones of one q1; the 243 pairs of every lane change hands in shared memory.
+constexpr int kExchangeBytes = 243 * 2 * 32 * 4;
+template <int L, PassKind KIND>
+__global__ void __launch_bounds__(288) tern_pass27(PassArgs a) {
+  constexpr int B = tern_block(L);
+  const int W = KIND == kFirst ? 4 : KIND == kFirstBits ? 1 : a.W;
+  extern __shared__ uint32_t X[];  // [q1][k2][coefficient][word][lane]
+  __shared__ RotEntry tab[kRotEntries], stab[KIND == kLastInverse ? kRotEntries : 1];
+  fill_tables<L, KIND>(tab, stab);
+  const TernShape s = tern_shape(a.e);
+  const uint16_t *sigmas = c_sigmas.v[a.e - kTernMinE];
+  const Butterfly b = tern_butterfly(s, sigmas, a.pass, blockIdx.x, pass_inverse(KIND));
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const Lane ln = lane_of<L, KIND>(blockIdx.y * 32 + lane, W);
+  const int w = ln.w, r = ln.r;
+  const uint64_t group = uint64_t(tern_points(s)) * tern_element(L);
+  const uint64_t at = uint64_t(blockIdx.z) * a.job_words + uint64_t(w) * group;
+  __syncthreads();
+  {
+    const uint32_t *src = pass_first(KIND) ? a.jobs.in[blockIdx.z] : a.src + at;
+    const int k2 = warp / 3, i0 = warp % 3;
+    G4 f[9][3];
+    if (ln.on) {
+      load_slots<L, 27, 9, KIND>(a, b, sigmas, src, tab, k2, 3, i0, r, w, f);
+      dft<9>(f);
+#pragma unroll
+      for (int q1 = 0; q1 < 9; q1++)
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          uint32_t *x = X + ((q1 * 3 + k2) * 9 + i0 + 3 * c) * 64 + lane;
+          x[0] = f[dft_slot<9>(q1)][c].a;
+          x[32] = f[dft_slot<9>(q1)][c].b;
+        }
+    }
+  }
+  __syncthreads();
+  if (!ln.on) return;
+  const int q1 = warp;
+  uint32_t *o[3];
+  RotBase rb[3];
+#pragma unroll
+  for (int q2 = 0; q2 < 3; q2++) {
+    const int q = q1 + 9 * q2, k = pass_inverse(KIND) ? (27 - q) % 27 : q;
+    rb[q2] = rot_base<L>(KIND == kLastInverse ? fwd_rotation<27>(b, k) : 0, r);
+    o[q2] = a.dst + at + (b.first + k * b.step) * tern_element(L) + rb[q2].off;
+  }
+#pragma unroll
+  for (int i = 0; i < 9; i++) {
+    G4 y[3];
+#pragma unroll
+    for (int k2 = 0; k2 < 3; k2++) {
+      const int d = i - q1 * k2, wraps = (8 - d) / 9;
+      const uint32_t *x = X + ((q1 * 3 + k2) * 9 + d + 9 * wraps) * 64 + lane;
+      y[k2] = dft27_twiddle(G4{x[0], x[32]}, wraps);
+    }
+    dft3(y[0], y[1], y[2]);
+#pragma unroll
+    for (int q2 = 0; q2 < 3; q2++) {
+      if constexpr (KIND == kLastInverse) {
+        store_pair(o[q2], stab[rb[q2].i + i], y[q2]);
+      } else {
+        o[q2][i * B] = y[q2].a;
+        o[q2][i * B + tern_part(L)] = y[q2].b;
+      }
+    }
+  }
+}
+
+// Radix 9 or 3: a thread holds three blocks' coefficients of all pieces.
+template <int L, int RAD, PassKind KIND>
+__global__ void __launch_bounds__(128) tern_pass9(PassArgs a) {
+  constexpr int B = tern_block(L);
+  __shared__ RotEntry tab[kRotEntries];
+  fill_tables<L, KIND>(tab, nullptr);
+  const TernShape s = tern_shape(a.e);
+  const uint16_t *sigmas = c_sigmas.v[a.e - kTernMinE];
+  const Butterfly b = tern_butterfly(s, sigmas, a.pass, blockIdx.x, pass_inverse(KIND));
+  const int id = blockIdx.y * 128 + threadIdx.x, i0 = id / (a.W * B);
+  const Lane ln = lane_of<L, KIND>(id % (a.W * B), a.W);
+  __syncthreads();
+  if (!ln.on || i0 >= 3) return;
+  const uint64_t at = uint64_t(blockIdx.z) * a.job_words + uint64_t(ln.w) * tern_points(s) * tern_element(L);
+  G4 f[RAD][3];
+  load_slots<L, RAD, RAD, KIND>(a, b, sigmas, a.src + at, tab, 0, 1, i0, ln.r, ln.w, f);
+  dft<RAD>(f);
+  uint32_t *o = a.dst + at + b.first * tern_element(L) + i0 * B + ln.r;
+  const int step = b.step * tern_element(L);
+#pragma unroll
+  for (int k = 0; k < RAD; k++) {
+    const int slot = pass_inverse(KIND) ? idft_slot<RAD>(k) : dft_slot<RAD>(k);
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      o[k * step + 3 * c * B] = f[slot][c].a;
+      o[k * step + 3 * c * B + tern_part(L)] = f[slot][c].b;
+    }
+  }
+}
+
+// The product in R_L of one point and 32 planes (blockIdx.x: point, y: word
+// group, z: job); CONSTS: the leaf constants of the element instead.
+template <class S>
+constexpr int inner_threads() {
+  return S::L == 243 ? 96 : 288;
+}
+template <class S, bool CONSTS>
+__global__ void __launch_bounds__(inner_threads<S>()) tern_inner(uint32_t *buf, uint64_t job_words, TernJobs jobs,
+                                                                 uint32_t *consts_out) {
+  extern __shared__ uint32_t V[];
+  constexpr int NT = inner_threads<S>();
+  static_assert(S::TASK0 <= NT && S::TASK1 <= NT && S::TASK2 <= NT, "one round of butterflies: every load before the first store");
+  const int tid = threadIdx.x;
+  uint32_t *x = buf + uint64_t(blockIdx.z) * job_words + (uint64_t(blockIdx.y) * gridDim.x + blockIdx.x) * tern_element(S::L);
+  if (tid < S::TASK0) p0<S>(x, V, tid);
+  __syncthreads();
+  {
+    const Task1 t = task1<S>(tid);
+    G4 f[S::R1][3];
+    if (tid < S::TASK1) p1_load<S>(V, t, f);
+    __syncthreads();
+    if (tid < S::TASK1) {
+      dft<S::R1>(f);
+      p1_store<S>(V, t, f);
+    }
+  }
+  __syncthreads();
+  const Task2 t2 = task2<S>(tid);
+  {
+    G4 f[3][S::G];
+    if (tid < S::TASK2) p2_load<S>(V, t2, f);
+    __syncthreads();
+    if (tid < S::TASK2) {
+      if constexpr (CONSTS) {
+#pragma unroll
+        for (int q = 0; q < 3; q++)
+#pragma unroll
+          for (int c = 0; c < S::G; c++) fwd_store<S::LP>(V + (t2.group * 3 + q) * S::ES, t2.r + 9 * c, f[q][c]);
+      } else {
+        p2_store<S>(V, t2, f);
+      }
+    }
+  }
+  __syncthreads();
+  if constexpr (CONSTS) {
+    uint32_t *o = consts_out + uint64_t(blockIdx.x) * kLeafWords * S::LEAVES;
+    for (int i = tid; i < S::LEAVES; i += NT) {
+      // a warp's evaluations are (nearly) one: no divergence between its cases
+      const int ev = i / S::NE, q = i / (2 * S::R1) % 3, group = i % (2 * S::R1);
+      uint32_t w[kLeafWords];
+      leaf_consts<S>(V + (group * 3 + q) * S::ES, ev, w);
+      const int id = leaf_id<S>(group, q, ev);
+#pragma unroll
+      for (int j = 0; j < kLeafWords; j++) o[j * S::LEAVES + id] = w[j];
+    }
+    return;
+  }
+  const uint32_t *cs = jobs.consts[blockIdx.z] + uint64_t(blockIdx.x) * kLeafWords * S::LEAVES;
+  for (int i = tid; i < S::LEAVES; i += NT) {
+    uint32_t v[18], w[kLeafWords];
+#pragma unroll
+    for (int j = 0; j < kLeafWords; j++) w[j] = __ldg(&cs[j * S::LEAVES + i]);
+#pragma unroll
+    for (int j = 0; j < 18; j++) v[j] = V[j * S::SL + i];
+    leaf9(v, w);
+#pragma unroll
+    for (int j = 0; j < 18; j++) V[j * S::SL + i] = v[j];
+  }
+  __syncthreads();
+  {
+    G4 f[3][S::G];
+    if (tid < S::TASK2) p4_load<S>(V, t2, f);
+    __syncthreads();
+    if (tid < S::TASK2) p4_store<S>(V, t2, f);
+  }
+  __syncthreads();
+  {
+    const Task1 t = task1<S>(tid);
+    G4 f[S::R1][3];
+    if (tid < S::TASK1) p5_load<S>(V, t, f);
+    __syncthreads();
+    if (tid < S::TASK1) {
+      dft<S::R1>(f);
+      p5_store<S>(V, t, f);
+    }
+  }
+  __syncthreads();
+  if (tid < S::TASK0) p6<S>(V, x, tid);
+}
+
+// A thread per coefficient: the word groups' coefficients of a warp are each
+// contiguous, and its blocks are written whole.
+template <int E>
+__global__ void __launch_bounds__(256) tern_final(const uint32_t *buf, uint64_t job_words, TernJobs jobs) {
+  constexpr TernShape s = tern_shape(E);
+  const uint32_t j = blockIdx.x * 256 + threadIdx.x;
+  const uint32_t *b = buf + uint64_t(blockIdx.z) * job_words;
+  constexpr uint64_t group = uint64_t(tern_points(s)) * tern_element(s.L);
+  uint4 v = make_uint4(tern_coefficient<E>(b, j), tern_coefficient<E>(b + group, j), tern_coefficient<E>(b + 2 * group, j),
+                       tern_coefficient<E>(b + 3 * group, j));
+  const uint4 *xi = reinterpret_cast<const uint4 *>(jobs.xor_in[blockIdx.z]);
+  if (xi) {
+    const uint4 x = xi[j];
+    v = make_uint4(v.x ^ x.x, v.y ^ x.y, v.z ^ x.z, v.w ^ x.w);
+  }
+  reinterpret_cast<uint4 *>(jobs.out[blockIdx.z])[j] = v;
+}
+
+uint64_t group_words(int e) {
+  const TernShape s = tern_shape(e);
+  return uint64_t(tern_points(s)) * tern_element(s.L);
+}
+
+template <int L, PassKind KIND>
+int pass27(const PassArgs &a, int njobs, cudaStream_t st) {
+  const cudaError_t e =
+      cudaFuncSetAttribute(tern_pass27<L, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, kExchangeBytes);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(CUOT_ECUDA, "QC shared-memory attribute failed: %s", cudaGetErrorString(e));
+  }
+  const dim3 grid(tern_points(tern_shape(a.e)) / 27, (a.W * tern_block(L) + 31) / 32, njobs);
+  tern_pass27<L, KIND><<<grid, 288, kExchangeBytes, st>>>(a);
+  return CUOT_OK;
+}
+template <int L, int RAD, PassKind KIND>
+int pass9(const PassArgs &a, int njobs, cudaStream_t st) {
+  const dim3 grid(tern_points(tern_shape(a.e)) / RAD, (3 * a.W * tern_block(L) + 127) / 128, njobs);
+  tern_pass9<L, RAD, KIND><<<grid, 128, 0, st>>>(a);
+  return CUOT_OK;
+}
+// Pass a.pass of the transform (KIND kForward: of the passes after the first).
+template <int L>
+int pass_of(const PassArgs &a, PassKind kind, int njobs, cudaStream_t st) {
+  const int rad = tern_radix(tern_shape(a.e).m, a.pass);
+  switch (kind) {
+    case kFirst: return pass27<L, kFirst>(a, njobs, st);
+    case kFirstBits: return pass27<L, kFirstBits>(a, njobs, st);
+    case kLastInverse: return pass27<L, kLastInverse>(a, njobs, st);
+    case kForward:
+      return rad == 27  ? pass27<L, kForward>(a, njobs, st)
+             : rad == 9 ? pass9<L, 9, kForward>(a, njobs, st)
+                        : pass9<L, 3, kForward>(a, njobs, st);
+    default:
+      return rad == 27  ? pass27<L, kInverse>(a, njobs, st)
+             : rad == 9 ? pass9<L, 9, kInverse>(a, njobs, st)
+                        : pass9<L, 3, kInverse>(a, njobs, st);
+  }
+}
+int pass(const PassArgs &a, PassKind kind, int njobs, cudaStream_t st) {
+  switch (tern_shape(a.e).L) {
+    case 243: return pass_of<243>(a, kind, njobs, st);
+    case 729: return pass_of<729>(a, kind, njobs, st);
+    case 1458: return pass_of<1458>(a, kind, njobs, st);
+    default: return pass_of<2187>(a, kind, njobs, st);
+  }
+}
+// Input -> values at the points; *buf: where they are (one of the two halves).
+int forward(int e, PassKind kind, const TernJobs &jobs, uint32_t *half[2], uint64_t job_words, int njobs, int *at,
+            cudaStream_t st) {
+  const int W = kind == kFirstBits ? 1 : 4, passes = tern_passes(tern_shape(e).m);
+  PassArgs a{e, 0, W, nullptr, half[0], job_words, jobs};
+  CUOT_TRY(pass(a, kind, njobs, st));
+  for (a.pass = 1; a.pass < passes; a.pass++) {
+    a.src = half[(a.pass - 1) & 1];
+    a.dst = half[a.pass & 1];
+    CUOT_TRY(pass(a, kForward, njobs, st));
+  }
+  *at = (passes - 1) & 1;
+  return CUOT_OK;
+}
+
+template <class S, bool CONSTS>
+int inner_launch(int P, uint32_t *buf, uint64_t job_words, const TernJobs &jobs, int njobs, uint32_t *consts_out,
+                 cudaStream_t st) {
+  const int smem = S::WORDS * 4;
+  const cudaError_t e = cudaFuncSetAttribute(tern_inner<S, CONSTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(CUOT_ECUDA, "QC shared-memory attribute failed: %s", cudaGetErrorString(e));
+  }
+  tern_inner<S, CONSTS><<<dim3(P, CONSTS ? 1 : 4, njobs), inner_threads<S>(), smem, st>>>(buf, job_words, jobs,
+                                                                                       consts_out);
+  return CUOT_OK;
+}
+template <bool CONSTS>
+int inner(const TernShape &s, uint32_t *buf, uint64_t job_words, const TernJobs &jobs, int njobs, uint32_t *consts_out,
+          cudaStream_t st) {
+  const int P = tern_points(s);
+  switch (s.L) {
+    case 243: return inner_launch<Inner<243, 27>, CONSTS>(P, buf, job_words, jobs, njobs, consts_out, st);
+    case 729: return inner_launch<Inner<729, 27>, CONSTS>(P, buf, job_words, jobs, njobs, consts_out, st);
+    case 1458: return inner_launch<Inner<1458, 54>, CONSTS>(P, buf, job_words, jobs, njobs, consts_out, st);
+    default: return inner_launch<Inner<2187, 81>, CONSTS>(P, buf, job_words, jobs, njobs, consts_out, st);
+  }
+}
+
+}  // namespace
+
+bool tern_supported(int e) { return e >= kTernMinE && e <= kTernMaxE; }
+
+uint64_t tern_ahat_bytes(int e) {
+  const TernShape s = tern_shape(e);
+  return uint64_t(tern_points(s)) * 2 * (s.L / s.Lp) * tern_evals(s.Lp) * kLeafWords * 4;
+}
+
+uint64_t tern_build_bytes(int e) { return 2 * group_words(e) * 4; }
+uint64_t tern_job_bytes(int e) { return 2 * group_words(e) * 16; }
+
+int tern_build_ahat(int e, const uint64_t *a_d, void *scratch, void *ahat, cudaStream_t st) {
+  uint32_t *half[2] = {static_cast<uint32_t *>(scratch), static_cast<uint32_t *>(scratch) + group_words(e)};
+  TernJobs jobs{};
+  jobs.in[0] = reinterpret_cast<const uint32_t *>(a_d);
+  int at = 0;
+  CUOT_TRY(forward(e, kFirstBits, jobs, half, 0, 1, &at, st));
+  CUOT_TRY(inner<true>(tern_shape(e), half[at], 0, jobs, 1, static_cast<uint32_t *>(ahat), st));
+  return launch_status(1 + tern_passes(tern_shape(e).m));
+}
+
+int tern_dual(int e, const TernJob *job, int njobs, void *scratch, cudaStream_t st) {
+  const TernShape s = tern_shape(e);
+  if (njobs > kTernMaxJobs) return fail(CUOT_EINVAL, "%d dual LPNs in one launch (at most %d)", njobs, kTernMaxJobs);
+  const uint64_t job_words = group_words(e) * 4;
+  uint32_t *half[2] = {static_cast<uint32_t *>(scratch), static_cast<uint32_t *>(scratch) + njobs * job_words};
+  const int passes = tern_passes(s.m);
+  TernJobs jobs{};
+  for (int j = 0; j < njobs; j++) {
+    jobs.in[j] = reinterpret_cast<const uint32_t *>(job[j].in);
+    jobs.xor_in[j] = reinterpret_cast<const uint32_t *>(job[j].xor_in);
+    jobs.out[j] = reinterpret_cast<uint32_t *>(job[j].out);
+    jobs.consts[j] = static_cast<const uint32_t *>(job[j].ahat);
+  }
+  int at = 0;
+  CUOT_TRY(forward(e, kFirst, jobs, half, job_words, njobs, &at, st));
+  CUOT_TRY(inner<false>(s, half[at], job_words, jobs, njobs, nullptr, st));
+  PassArgs a{e, 0, 4, nullptr, nullptr, job_words, jobs};
+  for (a.pass = passes - 1; a.pass >= 0; a.pass--, at ^= 1) {
+    a.src = half[at];
+    a.dst = half[at ^ 1];
+    CUOT_TRY(pass(a, a.pass ? kInverse : kLastInverse, njobs, st));
+  }
+  const uint32_t *buf = half[at];
+  const dim3 grid((1u << e) / 256, 1, njobs);
+  switch (e) {
+#define TERN_FINAL(E)                                          \
+  case E:                                                      \
+    tern_final<E><<<grid, 256, 0, st>>>(buf, job_words, jobs); \
+    break;
+    TERN_FINAL(16) TERN_FINAL(17) TERN_FINAL(18) TERN_FINAL(19)
+    TERN_FINAL(20) TERN_FINAL(21) TERN_FINAL(22)
+#undef TERN_FINAL
+  }
+  return launch_status(2 * passes + 2);
+}
+
+}  // namespace cuot

@@ -65,11 +65,13 @@ uint64_t cuot_ctx_scratch_bytes(const cuot_ctx *ctx);
  *   CUOT_TUNE_QC_PLANES     planes per QC pass, 0 = automatic (512 MiB of
  *                           intermediate)
  *   CUOT_TUNE_QC_BACKEND    transform of the exact QC encode: 0 automatic
- *                           (fp64 FFT for n <= 2^22; dual LPNs at 2^23 and
- *                           2^24 as GF(2) Karatsuba over 2^22 FFTs; the NTT
- *                           mod 469762049 above), 1 the NTT everywhere, 2 as
- *                           0.  Plans and batches keep the backend they were
- *                           created with; set it before creating them.
+ *                           (dual LPNs of 2^16 <= n <= 2^22 by the ternary
+ *                           GF(2) transform; otherwise as 2), 1 the NTT
+ *                           everywhere, 2 the fp64 FFT for n <= 2^22, dual
+ *                           LPNs at 2^23 and 2^24 as GF(2) Karatsuba over
+ *                           2^22 FFTs, the NTT mod 469762049 above.  Plans
+ *                           and batches keep the backend they were created
+ *                           with; set it before creating them.
  *   CUOT_TUNE_QC_STREAMS    streams of one FFT encode, 1 or 2 (default 2:
  *                           groups of about 32 MiB of intermediate alternate
  *                           between the caller's stream and a second stream
@@ -84,7 +86,8 @@ uint64_t cuot_ctx_scratch_bytes(const cuot_ctx *ctx);
  *                           distance |v - round(v)| between a computed
  *                           product coefficient and the integer it rounds to
  *                           (exactness needs < 1/2), read by
- *                           cuot_qc_fft_margin.  Setting 1 allocates and
+ *                           cuot_qc_fft_margin.  While it is 1, automatic
+ *                           dual LPNs keep to the FFT.  Setting 1 allocates and
  *                           zeroes one device word (synchronous: not during
  *                           stream capture); plans and batches made later
  *                           record too. */
@@ -298,10 +301,12 @@ int cuot_ferret_chi_sum(cuot_ctx *ctx, const cuot_block *leaves_d, uint64_t t,
  * consecutive) becomes a * plane_r mod (x^n - 1) over GF(2), exactly
  * (replaces the float cuFFT path of QuasiCyclic::encode_dense,
  * quasi_cyclic.cu:118-128).  n a power of two in [2^10, 2^25].  The
- * product is an fp64 FFT carrying four planes per transform for n <= 2^22
- * (exact: the rounding error of the convolution stays below 1/2), GF(2)
- * Karatsuba over that FFT for dual LPNs at 2^23 and 2^24, and a number-
- * theoretic transform mod 469762049 otherwise (CUOT_TUNE_QC_BACKEND).
+ * product is a transform over GF(2)[x] itself for dual LPNs of 2^16 <= n <=
+ * 2^22; an fp64 FFT carrying four planes per transform for plane encodes and
+ * other dual LPNs of n <= 2^22 (exact: the rounding error of the convolution
+ * stays below 1/2), GF(2) Karatsuba over that FFT for dual LPNs at 2^23 and
+ * 2^24, and a number-theoretic transform mod 469762049 otherwise
+ * (CUOT_TUNE_QC_BACKEND).
  * encode_sparse: out = a * e mod (x^n - 1), e = indicator of pos_d[0..w)
  * (QuasiCyclic::encode_sparse, quasi_cyclic.cu:130-161).
  * dual_lpn: io_d holds n blocks; block j becomes XOR_{i: a_i = 1}
