@@ -13,8 +13,8 @@
 //   tern_pass27 / pass9    inverse passes
 //   tern_final             pieces -> coefficients mod x^n - 1 (XORed with xor_in)
 // Measured on B200, one dual LPN through a plan, the fp64 FFT path against this:
-// n = 2^16 65 / 61 us, 2^17 102 / 90, 2^18 184 / 122, 2^19 371 / 215, 2^20 727
-// / 425, 2^21 1542 / 1118, 2^22 3346 / 2288.
+// n = 2^16 65 / 60 us, 2^17 102 / 83, 2^18 184 / 107, 2^19 371 / 189, 2^20 727
+// / 394, 2^21 1542 / 974, 2^22 3346 / 2000.
 #include "ctx.cuh"
 #include "qc_tern.cuh"
 
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(288) tern_pass27(PassArgs a) {
 
 // Radix 9 or 3: a thread holds three blocks' coefficients of all pieces.
 template <int L, int RAD, PassKind KIND>
-__global__ void __launch_bounds__(128) tern_pass9(PassArgs a) {
+__global__ void __launch_bounds__(128, 5) tern_pass9(PassArgs a) {  // 5: all 54 loads in flight (at 80 registers 150 us a pass at 2^22, at 96 125)
   constexpr int B = tern_block(L);
   __shared__ RotEntry tab[kRotEntries];
   fill_tables<L, KIND>(tab, nullptr);
@@ -213,20 +213,25 @@ __global__ void __launch_bounds__(128) tern_pass9(PassArgs a) {
 }
 
 // The product in R_L of one point and 32 planes (blockIdx.x: point, y: word
-// group, z: job); CONSTS: the leaf constants of the element instead.
+// group, z: job).
+// It is bound by the integer pipe (61-63 % busy in ncu), so CTAs are small:
+// fewer warps wait at the barriers between steps whose task counts differ, and
+// more registers per thread keep more independent XORs in flight.  288 threads
+// (one round of leaf products for L = 729) took 60 us at n = 2^18, 245 at 2^20,
+// 1268 at 2^22; these sizes 47, 221 and 1038.
 template <class S>
 constexpr int inner_threads() {
-  return S::L == 243 ? 96 : 288;
+  return S::L == 243 ? 96 : S::L == 1458 ? 256 : 192;
 }
-template <class S, bool CONSTS>
-__global__ void __launch_bounds__(inner_threads<S>()) tern_inner(uint32_t *buf, uint64_t job_words, TernJobs jobs,
-                                                                 uint32_t *consts_out) {
-  extern __shared__ uint32_t V[];
-  constexpr int NT = inner_threads<S>();
-  static_assert(S::TASK0 <= NT && S::TASK1 <= NT && S::TASK2 <= NT, "one round of butterflies: every load before the first store");
-  const int tid = threadIdx.x;
-  uint32_t *x = buf + uint64_t(blockIdx.z) * job_words + (uint64_t(blockIdx.y) * gridDim.x + blockIdx.x) * tern_element(S::L);
-  if (tid < S::TASK0) p0<S>(x, V, tid);
+template <class S>
+constexpr int inner_blocks() {
+  return S::L == 243 ? 8 : S::L == 729 ? 5 : S::L == 1458 ? 3 : 2;
+}
+// Steps 0..2: the element x -> the threads' radix-3 results (below TASK2).
+template <class S, int NT>
+__device__ __forceinline__ void inner_forward(const uint32_t *x, uint32_t *V, int tid, const Task2 &t2, G4 (&f2)[3][S::G]) {
+  static_assert(S::TASK1 <= NT && S::TASK2 <= NT, "one round of butterflies: every load before the first store");
+  for (int i = tid; i < S::TASK0; i += NT) p0<S>(x, V, i);
   __syncthreads();
   {
     const Task1 t = task1<S>(tid);
@@ -239,41 +244,39 @@ __global__ void __launch_bounds__(inner_threads<S>()) tern_inner(uint32_t *buf, 
     }
   }
   __syncthreads();
+  if (tid < S::TASK2) p2_load<S>(V, t2, f2);
+  __syncthreads();
+}
+
+template <class S>
+__global__ void __launch_bounds__(inner_threads<S>(), inner_blocks<S>()) tern_inner(uint32_t *buf, uint64_t job_words,
+                                                                                   TernJobs jobs) {
+  extern __shared__ uint32_t V[];
+  constexpr int NT = inner_threads<S>();
+  const int tid = threadIdx.x;
+  uint32_t *x = buf + uint64_t(blockIdx.z) * job_words +
+                (uint64_t(blockIdx.y) * gridDim.x + blockIdx.x) * tern_element(S::L);
+  const uint32_t *cs = jobs.consts[blockIdx.z] + uint64_t(blockIdx.x) * kLeafWords * S::LEAVES;
   const Task2 t2 = task2<S>(tid);
+  uint32_t next[kLeafWords] = {};
   {
     G4 f[3][S::G];
-    if (tid < S::TASK2) p2_load<S>(V, t2, f);
-    __syncthreads();
-    if (tid < S::TASK2) {
-      if constexpr (CONSTS) {
+    inner_forward<S, NT>(x, V, tid, t2, f);
+    if (tid < S::LEAVES) {
 #pragma unroll
-        for (int q = 0; q < 3; q++)
-#pragma unroll
-          for (int c = 0; c < S::G; c++) fwd_store<S::LP>(V + (t2.group * 3 + q) * S::ES, t2.r + 9 * c, f[q][c]);
-      } else {
-        p2_store<S>(V, t2, f);
-      }
+      for (int j = 0; j < kLeafWords; j++) next[j] = __ldg(&cs[j * S::LEAVES + tid]);
     }
+    if (tid < S::TASK2) p2_store<S>(V, t2, f);
   }
   __syncthreads();
-  if constexpr (CONSTS) {
-    uint32_t *o = consts_out + uint64_t(blockIdx.x) * kLeafWords * S::LEAVES;
-    for (int i = tid; i < S::LEAVES; i += NT) {
-      // a warp's evaluations are (nearly) one: no divergence between its cases
-      const int ev = i / S::NE, q = i / (2 * S::R1) % 3, group = i % (2 * S::R1);
-      uint32_t w[kLeafWords];
-      leaf_consts<S>(V + (group * 3 + q) * S::ES, ev, w);
-      const int id = leaf_id<S>(group, q, ev);
-#pragma unroll
-      for (int j = 0; j < kLeafWords; j++) o[j * S::LEAVES + id] = w[j];
-    }
-    return;
-  }
-  const uint32_t *cs = jobs.consts[blockIdx.z] + uint64_t(blockIdx.x) * kLeafWords * S::LEAVES;
+  // the next product's constants are on their way while this one is computed
   for (int i = tid; i < S::LEAVES; i += NT) {
     uint32_t v[18], w[kLeafWords];
 #pragma unroll
-    for (int j = 0; j < kLeafWords; j++) w[j] = __ldg(&cs[j * S::LEAVES + i]);
+    for (int j = 0; j < kLeafWords; j++) {
+      w[j] = next[j];
+      if (i + NT < S::LEAVES) next[j] = __ldg(&cs[j * S::LEAVES + i + NT]);
+    }
 #pragma unroll
     for (int j = 0; j < 18; j++) v[j] = V[j * S::SL + i];
     leaf9(v, w);
@@ -299,7 +302,48 @@ __global__ void __launch_bounds__(inner_threads<S>()) tern_inner(uint32_t *buf, 
     }
   }
   __syncthreads();
-  if (tid < S::TASK0) p6<S>(V, x, tid);
+  for (int i = tid; i < S::TASK0; i += NT) p6<S>(V, x, i);
+}
+
+// The leaf constants of a point of the transform of `a`.
+template <class S>
+__global__ void __launch_bounds__(192) tern_consts(const uint32_t *buf, uint32_t *consts) {
+  extern __shared__ uint32_t V[];
+  const int tid = threadIdx.x;
+  const Task2 t2 = task2<S>(tid);
+  {
+    G4 f[3][S::G];
+    inner_forward<S, 192>(buf + uint64_t(blockIdx.x) * tern_element(S::L), V, tid, t2, f);
+    if (tid < S::TASK2) {
+#pragma unroll
+      for (int q = 0; q < 3; q++)
+#pragma unroll
+        for (int c = 0; c < S::G; c++) fwd_store<S::LP>(V + (t2.group * 3 + q) * S::ES, t2.r + 9 * c, f[q][c]);
+    }
+  }
+  __syncthreads();
+  uint32_t *o = consts + uint64_t(blockIdx.x) * kLeafWords * S::LEAVES, *D = V + S::BASE;
+#pragma unroll 1
+  for (int h = 0; h < S::E / 5; h++) {
+    for (int i = tid; i < S::NE * 53; i += 192) {
+      const int el = i / 53, d = i % 53;
+      const G4 t = const_top<S>(V + el * S::ES, h, d - 26);
+      D[el * S::DIAGS + d] = t.a;
+      D[el * S::DIAGS + 53 + d] = t.b;
+    }
+    __syncthreads();
+    for (int i = tid; i < 5 * S::NE; i += 192) {
+      // a warp's evaluations are (nearly) one: little divergence between its cases
+      const int e1 = i / S::NE, q = i / (2 * S::R1) % 3, group = i % (2 * S::R1);
+      const uint32_t *d = D + (group * 3 + q) * S::DIAGS;
+      uint32_t w[kLeafWords];
+      leaf_consts(Diag{d, d + 53}, e1, w);
+      const int id = leaf_id<S>(group, q, 5 * h + e1);
+#pragma unroll
+      for (int j = 0; j < kLeafWords; j++) o[j * S::LEAVES + id] = w[j];
+    }
+    __syncthreads();
+  }
 }
 
 // A thread per coefficient: the word groups' coefficients of a warp are each
@@ -325,14 +369,16 @@ uint64_t group_words(int e) {
   return uint64_t(tern_points(s)) * tern_element(s.L);
 }
 
+template <typename F>
+int set_smem(F fn, int bytes) {
+  const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess) return CUOT_OK;
+  cudaGetLastError();
+  return fail(CUOT_ECUDA, "QC shared-memory attribute failed: %s", cudaGetErrorString(e));
+}
 template <int L, PassKind KIND>
 int pass27(const PassArgs &a, int njobs, cudaStream_t st) {
-  const cudaError_t e =
-      cudaFuncSetAttribute(tern_pass27<L, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, kExchangeBytes);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    return fail(CUOT_ECUDA, "QC shared-memory attribute failed: %s", cudaGetErrorString(e));
-  }
+  CUOT_TRY(set_smem(tern_pass27<L, KIND>, kExchangeBytes));
   const dim3 grid(tern_points(tern_shape(a.e)) / 27, (a.W * tern_block(L) + 31) / 32, njobs);
   tern_pass27<L, KIND><<<grid, 288, kExchangeBytes, st>>>(a);
   return CUOT_OK;
@@ -384,28 +430,35 @@ int forward(int e, PassKind kind, const TernJobs &jobs, uint32_t *half[2], uint6
   return CUOT_OK;
 }
 
-template <class S, bool CONSTS>
-int inner_launch(int P, uint32_t *buf, uint64_t job_words, const TernJobs &jobs, int njobs, uint32_t *consts_out,
-                 cudaStream_t st) {
-  const int smem = S::WORDS * 4;
-  const cudaError_t e = cudaFuncSetAttribute(tern_inner<S, CONSTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    return fail(CUOT_ECUDA, "QC shared-memory attribute failed: %s", cudaGetErrorString(e));
-  }
-  tern_inner<S, CONSTS><<<dim3(P, CONSTS ? 1 : 4, njobs), inner_threads<S>(), smem, st>>>(buf, job_words, jobs,
-                                                                                       consts_out);
+template <class S>
+int inner_launch(int P, uint32_t *buf, uint64_t job_words, const TernJobs &jobs, int njobs, cudaStream_t st) {
+  CUOT_TRY(set_smem(tern_inner<S>, S::WORDS * 4));
+  tern_inner<S><<<dim3(P, 4, njobs), inner_threads<S>(), S::WORDS * 4, st>>>(buf, job_words, jobs);
   return CUOT_OK;
 }
-template <bool CONSTS>
-int inner(const TernShape &s, uint32_t *buf, uint64_t job_words, const TernJobs &jobs, int njobs, uint32_t *consts_out,
-          cudaStream_t st) {
+template <class S>
+int consts_launch(int P, const uint32_t *buf, uint32_t *consts, cudaStream_t st) {
+  constexpr int smem = (S::BASE + S::NE * S::DIAGS) * 4;
+  CUOT_TRY(set_smem(tern_consts<S>, smem));
+  tern_consts<S><<<P, 192, smem, st>>>(buf, consts);
+  return CUOT_OK;
+}
+int inner(const TernShape &s, uint32_t *buf, uint64_t job_words, const TernJobs &jobs, int njobs, cudaStream_t st) {
   const int P = tern_points(s);
   switch (s.L) {
-    case 243: return inner_launch<Inner<243, 27>, CONSTS>(P, buf, job_words, jobs, njobs, consts_out, st);
-    case 729: return inner_launch<Inner<729, 27>, CONSTS>(P, buf, job_words, jobs, njobs, consts_out, st);
-    case 1458: return inner_launch<Inner<1458, 54>, CONSTS>(P, buf, job_words, jobs, njobs, consts_out, st);
-    default: return inner_launch<Inner<2187, 81>, CONSTS>(P, buf, job_words, jobs, njobs, consts_out, st);
+    case 243: return inner_launch<Inner<243, 27>>(P, buf, job_words, jobs, njobs, st);
+    case 729: return inner_launch<Inner<729, 27>>(P, buf, job_words, jobs, njobs, st);
+    case 1458: return inner_launch<Inner<1458, 54>>(P, buf, job_words, jobs, njobs, st);
+    default: return inner_launch<Inner<2187, 81>>(P, buf, job_words, jobs, njobs, st);
+  }
+}
+int consts(const TernShape &s, const uint32_t *buf, uint32_t *out, cudaStream_t st) {
+  const int P = tern_points(s);
+  switch (s.L) {
+    case 243: return consts_launch<Inner<243, 27>>(P, buf, out, st);
+    case 729: return consts_launch<Inner<729, 27>>(P, buf, out, st);
+    case 1458: return consts_launch<Inner<1458, 54>>(P, buf, out, st);
+    default: return consts_launch<Inner<2187, 81>>(P, buf, out, st);
   }
 }
 
@@ -427,7 +480,7 @@ int tern_build_ahat(int e, const uint64_t *a_d, void *scratch, void *ahat, cudaS
   jobs.in[0] = reinterpret_cast<const uint32_t *>(a_d);
   int at = 0;
   CUOT_TRY(forward(e, kFirstBits, jobs, half, 0, 1, &at, st));
-  CUOT_TRY(inner<true>(tern_shape(e), half[at], 0, jobs, 1, static_cast<uint32_t *>(ahat), st));
+  CUOT_TRY(consts(tern_shape(e), half[at], static_cast<uint32_t *>(ahat), st));
   return launch_status(1 + tern_passes(tern_shape(e).m));
 }
 
@@ -446,12 +499,13 @@ int tern_dual(int e, const TernJob *job, int njobs, void *scratch, cudaStream_t 
   }
   int at = 0;
   CUOT_TRY(forward(e, kFirst, jobs, half, job_words, njobs, &at, st));
-  CUOT_TRY(inner<false>(s, half[at], job_words, jobs, njobs, nullptr, st));
+  CUOT_TRY(inner(s, half[at], job_words, jobs, njobs, st));
   PassArgs a{e, 0, 4, nullptr, nullptr, job_words, jobs};
   for (a.pass = passes - 1; a.pass >= 0; a.pass--, at ^= 1) {
     a.src = half[at];
     a.dst = half[at ^ 1];
-    CUOT_TRY(pass(a, a.pass ? kInverse : kLastInverse, njobs, st));
+    // a single coset's pieces (y^m = 1) need no rotation in the end
+    CUOT_TRY(pass(a, a.pass || s.cosets == 1 ? kInverse : kLastInverse, njobs, st));
   }
   const uint32_t *buf = half[at];
   const dim3 grid((1u << e) / 256, 1, njobs);

@@ -289,7 +289,10 @@ struct Inner {
   // 16, so that a warp of consecutive groups (2 R1 of them) and residues
   // writes distinct banks.
   static constexpr int SL = LEAVES + ((9 - LEAVES % 16) + 16) % 16;
-  static constexpr int ES = 4 * LP_ + 1;       // words of a working copy, odd for the banks of consecutive groups
+  // Words of a working copy: its four blocks, padded so that consecutive
+  // elements lie (about) Lp / 3 banks apart, as a warp of radix-R1 butterflies
+  // wants them, and an odd number, as one of radix-3 butterflies does.
+  static constexpr int ES = LP_ == 27 ? 137 : LP_ == 54 ? 243 : 347;
   static constexpr int BASE = NE * ES;
   // Steps 0 and 6: a thread takes one coefficient p < Lp of CH consecutive pieces.
   static constexpr int CH = LP_ == 27 ? 3 : LP_ == 54 ? 6 : 9;
@@ -297,6 +300,7 @@ struct Inner {
   // Word of coefficient p of piece i in a part of an R_L element.
   TERN_HD static constexpr int word(int i, int p) { return i / (T / 9) * tern_block(L_) + i % (T / 9) * LP_ + p; }
   static constexpr int WORDS = 18 * SL > BASE ? 18 * SL : BASE;
+  static constexpr int DIAGS = 2 * 53;         // words of a 27 x 27 matrix's diagonals
   static_assert(R1 == 9 || R1 == 3, "inner passes");
 };
 
@@ -542,22 +546,52 @@ TERN_HD void p6(const uint32_t *V, uint32_t *x, int id) {
 
 // ---- leaves ----------------------------------------------------------------------
 // Constants of a 9 x 9 product: for each of its five 3 x 3 Toeplitz products
-// the five diagonals c = c0 + c1 w, as bits c0, c1, c0 ^ c1 (mask j = (e2 5 +
-// diagonal) 3 + {0, 1, 2}).  Mask j is bit 8 (j % 4) + 7 - (j % 32) / 4 of word
-// j / 32: after a shift by (j % 32) / 4 it is the top bit of a byte, which one
-// byte permute spreads over a word.
+// the five diagonals c = c0 + c1 w, as bits c0, c1, c0 ^ c1: bit j % 32 of word
+// j / 32, j = (e2 5 + diagonal) 3 + {0, 1, 2}.
 constexpr int kLeafMasks = 75, kLeafWords = 3;
-TERN_HD uint32_t leaf_mask(const uint32_t (&w)[kLeafWords], int j) {  // j: constant after unrolling
-  const uint32_t x = w[j / 32] << ((j % 32) / 4);
+
+// (a, b) of the N pairs o += c v, c of bits j, j + 1, j + 2.  On the device the
+// bits become predicates of the XORs (one operation each).
+template <int N>
+TERN_HD void leaf_diagonal(const uint32_t (&w)[kLeafWords], int j, const G4 *v0, G4 *o0) {
 #ifdef __CUDA_ARCH__
-  uint32_t m;  // selector bit 3 replicates the byte's sign (__byte_perm ignores that bit)
-  asm("prmt.b32 %0, %1, 0, %2;" : "=r"(m) : "r"(x), "r"(0x8888u + 0x1111u * uint32_t(j % 4)));
-  return m;
+  if constexpr (N == 1)
+    asm("{ .reg .pred p0, p1, p2; .reg .u32 t;\n"
+        "and.b32 t, %4, %7; setp.ne.u32 p0, t, 0; and.b32 t, %5, %8; setp.ne.u32 p1, t, 0;"
+        "and.b32 t, %6, %9; setp.ne.u32 p2, t, 0;\n"
+        "@p0 xor.b32 %0, %0, %2; @p1 xor.b32 %0, %0, %3; @p1 xor.b32 %1, %1, %2; @p2 xor.b32 %1, %1, %3; }"
+        : "+r"(o0[0].a), "+r"(o0[0].b)
+        : "r"(v0[0].a), "r"(v0[0].b), "r"(w[j / 32]), "r"(w[(j + 1) / 32]), "r"(w[(j + 2) / 32]),
+          "r"(1u << j % 32), "r"(1u << (j + 1) % 32), "r"(1u << (j + 2) % 32));
+  else if constexpr (N == 2)
+    asm("{ .reg .pred p0, p1, p2; .reg .u32 t;\n"
+        "and.b32 t, %8, %11; setp.ne.u32 p0, t, 0; and.b32 t, %9, %12; setp.ne.u32 p1, t, 0;"
+        "and.b32 t, %10, %13; setp.ne.u32 p2, t, 0;\n"
+        "@p0 xor.b32 %0, %0, %4; @p1 xor.b32 %0, %0, %5; @p1 xor.b32 %1, %1, %4; @p2 xor.b32 %1, %1, %5;\n"
+        "@p0 xor.b32 %2, %2, %6; @p1 xor.b32 %2, %2, %7; @p1 xor.b32 %3, %3, %6; @p2 xor.b32 %3, %3, %7; }"
+        : "+r"(o0[0].a), "+r"(o0[0].b), "+r"(o0[1].a), "+r"(o0[1].b)
+        : "r"(v0[0].a), "r"(v0[0].b), "r"(v0[1].a), "r"(v0[1].b), "r"(w[j / 32]), "r"(w[(j + 1) / 32]),
+          "r"(w[(j + 2) / 32]), "r"(1u << j % 32), "r"(1u << (j + 1) % 32), "r"(1u << (j + 2) % 32));
+  else
+    asm("{ .reg .pred p0, p1, p2; .reg .u32 t;\n"
+        "and.b32 t, %12, %15; setp.ne.u32 p0, t, 0; and.b32 t, %13, %16; setp.ne.u32 p1, t, 0;"
+        "and.b32 t, %14, %17; setp.ne.u32 p2, t, 0;\n"
+        "@p0 xor.b32 %0, %0, %6; @p1 xor.b32 %0, %0, %7; @p1 xor.b32 %1, %1, %6; @p2 xor.b32 %1, %1, %7;\n"
+        "@p0 xor.b32 %2, %2, %8; @p1 xor.b32 %2, %2, %9; @p1 xor.b32 %3, %3, %8; @p2 xor.b32 %3, %3, %9;\n"
+        "@p0 xor.b32 %4, %4, %10; @p1 xor.b32 %4, %4, %11; @p1 xor.b32 %5, %5, %10; @p2 xor.b32 %5, %5, %11; }"
+        : "+r"(o0[0].a), "+r"(o0[0].b), "+r"(o0[1].a), "+r"(o0[1].b), "+r"(o0[2].a), "+r"(o0[2].b)
+        : "r"(v0[0].a), "r"(v0[0].b), "r"(v0[1].a), "r"(v0[1].b), "r"(v0[2].a), "r"(v0[2].b), "r"(w[j / 32]),
+          "r"(w[(j + 1) / 32]), "r"(w[(j + 2) / 32]), "r"(1u << j % 32), "r"(1u << (j + 1) % 32),
+          "r"(1u << (j + 2) % 32));
 #else
-  return (x >> (8 * (j % 4) + 7)) & 1u ? ~0u : 0u;
+  uint32_t m[3];
+  for (int k = 0; k < 3; k++) m[k] = (w[(j + k) / 32] >> (j + k) % 32) & 1u ? ~0u : 0u;
+  for (int n = 0; n < N; n++) {
+    o0[n].a ^= (v0[n].a & m[0]) ^ (v0[n].b & m[1]);
+    o0[n].b ^= (v0[n].a & m[1]) ^ (v0[n].b & m[2]);
+  }
 #endif
 }
-constexpr int leaf_mask_bit(int j) { return 8 * (j % 4) + 7 - (j % 32) / 4; }
 
 // v (nine pairs) <- Toeplitz product.
 TERN_HD void leaf9(uint32_t (&v)[18], const uint32_t (&w)[kLeafWords]) {
@@ -571,22 +605,14 @@ TERN_HD void leaf9(uint32_t (&v)[18], const uint32_t (&w)[kLeafWords]) {
   }
 #pragma unroll
   for (int h = 0; h < 5; h++) {
-    uint32_t m[15];
+    // diagonal d: output r takes input r + 2 - d
 #pragma unroll
-    for (int j = 0; j < 15; j++) m[j] = leaf_mask(w, 15 * h + j);
-#pragma unroll
-    for (int r = 0; r < 3; r++) {
-      uint32_t a = 0, b = 0;
-#pragma unroll
-      for (int j = 0; j < 3; j++) {
-        const int d = r - j + 2;
-        a ^= e[h][j].a & m[3 * d];
-        a ^= e[h][j].b & m[3 * d + 1];
-        b ^= e[h][j].a & m[3 * d + 1];
-        b ^= e[h][j].b & m[3 * d + 2];
-      }
-      q[h][r] = G4{a, b};
-    }
+    for (int r = 0; r < 3; r++) q[h][r] = G4{0u, 0u};
+    leaf_diagonal<1>(w, 15 * h, &e[h][2], &q[h][0]);
+    leaf_diagonal<2>(w, 15 * h + 3, &e[h][1], &q[h][0]);
+    leaf_diagonal<3>(w, 15 * h + 6, &e[h][0], &q[h][0]);
+    leaf_diagonal<2>(w, 15 * h + 9, &e[h][0], &q[h][1]);
+    leaf_diagonal<1>(w, 15 * h + 12, &e[h][0], &q[h][2]);
   }
 #pragma unroll
   for (int i = 0; i < 3; i++) {
@@ -615,40 +641,32 @@ TERN_HD G4 toom_const(int e, G4 tm2, G4 tm1, G4 t0, G4 t1, G4 t2) {
   if (e == 3) return g_add(g_add(g_w1(tm1), g_w2(t0)), t1);
   return g_add(t2, tm1);
 }
+// Diagonal d (|d| <= 26) of evaluation h's 27 x 27 Toeplitz matrix, from the
+// element's working copy at V.
 template <class S>
-TERN_HD G4 const_top(const uint32_t *V, int h, int d) {  // diagonal of the split above the last two (27 x 27)
+TERN_HD G4 const_top(const uint32_t *V, int h, int d) {
   if constexpr (S::G == 3) {
     return fwd_load<S::LP>(V, d);
   } else if constexpr (S::G == 6) {
-    G4 t = h < 2 ? fwd_load<S::LP>(V, h == 0 ? d - 27 : d + 27) : G4{0u, 0u};
-    return g_add(t, fwd_load<S::LP>(V, d));
+    const G4 t = fwd_load<S::LP>(V, d);
+    return h < 2 ? g_add(t, fwd_load<S::LP>(V, h == 0 ? d - 27 : d + 27)) : t;
   } else {
-    // |d| <= 26; only the diagonals that evaluation h uses are read
-    const G4 z{0u, 0u};
-    const G4 tm2 = h == 0 ? fwd_load<S::LP>(V, d - 54) : z;
-    const G4 tm1 = h != 0 ? fwd_load<S::LP>(V, d - 27) : z;
-    const G4 t0 = h >= 1 && h <= 3 ? fwd_load<S::LP>(V, d) : z;
-    const G4 t1 = h != 4 ? fwd_load<S::LP>(V, d + 27) : z;
-    const G4 t2 = h == 4 ? fwd_load<S::LP>(V, d + 54) : z;
-    return toom_const(h, tm2, tm1, t0, t1, t2);
+    return toom_const(h, fwd_load<S::LP>(V, d - 54), fwd_load<S::LP>(V, d - 27), fwd_load<S::LP>(V, d),
+                      fwd_load<S::LP>(V, d + 27), fwd_load<S::LP>(V, d + 54));
   }
 }
-// Leaf words of evaluation ev = 5 h + e1 (e1 alone for Lp = 27) of the element
-// at V.  Word bits come from bit 0 of the data words.
-template <class S>
-TERN_HD void leaf_consts(const uint32_t *V, int ev, uint32_t (&w)[kLeafWords]) {
-  const int h = ev / 5, e1 = ev % 5;
+// Leaf words of evaluation e1 of the 27 x 27 matrix whose diagonals d are at
+// t[d + 26].  Word bits come from bit 0 of the data words.
+struct Diag {
+  const uint32_t *a, *b;  // words of diagonal -26
+};
+TERN_HD void leaf_consts(const Diag &t, int e1, uint32_t (&w)[kLeafWords]) {
   G4 s1[17];
 #pragma unroll
   for (int i = 0; i < 17; i++) {
-    const int d = i - 8;
-    const G4 z{0u, 0u};
-    const G4 tm2 = e1 == 0 ? const_top<S>(V, h, d - 18) : z;
-    const G4 tm1 = e1 != 0 ? const_top<S>(V, h, d - 9) : z;
-    const G4 t0 = e1 >= 1 && e1 <= 3 ? const_top<S>(V, h, d) : z;
-    const G4 t1 = e1 != 4 ? const_top<S>(V, h, d + 9) : z;
-    const G4 t2 = e1 == 4 ? const_top<S>(V, h, d + 18) : z;
-    s1[i] = toom_const(e1, tm2, tm1, t0, t1, t2);
+    const int d = i - 8 + 26;
+    s1[i] = toom_const(e1, G4{t.a[e1 ? d : d - 18], t.b[e1 ? d : d - 18]}, G4{t.a[d - 9], t.b[d - 9]}, G4{t.a[d], t.b[d]},
+                       G4{t.a[d + 9], t.b[d + 9]}, G4{t.a[d + (e1 < 4 ? 0 : 18)], t.b[d + (e1 < 4 ? 0 : 18)]});
   }
   w[0] = w[1] = w[2] = 0;
 #pragma unroll
@@ -658,9 +676,9 @@ TERN_HD void leaf_consts(const uint32_t *V, int ev, uint32_t (&w)[kLeafWords]) {
       const int d = i - 2 + 8;
       const G4 c = toom_const(e2, s1[d - 6], s1[d - 3], s1[d], s1[d + 3], s1[d + 6]);
       const int j = (5 * e2 + i) * 3;
-      w[j / 32] |= (c.a & 1u) << leaf_mask_bit(j);
-      w[(j + 1) / 32] |= (c.b & 1u) << leaf_mask_bit(j + 1);
-      w[(j + 2) / 32] |= ((c.a ^ c.b) & 1u) << leaf_mask_bit(j + 2);
+      w[j / 32] |= (c.a & 1u) << j % 32;
+      w[(j + 1) / 32] |= (c.b & 1u) << (j + 1) % 32;
+      w[(j + 2) / 32] |= ((c.a ^ c.b) & 1u) << (j + 2) % 32;
     }
 }
 

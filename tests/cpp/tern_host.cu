@@ -134,10 +134,18 @@ static void point_consts(const uint32_t *x, uint32_t *consts) {  // [word][leaf]
         fwd_store<S::LP>(V.data() + (t.group * 3 + q) * S::ES, t.r + 9 * c, f2[id][q * S::G + c]);
   }
   for (int el = 0; el < S::NE; el++)
-    for (int ev = 0; ev < S::E; ev++) {
-      uint32_t w[kLeafWords];
-      leaf_consts<S>(V.data() + el * S::ES, ev, w);
-      for (int j = 0; j < kLeafWords; j++) consts[j * S::LEAVES + leaf_id<S>(el / 3, el % 3, ev)] = w[j];
+    for (int h = 0; h < S::E / 5; h++) {
+      uint32_t diag[S::DIAGS];
+      for (int d = -26; d <= 26; d++) {
+        const G4 t = const_top<S>(V.data() + el * S::ES, h, d);
+        diag[d + 26] = t.a;
+        diag[53 + d + 26] = t.b;
+      }
+      for (int e1 = 0; e1 < 5; e1++) {
+        uint32_t w[kLeafWords];
+        leaf_consts(Diag{diag, diag + 53}, e1, w);
+        for (int j = 0; j < kLeafWords; j++) consts[j * S::LEAVES + leaf_id<S>(el / 3, el % 3, 5 * h + e1)] = w[j];
+      }
     }
 }
 
