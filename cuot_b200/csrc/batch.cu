@@ -107,8 +107,14 @@ struct LpnBatchArgs {
   const uint32_t *t0;
 };
 
-// Two CTAs per SM: a dual-role group keeps both roles' accumulators live.
-__global__ void __launch_bounds__(kLpnThreads, 2) lpn_batch_kernel(LpnBatchArgs b) {
+// The interleaved kk of every instance with d = 10 (blockIdx.y: job).
+__global__ void __launch_bounds__(256) lpn_interleave_batch(const LpnArgs *jobs) {
+  const LpnArgs &a = jobs[blockIdx.y];
+  if (!a.kk12) return;
+  for (int64_t j = int64_t(blockIdx.x) * 256 + threadIdx.x; j < a.k; j += int64_t(gridDim.x) * 256) lpn_interleave(a, j);
+}
+
+__global__ void __launch_bounds__(kLpnThreads, 3) lpn_batch_kernel(LpnBatchArgs b) {
   extern __shared__ __align__(16) uint32_t smem_tab[];
   __shared__ __align__(16) LpnArgs s_job;
   __shared__ uint32_t s_task;
@@ -126,10 +132,16 @@ __global__ void __launch_bounds__(kLpnThreads, 2) lpn_batch_kernel(LpnBatchArgs 
       reinterpret_cast<uint32_t *>(&s_job)[i] = src[i];
     __syncthreads();
     const LpnArgs &a = s_job;  // every job holds both roles (make_lpn_job)
-    for (int64_t w = tk.w0 + threadIdx.x; w < tk.w1; w += blockDim.x) {
+    int64_t first = tk.w0;
+    if (a.kk12) {
+      const int64_t end = a.g0 + (tk.w1 < a.ngroups ? tk.w1 : a.ngroups);
+      for (int64_t g = a.g0 + tk.w0 + 6 * (threadIdx.x >> 5); g < end; g += 6 * (kLpnThreads / 32))
+        lpn_split6<kInterleaved>(a, T, g, end);
+      first = tk.w0 > a.ngroups ? tk.w0 : a.ngroups;
+    }
+    for (int64_t w = first + threadIdx.x; w < tk.w1; w += blockDim.x) {
       if (w < a.ngroups) {
-        if (a.d == 10) lpn_group4<10, true>(a, T, a.g0 + w);
-        else lpn_group4_dyn(a, T, a.g0 + w);
+        lpn_group4_dyn(a, T, a.g0 + w);
       } else {
         lpn_row1(a, T, a.j0 + (w - a.ngroups));
       }
@@ -197,6 +209,8 @@ struct cuot_batch {
   // LPN: one job per Ferret instance, both roles
   LpnBatchArgs lpn{};
   int lpn_grid = 0;
+  int lpn_jobs = 0;
+  int64_t lpn_kmax = 0;  // largest k of the jobs with an interleaved kk (0: none)
   unsigned int *counters = nullptr;  // [kCounters]
   // SOT: sizes, largest first, grouped into lanes (qc_lane) that run side by side
   std::vector<SotClass> classes;
@@ -309,8 +323,12 @@ int select_launch(cuot_batch *b, cudaStream_t st) {
 
 int lpn_launch(cuot_batch *b, cudaStream_t st) {
   if (!b->lpn.ntasks) return 0;
+  if (b->lpn_kmax) {
+    const unsigned gx = unsigned(std::min<int64_t>((b->lpn_kmax + 255) / 256, 592));
+    lpn_interleave_batch<<<dim3(gx, b->lpn_jobs), 256, 0, st>>>(b->lpn.jobs);
+  }
   lpn_batch_kernel<<<b->lpn_grid, kLpnThreads, kTableBytes, st>>>(b->lpn);
-  return 1;
+  return b->lpn_kmax ? 2 : 1;
 }
 
 // Records completion group g's event on `st`: under stream capture as an
@@ -534,13 +552,26 @@ int cuot_batch_create(cuot_ctx *ctx, const cuot_batch_item *items, int count,
   if (b->nsel && (st = upload(b, &b->sel_d, sel))) return cleanup(st);
 
   // ---- LPN: one job per Ferret item (both roles), tasks of rows_per_task rows
-  const int64_t rows_per_task = b->cfg.lpn_rows_per_task > 0 ? (b->cfg.lpn_rows_per_task + 3) / 4 * 4 : 65536;
+  // (default: about four tasks per CTA, whole rounds of a CTA, at most 65,536
+  // rows; 65,536 for every batch left a 16-session one with 33 tasks for the
+  // resident CTAs, LPN 1.12 ms against 0.2)
+  int64_t lpn_rows = 0;
+  for (int i = 0; i < count; i++)
+    if (items[i].kind == CUOT_KIND_FERRET) lpn_rows += int64_t(items[i].t << items[i].h);
+  constexpr int64_t kRound = 4 * 4 * 6 * (kLpnThreads / 32);  // four rounds of a CTA
+  const int64_t fill = lpn_rows / (int64_t(sms) * per_sm * 4) / kRound * kRound;
+  const int64_t rows_per_task = b->cfg.lpn_rows_per_task > 0 ? (b->cfg.lpn_rows_per_task + 3) / 4 * 4
+                                                             : std::min<int64_t>(std::max(fill, kRound), 65536);
   std::vector<LpnArgs> jobs;
   std::vector<LpnTask> ltasks;
   for (int i = 0; i < count; i++) {
     const cuot_batch_item &it = items[i];
     if (it.kind != CUOT_KIND_FERRET) continue;
-    const LpnArgs a = make_lpn_job(it, ctx->t0_d);
+    LpnArgs a = make_lpn_job(it, ctx->t0_d);
+    if (a.d == 10) {
+      if ((st = balloc(b, &a.kk12, uint64_t(a.k) * 32))) return cleanup(st);
+      b->lpn_kmax = std::max(b->lpn_kmax, a.k);
+    }
     const uint32_t j = uint32_t(jobs.size());
     jobs.push_back(a);
     const int64_t total = a.ngroups + a.ntail, chunk = rows_per_task / 4;
@@ -551,6 +582,7 @@ int cuot_batch_create(cuot_ctx *ctx, const cuot_batch_item *items, int count,
     LpnTask *ltd = nullptr;
     if ((st = upload(b, &jd, jobs)) || (st = upload(b, &ltd, ltasks))) return cleanup(st);
     b->lpn = LpnBatchArgs{jd, ltd, uint32_t(ltasks.size()), b->counters + 4, ctx->t0_d};
+    b->lpn_jobs = int(jobs.size());
     b->lpn_grid = int(std::min<uint64_t>(uint64_t(sms) * per_sm, ltasks.size()));
   }
 

@@ -14,8 +14,7 @@
 
 namespace cuot {
 
-// D = 0: any d (a.d); D > 0: d = D.  DUAL: both roles (a.kk2 / a.e2 set).
-template <int D, bool DUAL>
+// Any d (a.d), both roles when a.kk2 is set: a thread per 4-row group.
 __global__ void __launch_bounds__(kLpnThreads) lpn_kernel(LpnArgs a) {
   extern __shared__ __align__(16) uint32_t smem_tab[];
   stage_table(smem_tab, a.t0);
@@ -24,13 +23,27 @@ __global__ void __launch_bounds__(kLpnThreads) lpn_kernel(LpnArgs a) {
   const int64_t total = a.ngroups + a.ntail;
   for (int64_t w = int64_t(blockIdx.x) * kLpnThreads + threadIdx.x; w < total;
        w += int64_t(gridDim.x) * kLpnThreads) {
-    if (w < a.ngroups) {
-      if (D > 0) lpn_group4<(D > 0 ? D : 1), DUAL>(a, T, a.g0 + w);
-      else lpn_group4_dyn(a, T, a.g0 + w);
-    } else {
-      lpn_row1(a, T, a.j0 + (w - a.ngroups));
-    }
+    if (w < a.ngroups) lpn_group4_dyn(a, T, a.g0 + w);
+    else lpn_row1(a, T, a.j0 + (w - a.ngroups));
   }
+}
+
+// d = 10: five lanes per group (lpn_split6), persistent CTAs.
+template <LpnRoles ROLES>
+__global__ void __launch_bounds__(kLpnThreads, 3) lpn_split_kernel(LpnArgs a) {
+  extern __shared__ __align__(16) uint32_t smem_tab[];
+  stage_table(smem_tab, a.t0);
+  __syncthreads();
+  const TabRef T{reinterpret_cast<const char *>(smem_tab), uint32_t(threadIdx.x & 31) * 4u};
+  const int64_t warps = int64_t(gridDim.x) * (kLpnThreads / 32), end = a.g0 + a.ngroups;
+  const int64_t warp = int64_t(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+  for (int64_t g = a.g0 + 6 * warp; g < end; g += 6 * warps) lpn_split6<ROLES>(a, T, g, end);
+  if (blockIdx.x == gridDim.x - 1)
+    for (int64_t j = threadIdx.x; j < a.ntail; j += kLpnThreads) lpn_row1(a, T, a.j0 + j);
+}
+
+__global__ void __launch_bounds__(256) lpn_interleave_kernel(LpnArgs a) {
+  for (int64_t j = int64_t(blockIdx.x) * 256 + threadIdx.x; j < a.k; j += int64_t(gridDim.x) * 256) lpn_interleave(a, j);
 }
 
 // Plain in-place AES-128 ECB, two blocks per thread.
@@ -79,13 +92,46 @@ static int set_smem(F fn) {
   return CUOT_OK;
 }
 
-template <int D, bool DUAL>
-int launch_lpn(cuot_ctx *ctx, const LpnArgs &a, cudaStream_t st) {
-  CUOT_TRY(set_smem(lpn_kernel<D, DUAL>));
+int launch_any(cuot_ctx *ctx, const LpnArgs &a, cudaStream_t st) {
+  CUOT_TRY(set_smem(lpn_kernel));
   int grid = 1;
-  grid_for(ctx, (const void *)lpn_kernel<D, DUAL>, a.ngroups + a.ntail, &grid);
-  lpn_kernel<D, DUAL><<<grid, kLpnThreads, kTableBytes, st>>>(a);
+  grid_for(ctx, (const void *)lpn_kernel, a.ngroups + a.ntail, &grid);
+  lpn_kernel<<<grid, kLpnThreads, kTableBytes, st>>>(a);
   return launch_status();
+}
+
+template <LpnRoles ROLES>
+int launch_split(cuot_ctx *ctx, const LpnArgs &a, cudaStream_t st) {
+  CUOT_TRY(set_smem(lpn_split_kernel<ROLES>));
+  int per_sm = 0, sms = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lpn_split_kernel<ROLES>, kLpnThreads, kTableBytes);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+  const int64_t tasks = (a.ngroups + 5) / 6, cap = int64_t(per_sm < 1 ? 1 : per_sm) * sms;
+  lpn_split_kernel<ROLES><<<unsigned(tasks < 1 ? 1 : tasks < cap ? tasks : cap), kLpnThreads, kTableBytes, st>>>(a);
+  return launch_status();
+}
+
+// Both roles, d = 10.  From kInterleaveRows rows on, kk and kk2 are first copied
+// side by side into the context's scratch (470,016 rows 66.8 -> 58.6 us with the
+// copy, 10,485,760 rows 1197 -> 927; at 131,072 rows the 3 us that the gathers
+// would save are the copy's launch).  Not while `st` is captured: the arena may
+// neither grow then nor, as far as this call goes, stay where it is until the
+// graph runs.
+constexpr int64_t kInterleaveRows = 1 << 18;
+int launch_dual(cuot_ctx *ctx, LpnArgs a, cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (a.ngroups * 4 < kInterleaveRows || a.k > a.ngroups || cudaStreamIsCapturing(st, &cap) != cudaSuccess ||
+      cap != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return launch_split<kTwoRoles>(ctx, a, st);
+  }
+  void *scr = nullptr;
+  CUOT_TRY(scratch(ctx, uint64_t(a.k) * 32, &scr));
+  a.kk12 = static_cast<Blk *>(scr);
+  const int64_t grid = (a.k + 255) / 256;
+  lpn_interleave_kernel<<<unsigned(grid < 148 * 8 ? grid : 148 * 8), 256, 0, st>>>(a);
+  CUOT_TRY(launch_status());
+  return launch_split<kInterleaved>(ctx, a, st);
 }
 
 // Rows [row_lo, row_hi) of one task over [0, n) (lpn_f2.h:72-79), for one
@@ -123,8 +169,8 @@ int lpn_rows(cuot_ctx *ctx, const uint8_t seed[16], const cuot_block *kk_d, cons
   a.ntail = row_hi > a.j0 ? row_hi - a.j0 : 0;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const bool dual = kk2_d != nullptr;
-  if (d == 10) return dual ? launch_lpn<10, true>(ctx, a, st) : launch_lpn<10, false>(ctx, a, st);
-  return launch_lpn<0, false>(ctx, a, st);  // lpn_group4_dyn / lpn_row1 read a.kk2 themselves
+  if (d == 10) return dual ? launch_dual(ctx, a, st) : launch_split<kOneRole>(ctx, a, st);
+  return launch_any(ctx, a, st);
 }
 
 }  // namespace cuot

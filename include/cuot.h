@@ -401,7 +401,8 @@ typedef struct {
 typedef struct {
   int pprf_threads;        /* threads per tree CTA: 128 or 256 (0: 256) */
   int ctas_per_sm;         /* persistent PPRF/LPN grid: CTAs per SM (0: 3) */
-  int lpn_rows_per_task;   /* LPN work-queue granularity, multiple of 4 (0: 65536) */
+  int lpn_rows_per_task;   /* LPN work-queue granularity, multiple of 4 (0:
+                            from the batch's rows, at most 65536) */
   int qc_planes_per_pass;  /* planes per QC pass (0: 512 MiB of intermediate) */
   int use_graph;           /* capture into a CUDA graph on first run */
   int schedule;            /* CUOT_BATCH_SERIAL (0, default): every launch
