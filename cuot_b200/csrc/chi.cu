@@ -8,24 +8,30 @@
 // little-endian block is the coefficient of x^i), reduction polynomial
 // x^128 + x^7 + x^2 + x + 1 (emp-tool's gfmul).
 //
-// B200 has no carry-less multiply, so one CTA per tree turns the sum into a
-// polynomial evaluation with a single repeated multiplier:
-//   thread j (of 256) runs Horner over its leaves i = j + 256 q with the
-//   multiplier u = s^256:  P_j = sum_q v_{j+256q} u^q;
-//   then sum_j s^j P_j is folded in 8 levels of a binary tree (level l
-//   multiplies by s^(2^l)), and V = s * (that sum).
-// Multiplication by the fixed u uses byte tables in shared memory: T[k][b] =
-// u * (b x^(8k)), so u * x = XOR_k T[k][byte k of x] -- 16 conflict-light
-// 128-bit lookups per leaf instead of a 128 x 128 carry-less product.  The
-// squarings s^(2^l) spread bits (squaring is linear in characteristic 2);
-// the few general products (tree levels) are bit-serial.
+// B200 has no carry-less multiply, so one CTA per tree turns the sum into
+// polynomial evaluations with repeated multipliers:
+//   thread j (of 128) runs Horner over its leaves i = j + 128 q with the
+//   multiplier u = s^128:  P_j = sum_q v_{j+128q} u^q;
+//   warp w (of 4) runs Horner over P_{w+4q} with s^4, and warp 0 over the four
+//   results with s, the last product with s included.
+// The leaves' products use nibble tables of u in shared memory: u * x = XOR_k
+// T[k][nibble k of x], 32 lookups of 16 bytes.  Every entry is held eight
+// times, once per group of four banks, and a lane reads the copy of its own
+// group: four wavefronts per lookup, where 256-entry byte tables (16 lookups,
+// also 64 KiB) met about eleven, and an eighth of the entries to compute.  The
+// 132 products of the fold are a warp's each: lane l holds c x^(4l + b), b < 4,
+// for the multiplier c and adds those whose bits of x are set; four XOR
+// reductions over the warp give the product (bit-serial ones by single
+// threads, level by level, took as long as the leaves).
+// Bound by the lookups' wavefronts: 32 x 4 per 32 leaves and SM, 145 us for
+// 2,507 trees of depth 12.  Measured there 675 -> 196 us (64 trees of depth 10: 48 -> 13).
 #include "ctx.cuh"
 
 namespace cuot {
 namespace {
 
-constexpr int kChiThreads = 256;
-constexpr int kChiTableBytes = 16 * 256 * 16;
+constexpr int kChiThreads = 128;
+constexpr int kChiTableBytes = 32 * 16 * 8 * 16;  // [nibble][value][copy]
 
 struct U128 {
   uint64_t lo, hi;
@@ -43,19 +49,23 @@ __device__ __forceinline__ U128 mulx(U128 a) {
   const uint64_t c = a.hi >> 63;
   return U128{(a.lo << 1) ^ (c * 0x87ull), (a.hi << 1) | (a.lo >> 63)};
 }
-// general product: r = XOR_i a_i (b x^i), with b x^i advanced by one mulx per
-// bit, so the dependency chain is the short mulx and the accumulation
-// pipelines behind it
-__device__ U128 gmul(U128 a, U128 b) {
-  U128 r{0, 0}, bx = b;
-#pragma unroll 8
-  for (int i = 0; i < 128; i++) {
-    const uint64_t m = 0 - ((i < 64 ? a.lo >> i : a.hi >> (i - 64)) & 1);
-    r.lo ^= bx.lo & m;
-    r.hi ^= bx.hi & m;
-    bx = mulx(bx);
+// r3:r2:r1:r0 mod x^128 + x^7 + x^2 + x + 1 (the first fold spills at most 7 bits)
+__device__ __forceinline__ U128 reduce256(uint64_t r0, uint64_t r1, uint64_t r2, uint64_t r3) {
+#pragma unroll
+  for (int pass = 0; pass < 2; pass++) {
+    const uint64_t h0 = r2, h1 = r3;
+    r2 = r3 = 0;
+    r0 ^= h0 ^ (h0 << 1) ^ (h0 << 2) ^ (h0 << 7);
+    r1 ^= h1 ^ (h1 << 1) ^ (h1 << 2) ^ (h1 << 7) ^ (h0 >> 63) ^ (h0 >> 62) ^ (h0 >> 57);
+    r2 ^= (h1 >> 63) ^ (h1 >> 62) ^ (h1 >> 57);
   }
-  return r;
+  return U128{r0, r1};
+}
+// a * x^m, 0 <= m < 128
+__device__ __forceinline__ U128 mulxn(U128 a, int m) {
+  const int b = m & 63;
+  const uint64_t lo = a.lo << b, mid = (a.hi << b) | (b ? a.lo >> (64 - b) : 0), hi = b ? a.hi >> (64 - b) : 0;
+  return m < 64 ? reduce256(lo, mid, hi, 0) : reduce256(0, lo, mid, hi);
 }
 // bits i -> 2i of a 32-bit word
 __device__ __forceinline__ uint64_t spread32(uint32_t x) {
@@ -67,94 +77,113 @@ __device__ __forceinline__ uint64_t spread32(uint32_t x) {
   v = (v | (v << 1)) & 0x5555555555555555ull;
   return v;
 }
-// a^2: squaring is GF(2)-linear (bit i -> bit 2i), then the high 128 bits
-// are folded with x^128 = x^7 + x^2 + x + 1 (twice: the first fold spills
-// at most 7 bits)
-__device__ U128 gsqr(U128 a) {
-  uint64_t r0 = spread32(uint32_t(a.lo)), r1 = spread32(uint32_t(a.lo >> 32));
-  uint64_t r2 = spread32(uint32_t(a.hi)), r3 = spread32(uint32_t(a.hi >> 32));
-#pragma unroll
-  for (int pass = 0; pass < 2; pass++) {
-    const uint64_t h0 = r2, h1 = r3;
-    r2 = r3 = 0;
-    r0 ^= h0 ^ (h0 << 1) ^ (h0 << 2) ^ (h0 << 7);
-    r1 ^= h1 ^ (h1 << 1) ^ (h1 << 2) ^ (h1 << 7) ^ (h0 >> 63) ^ (h0 >> 62) ^ (h0 >> 57);
-    r2 ^= (h1 >> 63) ^ (h1 >> 62) ^ (h1 >> 57);
-  }
-  return U128{r0, r1};
+// a^2: squaring is GF(2)-linear (bit i -> bit 2i)
+__device__ __forceinline__ U128 gsqr(U128 a) {
+  return reduce256(spread32(uint32_t(a.lo)), spread32(uint32_t(a.lo >> 32)), spread32(uint32_t(a.hi)),
+                   spread32(uint32_t(a.hi >> 32)));
 }
 
-// u * x with the byte tables T (16 x 256 entries)
-__device__ __forceinline__ U128 tmul(const uint4 *__restrict__ T, const uint4 x) {
+// u * x with the nibble tables; T: this lane's copies.
+__device__ __forceinline__ U128 tmul(const char *T, const uint4 x) {
   uint4 r = make_uint4(0, 0, 0, 0);
   const uint32_t w[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-  for (int k = 0; k < 16; k++) {
-    const uint4 e = T[k * 256 + ((w[k >> 2] >> (8 * (k & 3))) & 255)];
+  for (int k = 0; k < 32; k++) {
+    const int sh = 4 * (k & 7);  // nibble at bits 7..10: its entry's offset
+    const uint32_t off = (sh > 7 ? w[k >> 3] >> (sh > 7 ? sh - 7 : 0) : w[k >> 3] << (sh > 7 ? 0 : 7 - sh)) & 0x780u;
+    const uint4 e = *reinterpret_cast<const uint4 *>(T + k * 2048 + off);
     r.x ^= e.x; r.y ^= e.y; r.z ^= e.z; r.w ^= e.w;
   }
   return u128(r);
 }
 
+// A warp's products with a fixed c: lane l holds c x^(4l), ..., c x^(4l + 3).
+struct WarpMul {
+  uint4 y[4];
+  __device__ __forceinline__ WarpMul(U128 c, int lane) {
+    U128 v = mulxn(c, 4 * lane);
+#pragma unroll
+    for (int b = 0; b < 4; b++) {
+      y[b] = to_u4(v);
+      v = mulx(v);
+    }
+  }
+  // c * x, x and the result in every lane
+  __device__ __forceinline__ uint4 operator()(uint4 x, int lane) const {
+    const uint32_t lo = lane & 8 ? x.y : x.x, hi = lane & 8 ? x.w : x.z;
+    const uint32_t n = (lane & 16 ? hi : lo) >> (4 * (lane & 7));
+    uint4 r = make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int b = 0; b < 4; b++) {
+      const uint32_t m = 0u - ((n >> b) & 1u);
+      r.x ^= y[b].x & m; r.y ^= y[b].y & m; r.z ^= y[b].z & m; r.w ^= y[b].w & m;
+    }
+    return make_uint4(__reduce_xor_sync(0xffffffffu, r.x), __reduce_xor_sync(0xffffffffu, r.y),
+                      __reduce_xor_sync(0xffffffffu, r.z), __reduce_xor_sync(0xffffffffu, r.w));
+  }
+};
+__device__ __forceinline__ uint4 xor4(uint4 a, uint4 b) {
+  return make_uint4(a.x ^ b.x, a.y ^ b.y, a.z ^ b.z, a.w ^ b.w);
+}
+
 __global__ void __launch_bounds__(kChiThreads) chi_sum_kernel(const uint4 *__restrict__ leaves, int h,
                                                               const uint4 *__restrict__ seeds,
                                                               uint4 *__restrict__ out) {
-  extern __shared__ uint4 T[];         // [16][256]: u * (b x^(8k))
-  __shared__ uint4 basis[128];         // u * x^m
-  __shared__ uint4 P[kChiThreads];     // per-thread partial sums, then the tree
-  __shared__ uint4 spow[9];            // s^(2^l), l = 0..8 (spow[8] = u)
-  const int tree = blockIdx.x;
-  const U128 s = u128(__ldg(&seeds[tree]));
-  if (threadIdx.x == 0) {
-    U128 c = s;
-    spow[0] = to_u4(c);
-    for (int l = 1; l <= 8; l++) {
-      c = gsqr(c);
-      spow[l] = to_u4(c);
-    }
-    U128 b = c;  // u * x^0
-    for (int m = 0; m < 128; m++) {
-      basis[m] = to_u4(b);
-      b = mulx(b);
-    }
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < 16 * 256; e += blockDim.x) {
-    const int k = e >> 8, byte = e & 255;
-    uint4 r = make_uint4(0, 0, 0, 0);
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-      if ((byte >> j) & 1) {
-        const uint4 v = basis[8 * k + j];
-        r.x ^= v.x; r.y ^= v.y; r.z ^= v.z; r.w ^= v.w;
-      }
-    }
-    T[e] = r;
-  }
-  __syncthreads();
-  // Horner over this thread's leaves j + 256 q, highest q first
-  const int64_t L = int64_t(1) << h;
+  extern __shared__ uint4 T[];       // [32][16][8]
+  __shared__ uint4 P[kChiThreads];   // u x^m, then the threads' partial sums
+  __shared__ uint4 R[4];
+  const int tree = blockIdx.x, j = threadIdx.x, lane = j & 31, warp = j >> 5;
+  const int64_t L = int64_t(1) << h, Q = L / kChiThreads;  // leaves per thread (0: some threads have one)
   const uint4 *lv = leaves + tree * L;
-  const int j = threadIdx.x;
-  U128 acc{0, 0};
-  if (j < L) {
-    const int64_t Q = L > kChiThreads ? L / kChiThreads : 1;
-    for (int64_t q = Q - 1; q >= 0; q--) {
-      acc = xor128(tmul(T, to_u4(acc)), u128(__ldg(&lv[j + kChiThreads * q])));
-    }
-  }
-  P[j] = to_u4(acc);
-  __syncthreads();
-  // sum_j s^j P_j: level l folds P[i + 2^l] * s^(2^l) into P[i], i = 0 mod 2^(l+1)
-  for (int l = 0; l < 8; l++) {
-    const int stride = 1 << l;
-    if ((j & (2 * stride - 1)) == 0) {
-      const U128 c = u128(spow[l]);
-      P[j] = to_u4(xor128(u128(P[j]), gmul(c, u128(P[j + stride]))));
+  const U128 s = u128(__ldg(&seeds[tree])), s4 = gsqr(gsqr(s));
+  uint4 acc = make_uint4(0, 0, 0, 0);
+  if (Q > 1) {
+    U128 u = s4;
+#pragma unroll 1
+    for (int l = 0; l < 5; l++) u = gsqr(u);
+    P[j] = to_u4(mulxn(u, j));
+    __syncthreads();
+    // four threads per nibble k: value v = 4 (j % 4) + i, eight copies each
+    const int k = j >> 2, v4 = j & 3;
+    uint4 base = make_uint4(0, 0, 0, 0);
+    if (v4 & 1) base = xor4(base, P[4 * k + 2]);
+    if (v4 & 2) base = xor4(base, P[4 * k + 3]);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      uint4 e = base;
+      if (i & 1) e = xor4(e, P[4 * k]);
+      if (i & 2) e = xor4(e, P[4 * k + 1]);
+#pragma unroll
+      for (int c = 0; c < 8; c++) T[(k * 16 + 4 * v4 + i) * 8 + ((c + lane) & 7)] = e;
     }
     __syncthreads();
+    const char *mine = reinterpret_cast<const char *>(T + (lane & 7));
+    acc = __ldg(&lv[j + kChiThreads * (Q - 1)]);
+    for (int64_t q = Q - 2; q >= 0; q--) {
+      const uint4 next = __ldg(&lv[j + kChiThreads * q]);
+      acc = xor4(to_u4(tmul(mine, acc)), next);
+    }
+  } else if (j < L) {
+    acc = __ldg(&lv[j]);
   }
-  if (j == 0) out[tree] = to_u4(gmul(s, u128(P[0])));
+  P[j] = acc;  // (the table's readers of P are past the barrier above)
+  __syncthreads();
+  {
+    const WarpMul mul(s4, lane);
+    uint4 r = P[warp + 4 * 31];
+#pragma unroll 1
+    for (int q = 30; q >= 0; q--) r = xor4(mul(r, lane), P[warp + 4 * q]);
+    if (lane == 0) R[warp] = r;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    const WarpMul mul(s, lane);
+    uint4 r = R[3];
+#pragma unroll
+    for (int q = 2; q >= 0; q--) r = xor4(mul(r, lane), R[q]);
+    r = mul(r, lane);
+    if (lane == 0) out[tree] = r;
+  }
 }
 
 }  // namespace

@@ -57,3 +57,17 @@ def test_chi_sum_check_identity_b13(ctx):
             pos = pos * 2 + 1 - int(ch[j, d])
         exp = oracle.gf128_mul(gf_pow(seeds[j], pos + 1), delta)
         assert np.array_equal(Vh[j] ^ Wh[j], exp)
+
+
+@pytest.mark.parametrize("t,h", [(1, 2), (3, 6), (2, 9), (1, 12), (448, 8)])
+def test_chi_sum_table_edges(ctx, t, h):
+    """Fewer leaves than threads, one leaf per thread (no table), two and more
+    per thread (tables), and extreme seeds: 0, 1, x^127, all ones."""
+    rng = np.random.default_rng(t * 57 + h)
+    leaves, seeds = rng_blocks(rng, t << h), rng_blocks(rng, t)
+    for special in (None, 0, 1, 1 << 127, (1 << 128) - 1):
+        if special is not None:
+            seeds[t // 2] = np.frombuffer(special.to_bytes(16, "little"), np.uint8)
+        out = torch.empty((t, 16), dtype=torch.uint8, device="cuda")
+        ctx.ferret_chi_sum(to_dev(leaves), h, to_dev(seeds), out)
+        assert np.array_equal(to_host(out), oracle.ferret_chi_sum(leaves, h, seeds, threads=8))
