@@ -3,9 +3,9 @@
 //
 // Two independent branches (run as one chain by default, see cfg.schedule):
 //   Ferret branch: a persistent PPRF launch over every Ferret sender tree
-//     (each CTA pulls (instance, tree) tasks from an atomic work counter,
-//     deepest trees first, and expands one whole tree per task with
-//     pprf_tree, in a per-CTA scratch slot for the level ping-pong); one
+//     (each group of threads pulls (instance, tree) tasks from an atomic work
+//     counter, deepest trees first, and expands one whole tree per task with
+//     pprf_tree, in its own scratch slot for the level ping-pong); one
 //     launch selecting the receivers' OT messages (ideal OT of the sender's
 //     level sums, as emp-ot's OTIdeal, ideal.h:7-31); the same persistent
 //     launch over the receiver trees; one persistent LPN launch over chunks
@@ -47,36 +47,32 @@ struct PprfTask {
 
 struct PprfBatchArgs {
   const PprfArgs *items;  // one per instance
-  const int *modes;       // PprfMode per instance
+  const int *sot;         // per instance: an SOT one
   const PprfTask *tasks;  // deepest trees first
   uint32_t ntasks;
   unsigned int *counter;
-  Blk *scratch;  // gridDim.x slots of 2^hmax blocks
+  Blk *scratch;  // a slot of 2^hmax blocks per group
   int hmax;
   const uint32_t *t0;
 };
 
+// Every group of G threads pulls trees (of senders or of receivers, Ferret's and
+// SOT's) from the queue.
+template <bool SEND, int G>
 __global__ void __launch_bounds__(kPprfThreads, 3) pprf_batch_kernel(PprfBatchArgs b) {
-  extern __shared__ __align__(16) uint32_t smem_tab[];
-  __shared__ PprfSmem sm;
-  __shared__ uint32_t s_task;
+  __shared__ uint32_t s_task[kPprfThreads / G];
   stage_table(smem_tab, b.t0);
-  const TabRef T{reinterpret_cast<const char *>(smem_tab), uint32_t(threadIdx.x & 31) * 4u};
-  Blk *slot = b.scratch + (uint64_t(blockIdx.x) << b.hmax);
+  __syncthreads();
+  const int group = threadIdx.x / G, tid = threadIdx.x % G;
+  Blk *slot = b.scratch + ((uint64_t(blockIdx.x) * (blockDim.x / G) + group) << b.hmax);
   for (;;) {
-    __syncthreads();  // table staged; previous task finished with s_task
-    if (threadIdx.x == 0) s_task = atomicAdd(b.counter, 1u);
-    __syncthreads();
-    const uint32_t task = s_task;
+    group_sync<G>(group);  // previous task finished with s_task and the shared state
+    if (tid == 0) s_task[group] = atomicAdd(b.counter, 1u);
+    group_sync<G>(group);
+    const uint32_t task = s_task[group];
     if (task >= b.ntasks) break;
     const PprfTask tk = b.tasks[task];
-    const PprfArgs &a = b.items[tk.item];
-    switch (b.modes[tk.item]) {
-      case FERRET_SEND: pprf_tree<FERRET_SEND>(a, tk.tree, slot, T, sm); break;
-      case FERRET_RECV: pprf_tree<FERRET_RECV>(a, tk.tree, slot, T, sm); break;
-      case SOT_SEND: pprf_tree<SOT_SEND>(a, tk.tree, slot, T, sm); break;
-      default: pprf_tree<SOT_RECV>(a, tk.tree, slot, T, sm); break;
-    }
+    pprf_tree<SEND, G>(b.items[tk.item], b.sot[tk.item] != 0, tk.tree, slot, group, tid);
   }
 }
 
@@ -149,6 +145,15 @@ __global__ void __launch_bounds__(kLpnThreads, 3) lpn_batch_kernel(LpnBatchArgs 
   }
 }
 
+template <bool SEND>
+cudaError_t batch_smem() {
+  constexpr auto kAttr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  cudaError_t e = cudaFuncSetAttribute(pprf_batch_kernel<SEND, 64>, kAttr, pprf_smem_bytes<64>());
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(pprf_batch_kernel<SEND, 128>, kAttr, pprf_smem_bytes<128>());
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(pprf_batch_kernel<SEND, 256>, kAttr, pprf_smem_bytes<256>());
+  return e;
+}
+
 // Per-device one-time set-up of this file's constants and kernel attributes.
 int batch_setup_device() {
   static std::mutex mu;
@@ -159,7 +164,8 @@ int batch_setup_device() {
   if (dev >= 0 && dev < 64 && ready[dev]) return CUOT_OK;
   cudaError_t e = pprf_upload_keys();
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(pprf_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTableBytes);
+    e = batch_smem<true>();
+  if (e == cudaSuccess) e = batch_smem<false>();
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(lpn_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTableBytes);
   if (e != cudaSuccess) {
@@ -201,7 +207,7 @@ struct cuot_batch {
   // PPRF per branch (kBrFerret, kBrSot)
   PprfBatchArgs send[2]{}, recv[2]{};
   int pprf_grid[2] = {0, 0};
-  int pprf_threads = 256;
+  int pprf_group[2] = {256, 256};  // threads per tree
   // Ferret selection
   SelItem *sel_d = nullptr;
   int nsel = 0;
@@ -308,9 +314,15 @@ LpnArgs make_lpn_job(const cuot_batch_item &it, const uint32_t *t0) {
   return a;
 }
 
+template <bool SEND>
 int pprf_launch(cuot_batch *b, const PprfBatchArgs &args, int br, cudaStream_t st) {
   if (!args.ntasks) return 0;
-  pprf_batch_kernel<<<b->pprf_grid[br], b->pprf_threads, kTableBytes, st>>>(args);
+  const int grid = b->pprf_grid[br], threads = b->cfg.pprf_threads == 128 ? 128 : kPprfThreads;
+  switch (b->pprf_group[br]) {
+    case 256: pprf_batch_kernel<SEND, 256><<<grid, threads, pprf_smem_bytes<256>(), st>>>(args); break;
+    case 128: pprf_batch_kernel<SEND, 128><<<grid, threads, pprf_smem_bytes<128>(), st>>>(args); break;
+    default: pprf_batch_kernel<SEND, 64><<<grid, threads, pprf_smem_bytes<64>(), st>>>(args); break;
+  }
   return 1;
 }
 
@@ -389,12 +401,12 @@ int enqueue(cuot_batch *b, cudaStream_t st, cudaEvent_t *ev = nullptr) {
   if (sched == CUOT_BATCH_SERIAL) {
     int launches = 0;
     mark(0);
-    launches += pprf_launch(b, b->send[kBrSot], kBrSot, st);
-    launches += pprf_launch(b, b->send[kBrFerret], kBrFerret, st);
+    launches += pprf_launch<true>(b, b->send[kBrSot], kBrSot, st);
+    launches += pprf_launch<true>(b, b->send[kBrFerret], kBrFerret, st);
     launches += select_launch(b, st);
     mark(1);
-    launches += pprf_launch(b, b->recv[kBrSot], kBrSot, st);
-    launches += pprf_launch(b, b->recv[kBrFerret], kBrFerret, st);
+    launches += pprf_launch<false>(b, b->recv[kBrSot], kBrSot, st);
+    launches += pprf_launch<false>(b, b->recv[kBrFerret], kBrFerret, st);
     mark(2);
     launches += lpn_launch(b, st);
     CUOT_TRY(launch_status(launches));
@@ -409,17 +421,17 @@ int enqueue(cuot_batch *b, cudaStream_t st, cudaEvent_t *ev = nullptr) {
     if (fer) {  // Ferret branch on streams[0]
       cudaStream_t sf = b->streams[0];
       if (cudaStreamWaitEvent(sf, E[kEvFork], 0) != cudaSuccess) return ev_fail();
-      int launches = pprf_launch(b, b->send[kBrFerret], kBrFerret, sf);
+      int launches = pprf_launch<true>(b, b->send[kBrFerret], kBrFerret, sf);
       launches += select_launch(b, sf);
-      launches += pprf_launch(b, b->recv[kBrFerret], kBrFerret, sf);
+      launches += pprf_launch<false>(b, b->recv[kBrFerret], kBrFerret, sf);
       launches += lpn_launch(b, sf);
       CUOT_TRY(launch_status(launches));
       if (b->lpn.ntasks) CUOT_TRY(record_done(b, 0, sf));
       if (cudaEventRecord(E[kEvFerret], sf) != cudaSuccess) return ev_fail();
     }
     // SOT branch: PPRFs on the caller's stream, then the lanes side by side
-    CUOT_TRY(launch_status(pprf_launch(b, b->send[kBrSot], kBrSot, st) +
-                           pprf_launch(b, b->recv[kBrSot], kBrSot, st)));
+    CUOT_TRY(launch_status(pprf_launch<true>(b, b->send[kBrSot], kBrSot, st) +
+                           pprf_launch<false>(b, b->recv[kBrSot], kBrSot, st)));
     const bool sizes = sched == CUOT_BATCH_FORK_SIZES;
     if (sizes) {
       if (cudaEventRecord(E[kEvSotPprf], st) != cudaSuccess) return ev_fail();
@@ -470,7 +482,6 @@ int cuot_batch_create(cuot_ctx *ctx, const cuot_batch_item *items, int count,
   if (b->cfg.schedule != CUOT_BATCH_SERIAL && b->cfg.schedule != CUOT_BATCH_FORK_FERRET &&
       b->cfg.schedule != CUOT_BATCH_FORK_SIZES)
     return cleanup(fail(CUOT_EINVAL, "schedule must be one of CUOT_BATCH_SERIAL / FORK_FERRET / FORK_SIZES"));
-  b->pprf_threads = b->cfg.pprf_threads ? b->cfg.pprf_threads : 256;
 
   // ---- per-item device state
   b->lsum.assign(count, nullptr); b->rsum.assign(count, nullptr); b->ss.assign(count, nullptr);
@@ -478,7 +489,7 @@ int cuot_batch_create(cuot_ctx *ctx, const cuot_batch_item *items, int count,
   b->item_ahat.assign(count, nullptr);
   b->plans.assign(count, nullptr);
   std::vector<PprfArgs> sargs(count), rargs(count);
-  std::vector<int> smodes(count), rmodes(count);
+  std::vector<int> sot(count);
   std::vector<SelItem> sel;
   int hmax[2] = {1, 1};
   for (int i = 0; i < count; i++) {
@@ -501,7 +512,6 @@ int cuot_batch_create(cuot_ctx *ctx, const cuot_batch_item *items, int count,
         return cleanup(st);
       s.lsum = b->lsum[i]; s.rsum = b->rsum[i]; s.ss_out = b->ss[i];
       r.mc = b->mc[i]; r.choice = it.choice_d; r.ss_in = b->ss[i];
-      smodes[i] = FERRET_SEND; rmodes[i] = FERRET_RECV;
       sel.push_back(SelItem{it.choice_d, b->lsum[i], b->rsum[i], b->mc[i], t * h});
       b->sel_max = std::max(b->sel_max, t * h);
     } else {
@@ -513,15 +523,14 @@ int cuot_batch_create(cuot_ctx *ctx, const cuot_batch_item *items, int count,
       r.m0_in = b->m0[i]; r.m1_in = b->m1[i];
       r.mc = reinterpret_cast<const Blk *>(it.mc_d);
       r.choice = it.choice_d;
-      smodes[i] = SOT_SEND; rmodes[i] = SOT_RECV;
+      sot[i] = 1;
     }
     sargs[i] = s;
     rargs[i] = r;
   }
   PprfArgs *sd = nullptr, *rd = nullptr;
-  int *smd = nullptr, *rmd = nullptr;
-  if ((st = upload(b, &sd, sargs)) || (st = upload(b, &rd, rargs)) || (st = upload(b, &smd, smodes)) ||
-      (st = upload(b, &rmd, rmodes)) || (st = balloc(b, &b->counters, kCounters * sizeof(unsigned int))))
+  int *sotd = nullptr;
+  if ((st = upload(b, &sd, sargs)) || (st = upload(b, &rd, rargs)) || (st = upload(b, &sotd, sot)) || (st = balloc(b, &b->counters, kCounters * sizeof(unsigned int))))
     return cleanup(st);
   // ---- PPRF tasks: every tree, deepest first.  Concurrent schedules keep
   // one list per branch, each with its own per-CTA scratch slots (the
@@ -538,14 +547,27 @@ int cuot_batch_create(cuot_ctx *ctx, const cuot_batch_item *items, int count,
       if (merged ? br == 0 : (items[i].kind == CUOT_KIND_FERRET) == (br == kBrFerret))
         for (uint64_t tr = 0; tr < items[i].t; tr++) tasks.push_back(PprfTask{uint32_t(i), uint32_t(tr)});
     if (tasks.empty()) continue;
-    b->pprf_grid[br] = int(std::min<uint64_t>(uint64_t(sms) * per_sm, tasks.size()));
+    // as many trees of the largest depth as the leaves would make: a deep tree
+    // that a small group drags on with alone would end the launch
+    int deepest = 1;
+    uint64_t leaves = 0;
+    for (const PprfTask &tk : tasks) {
+      deepest = std::max(deepest, items[tk.item].h);
+      leaves += 1ull << items[tk.item].h;
+    }
+    const uint64_t ctas = uint64_t(sms) * per_sm;
+    b->pprf_group[br] =
+        b->cfg.pprf_threads == 128 ? 128 : pprf_group_size(leaves >> deepest, deepest, ctas);
+    b->pprf_grid[br] = int(std::min<uint64_t>(ctas, tasks.size()));
+    const uint64_t slots =
+        uint64_t(b->pprf_grid[br]) * ((b->cfg.pprf_threads == 128 ? 128 : kPprfThreads) / b->pprf_group[br]);
     PprfTask *td = nullptr;
     Blk *pscr = nullptr;
-    if ((st = upload(b, &td, tasks)) || (st = balloc(b, &pscr, (uint64_t(b->pprf_grid[br]) << hmax[br]) * 16)))
+    if ((st = upload(b, &td, tasks)) || (st = balloc(b, &pscr, (slots << hmax[br]) * 16)))
       return cleanup(st);
-    b->send[br] = PprfBatchArgs{sd, smd, td, uint32_t(tasks.size()), b->counters + 2 * br, pscr, hmax[br],
+    b->send[br] = PprfBatchArgs{sd, sotd, td, uint32_t(tasks.size()), b->counters + 2 * br, pscr, hmax[br],
                                 ctx->t0_d};
-    b->recv[br] = PprfBatchArgs{rd, rmd, td, uint32_t(tasks.size()), b->counters + 2 * br + 1, pscr, hmax[br],
+    b->recv[br] = PprfBatchArgs{rd, sotd, td, uint32_t(tasks.size()), b->counters + 2 * br + 1, pscr, hmax[br],
                                 ctx->t0_d};
   }
   b->nsel = int(sel.size());

@@ -197,12 +197,10 @@ __device__ __forceinline__ void aes_enc2_from_round2(const TabRef &t, uint32_t (
 }
 
 // ---------------------------------------------------------------------------
-// Warp / block XOR reductions of a block value.
+// XOR of a block value over the warp, in every lane.
 __device__ __forceinline__ Blk warp_xor(Blk v) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-    for (int i = 0; i < 4; i++) v.w[i] ^= __shfl_xor_sync(0xffffffffu, v.w[i], o);
+  for (int i = 0; i < 4; i++) v.w[i] = __reduce_xor_sync(0xffffffffu, v.w[i]);
   return v;
 }
 

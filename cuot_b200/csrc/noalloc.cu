@@ -61,8 +61,9 @@ int setup_current_device(DeviceState **out) {
       return setup_error("cudaGetSymbolAddress(scratch)", e);
     if ((e = cudaGetSymbolAddress(reinterpret_cast<void **>(&s.t0), g_noalloc_t0)) != cudaSuccess)
       return setup_error("cudaGetSymbolAddress(table)", e);
-    if ((e = cudaFuncSetAttribute(pprf_tree_kernel<FERRET_SEND>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, kTableBytes)) != cudaSuccess)
+    if ((e = cudaFuncSetAttribute(pprf_tree_kernel<FERRET_SEND, kPprfThreads>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  pprf_smem_bytes<kPprfThreads>())) != cudaSuccess)
       return setup_error("cudaFuncSetAttribute", e);
     s.ready = true;
   }
@@ -101,7 +102,7 @@ extern "C" int cuot_ferret_pprf_sender_noalloc(const cuot_block *roots_d, uint64
   a.lsum = reinterpret_cast<Blk *>(lsum_d);
   a.rsum = reinterpret_cast<Blk *>(rsum_d);
   a.ss_out = reinterpret_cast<Blk *>(secret_sum_d);
-  pprf_tree_kernel<FERRET_SEND><<<dim3(unsigned(t)), kPprfThreads, kTableBytes,
-                                  static_cast<cudaStream_t>(stream)>>>(a);
+  pprf_tree_kernel<FERRET_SEND, kPprfThreads>
+      <<<dim3(unsigned(t)), kPprfThreads, pprf_smem_bytes<kPprfThreads>(), static_cast<cudaStream_t>(stream)>>>(a);
   return launch_status();
 }

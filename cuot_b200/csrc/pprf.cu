@@ -1,18 +1,24 @@
 // pprf.cu -- GGM PPRF expansion (Ferret MPCOT and SOT seed expansion).
 //
-// One CTA expands one whole tree, level by level: level l+1 = children of
-// level l with the emp-ot TwoKeyPRP node function (left = AES_k0(p) ^ p,
-// right = AES_k1(p) ^ p, ferret/twokeyprp.h:7-63).  The per-level left/right
-// XOR sums are reduced in-CTA with warp shuffles, so no level ever goes to
-// the host and no per-level launch or device synchronisation is needed
-// (cuOT launches aesExpand128 + xor_reduce passes + two cudaMemcpy2D per
-// level, dev_layer.cu:36-42).  The receiver's punctured-path correction is
-// applied in the same kernel right after the level's sums are known.
+// A group of 64 to 256 threads expands one whole tree, level by level: level
+// l+1 = children of level l with the emp-ot TwoKeyPRP node function (left =
+// AES_k0(p) ^ p, right = AES_k1(p) ^ p, ferret/twokeyprp.h:7-63).  The per-level
+// left/right XOR sums are reduced in the group (warp reductions, then one
+// warp), so no level ever goes to the host and no per-level launch or device
+// synchronisation is needed (cuOT launches aesExpand128 + xor_reduce passes +
+// two cudaMemcpy2D per level, dev_layer.cu:36-42).  The receiver's
+// punctured-path correction is applied in the same kernel right after the
+// level's sums are known.
 //
-// Levels ping-pong between the caller's leaf buffer and a scratch buffer of
-// the same size (the tree's slice of each), chosen so that the last level
-// lands in the leaf buffer.  Intermediate levels stay in L2 (at most
-// 3 CTAs x 2 x 2^(h-1) blocks per SM are live).
+// Levels of up to the group's size stay in shared memory; larger ones
+// ping-pong between the tree's slice of the caller's leaf buffer and the
+// group's slot of a scratch buffer, chosen so that the last level lands in
+// the leaf buffer.
+//
+// Bound by the T-table lookups' wavefronts (320 per node and warp) once the
+// chip is full, by the levels' AES latencies below that.
+#include <atomic>
+
 #include "pprf_kernel.cuh"
 
 namespace cuot {
@@ -26,26 +32,55 @@ int pprf_init_device() {
   return CUOT_OK;
 }
 
-template <int MODE>
-static int launch_pprf(cuot_ctx *ctx, PprfArgs &a, cudaStream_t st) {
-  static bool attr_set[64] = {false};
+// Resident CTAs of the tree kernel on ctx's device, with its shared memory set.
+template <int MODE, int G>
+static int pprf_capacity(const cuot_ctx *ctx, uint64_t *cap) {
+  static std::atomic<int> known[64];
   const int dev = ctx->device;
-  if (dev < 64 && !attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(pprf_tree_kernel<MODE>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         kTableBytes);
+  int c = dev < 64 ? known[dev].load() : 0;
+  if (!c) {
+    int per_sm = 0, sms = 0;
+    cudaError_t e = cudaFuncSetAttribute(pprf_tree_kernel<MODE, G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         pprf_smem_bytes<G>());
+    if (e == cudaSuccess)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pprf_tree_kernel<MODE, G>, kPprfThreads,
+                                                        pprf_smem_bytes<G>());
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) {
       cudaGetLastError();
-      return fail(CUOT_ECUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(e));
+      return fail(CUOT_ECUDA, "PPRF kernel set-up failed: %s", cudaGetErrorString(e));
     }
-    attr_set[dev] = true;
+    c = (per_sm < 1 ? 1 : per_sm) * sms;
+    if (dev < 64) known[dev].store(c);
   }
+  *cap = uint64_t(c);
+  return CUOT_OK;
+}
+
+template <int MODE, int G>
+static int launch_groups(cuot_ctx *ctx, PprfArgs &a, int threads, cudaStream_t st) {
+  uint64_t cap = 0;
+  CUOT_TRY((pprf_capacity<MODE, G>(ctx, &cap)));
+  // fewer trees than groups: one tree per CTA as far as the CTAs go
+  const uint64_t grid = a.t < cap ? a.t : cap, groups = grid * (threads / G);
   a.t0 = ctx->t0_d;
   void *scr = nullptr;
-  CUOT_TRY(scratch(ctx, (a.t << a.h) * sizeof(Blk), &scr));
+  CUOT_TRY(scratch(ctx, ((a.t < groups ? a.t : groups) << a.h) * sizeof(Blk), &scr));
   a.scratch = static_cast<Blk *>(scr);
-  pprf_tree_kernel<MODE><<<dim3((unsigned)a.t), ctx->pprf_threads, kTableBytes, st>>>(a);
+  pprf_tree_kernel<MODE, G><<<unsigned(grid), threads, pprf_smem_bytes<G>(), st>>>(a);
   return launch_status();
+}
+
+template <int MODE>
+static int launch_pprf(cuot_ctx *ctx, PprfArgs &a, cudaStream_t st) {
+  if (ctx->pprf_threads == 128) return launch_groups<MODE, 128>(ctx, a, 128, st);
+  uint64_t cap = 0;
+  CUOT_TRY((pprf_capacity<MODE, 256>(ctx, &cap)));
+  switch (pprf_group_size(a.t, a.h, cap)) {
+    case 256: return launch_groups<MODE, 256>(ctx, a, kPprfThreads, st);
+    case 128: return launch_groups<MODE, 128>(ctx, a, kPprfThreads, st);
+    default: return launch_groups<MODE, 64>(ctx, a, kPprfThreads, st);
+  }
 }
 
 static int check_tree_shape(uint64_t t, int h) {

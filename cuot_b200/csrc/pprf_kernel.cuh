@@ -1,5 +1,5 @@
-// pprf_kernel.cuh -- the GGM PPRF tree kernel (one CTA per tree), shared by
-// the translation units that launch it.  Each including file gets its own
+// pprf_kernel.cuh -- the GGM PPRF tree kernel (a group of threads per tree),
+// shared by the translation units that launch it.  Each including file gets its own
 // copy of the fixed-key schedule in constant memory and must upload it once
 // per device before the first launch (pprf_upload_keys).
 #pragma once
@@ -45,8 +45,7 @@ struct PprfArgs {
   const Blk *m0_in, *m1_in;
 };
 
-// Threads per tree (CTA size): 256 by default, 128 selectable (tuning);
-// the kernels are compiled for at most kPprfThreads.
+// Threads per CTA at most: one group of 256 or 128 threads, two of 128, four of 64.
 constexpr int kPprfThreads = 256;
 
 __device__ __forceinline__ Blk mask_lsb(Blk b) {
@@ -54,44 +53,75 @@ __device__ __forceinline__ Blk mask_lsb(Blk b) {
   return b;
 }
 
-// Shared-memory state of one tree expansion: per-warp level sums (left,
-// right), double-buffered by level parity, and the receiver's path.
+// Shared-memory state of a group of G threads (256, 128 or 64): the levels of up to G nodes, the
+// warps' level sums (left, right), double-buffered by level parity, and the
+// receiver's path.
+template <int G>
 struct PprfSmem {
-  Blk red[2][2][kPprfThreads / 32];
+  Blk lev[G + G / 2];
+  Blk red[2][2][G / 32];
   unsigned long long ap;
+  // Level of 2^k <= G nodes: levels alternate between the two parts.
+  __device__ Blk *level(int k) {
+    constexpr int kLog = G == 256 ? 8 : G == 128 ? 7 : 6;
+    return lev + ((k ^ kLog) & 1 ? G : 0);
+  }
 };
+// Dynamic shared memory of a CTA: the T-table, then the groups' states.
+template <int G>
+constexpr int pprf_smem_bytes() {
+  return kTableBytes + kPprfThreads / G * int(sizeof(PprfSmem<G>));
+}
+// Barrier of the group (named, since a CTA may hold several).
+template <int G>
+__device__ __forceinline__ void group_sync(int group) {
+  asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "n"(G) : "memory");
+}
 
-// Expands tree `tree` of the instance described by `a` with the whole CTA
-// (blockDim.x <= kPprfThreads threads, a multiple of 32).  scratch_tree: 2^h blocks for the level ping-pong.
+// Expands tree `tree` of the instance described by `a` with a group of G
+// threads (tid: thread of the group).  slot: 2^h blocks for the ping-pong of the
+// levels above G nodes; smaller ones stay in shared memory, where a level costs
+// one AES latency and a barrier and no trip to L2 and back.
 // The T-table must already be staged (and synced) in shared memory.
-template <int MODE>
-__device__ __forceinline__ void pprf_tree(const PprfArgs &a, uint64_t tree, Blk *scratch_tree,
-                                          const TabRef &T, PprfSmem &sm) {
-  unsigned long long &s_ap = sm.ap;
-  // Senders: the sums of level l leave the CTA (global stores by thread 0)
-  // and nothing of them is read back, so one barrier per level suffices,
-  // with the warp partials double-buffered by level parity: thread 0 reads
+extern __shared__ __align__(16) uint32_t smem_tab[];
+// sot: SOT modes (an argument, so that a kernel over trees of both kinds holds
+// the AES loop once).
+template <bool SEND, int G>
+__device__ __forceinline__ void pprf_tree(const PprfArgs &a, bool sot, uint64_t tree, Blk *slot, int group, int tid) {
+  PprfSmem<G> &sm = reinterpret_cast<PprfSmem<G> *>(smem_tab + kTableWords)[group];
+  const TabRef T{reinterpret_cast<const char *>(smem_tab), uint32_t(tid & 31) * 4u};
+  // Senders: the sums of level l leave the group (global stores by its first
+  // warp) and nothing of them is read back, so one barrier per level suffices,
+  // with the warp sums double-buffered by level parity: the first warp reads
   // red[l & 1] before it enters level l + 1, and red[l & 1] is written again
   // only after the barrier that ends level l + 1.  Receivers patch a node of
   // the level just written, which the next level reads, so they keep a
   // second barrier.
-  constexpr bool kSend = MODE == FERRET_SEND || MODE == SOT_SEND;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int lane = tid & 31, warp = tid >> 5;
   const int h = a.h;
   const uint64_t W = 1ull << h;
-  Blk *const bufs[2] = {a.leaves + tree * W, scratch_tree};
+  Blk *const leaves = a.leaves + tree * W;
   Blk root{{0, 0, 0, 0}};
-  if (MODE == FERRET_SEND || MODE == SOT_SEND) root = ldg_blk(a.roots + tree);
-  if (tid == 0) s_ap = 0;
-  __syncthreads();
+  if (SEND) root = ldg_blk(a.roots + tree);
+  uint64_t ap = 0;  // receivers' path (first thread)
 
   for (int l = 0; l < h; l++) {
-    const Blk *in = bufs[(h - l) & 1];
-    Blk *out = bufs[(h - l - 1) & 1];
     const bool last = (l == h - 1);
-    const uint64_t np = 1ull << l;
+    const uint32_t np = 1u << l;  // h <= 30
+    const Blk *in = np <= unsigned(G) ? sm.level(l) : (h - l) & 1 ? slot : leaves;
+    Blk *out = !last && 2 * np <= unsigned(G) ? sm.level(l + 1) : (h - l) & 1 ? leaves : slot;
+    // receivers: the level's choice and message, on their way during the AES
+    Blk x0{{0, 0, 0, 0}};
+    int bit = 0;
+    const uint64_t of = tree * h + l, os = uint64_t(l) * a.t + tree;
+    if (!SEND && tid == 0) {
+      bit = a.choice[sot ? os : of] ? 1 : 0;
+      x0 = ldg_blk(a.mc + (sot ? os : of));
+      if (sot) x0 = blk_xor(x0, ldg_blk((bit ? a.m1_in : a.m0_in) + os));
+    }
+    const uint32_t keep = last && !sot ? ~1u : ~0u;  // Ferret leaves: emp-ot `& one`
     Blk accL{{0, 0, 0, 0}}, accR{{0, 0, 0, 0}};
-    for (uint64_t i = tid; i < np; i += blockDim.x) {
+    for (uint32_t i = tid; i < np; i += G) {
       const Blk p = (l == 0) ? root : ld_blk(in + i);
       uint32_t L[4] = {p.w[0], p.w[1], p.w[2], p.w[3]};
       uint32_t R[4] = {p.w[0], p.w[1], p.w[2], p.w[3]};
@@ -100,10 +130,8 @@ __device__ __forceinline__ void pprf_tree(const PprfArgs &a, uint64_t tree, Blk 
       Blk cr{{R[0] ^ p.w[0], R[1] ^ p.w[1], R[2] ^ p.w[2], R[3] ^ p.w[3]}};
       accL = blk_xor(accL, cl);
       accR = blk_xor(accR, cr);
-      if ((MODE == FERRET_SEND || MODE == FERRET_RECV) && last) {
-        cl = mask_lsb(cl);
-        cr = mask_lsb(cr);
-      }
+      cl.w[0] &= keep;
+      cr.w[0] &= keep;
       if (last) {
         st_blk_cs(out + 2 * i, cl);
         st_blk_cs(out + 2 * i + 1, cr);
@@ -112,90 +140,109 @@ __device__ __forceinline__ void pprf_tree(const PprfArgs &a, uint64_t tree, Blk 
         st_blk(out + 2 * i + 1, cr);
       }
     }
-    accL = warp_xor(accL);
-    accR = warp_xor(accR);
-    Blk(&red)[2][kPprfThreads / 32] = sm.red[l & 1];
-    if (lane == 0) {
-      red[0][warp] = accL;
-      red[1][warp] = accR;
+    // Warps that had nodes (np: a power of two) add up theirs.
+    const int nw = np >= unsigned(G) ? G / 32 : np > 32 ? int(np / 32) : 1;
+    Blk(&red)[2][G / 32] = sm.red[l & 1];
+    if (warp < nw) {
+      accL = warp_xor(accL);
+      accR = warp_xor(accR);
+      if (nw > 1 && lane == 0) {
+        red[0][warp] = accL;
+        red[1][warp] = accR;
+      }
     }
-    __syncthreads();
-    if (tid == 0) {
-      Blk S[2] = {{{0, 0, 0, 0}}, {{0, 0, 0, 0}}};
+    group_sync<G>(group);
+    if (warp == 0) {
+      Blk S[2] = {accL, accR};
+      if (nw > 1) {  // lanes 0..: left sums, lanes 16..: right sums
+        Blk v{{0, 0, 0, 0}};
+        if ((lane & 15) < nw) v = ld_blk(&red[lane >> 4][lane & 15]);
 #pragma unroll
-      for (int w = 0; w < int(blockDim.x >> 5); w++) {
-        S[0] = blk_xor(S[0], red[0][w]);
-        S[1] = blk_xor(S[1], red[1][w]);
+        for (int o = G / 64; o > 0; o >>= 1)
+#pragma unroll
+          for (int i = 0; i < 4; i++) v.w[i] ^= __shfl_xor_sync(0xffffffffu, v.w[i], o);
+        S[0] = S[1] = v;
+#pragma unroll
+        for (int i = 0; i < 4; i++) S[1].w[i] = __shfl_down_sync(0xffffffffu, v.w[i], 16);
       }
-      if (MODE == FERRET_SEND) {
-        // ot_msg_0/1 of level l (spcot_sender.h:66-84), host layout [t][h]
-        st_blk(a.lsum + tree * h + l, S[0]);
-        st_blk(a.rsum + tree * h + l, S[1]);
-        if (last)  // secret_sum = XOR(masked leaves) ^ delta (spcot_sender.h:49-58)
-          st_blk(a.ss_out + tree, blk_xor(mask_lsb(blk_xor(S[0], S[1])), a.delta));
-      } else if (MODE == SOT_SEND) {
-        const uint64_t o = uint64_t(l) * a.t + tree;
-        const Blk b0 = ldg_blk(a.base0 + o), b1 = ldg_blk(a.base1 + o);
-        st_blk(a.m0 + o, blk_xor(b0, S[0]));
-        st_blk(a.m1 + o, blk_xor(b1, S[1]));
-        if (last) {  // extra row that carries delta (silent/sender.cu:97-102)
-          const uint64_t o2 = uint64_t(l + 1) * a.t + tree;
-          st_blk(a.m0 + o2, blk_xor(blk_xor(b0, S[1]), a.delta));
-          st_blk(a.m1 + o2, blk_xor(blk_xor(b1, S[0]), a.delta));
-        }
-      } else if (MODE == FERRET_RECV) {
-        // spcot_recver.h:71-95: b = 0 -> fill the even child, puncture the odd.
-        const int b = a.choice[tree * h + l] ? 1 : 0;
-        const Blk m = ldg_blk(a.mc + tree * h + l);
-        const uint64_t ap = s_ap;
-        const uint64_t f = 2 * ap + b, pun = 2 * ap + 1 - b;
-        // The node at f currently holds X (garbage, derived from the unknown
-        // punctured parent).  S_b includes X, so X ^ S_b ^ m is the XOR of
-        // the other same-side nodes with m: the sender's node.
-        const Blk fix = blk_xor(S[b], m);
-        if (!last) {
-          st_blk(out + f, blk_xor(ld_blk(out + f), fix));
-          s_ap = pun;
-        } else {
-          // Leaves are stored masked.  Filled leaf (masked) = X' ^ mask(fix).
-          st_blk(out + f, blk_xor(ld_blk(out + f), mask_lsb(fix)));
-          // Punctured leaf = XOR of all other masked leaves ^ secret_sum
-          // (spcot_recver.h:53-64) = mask(S0 ^ S1 ^ fix) ^ G' ^ ss, with G'
-          // the masked garbage leaf at `pun` (its term cancels).
-          const Blk g = ld_blk(out + pun);
-          Blk r = blk_xor(mask_lsb(blk_xor(blk_xor(S[0], S[1]), fix)), g);
-          r = blk_xor(r, ldg_blk(a.ss_in + tree));
-          st_blk(out + pun, r);
-        }
-      } else {  // SOT_RECV (silent/recver.cu:98-115, 143-155)
-        const uint64_t o = uint64_t(l) * a.t + tree;
-        const int c = a.choice[o] ? 1 : 0;
-        const Blk *mcur = c ? a.m1_in : a.m0_in;
-        const Blk mcv = ldg_blk(a.mc + o);
-        const Blk dec = blk_xor(ldg_blk(mcur + o), mcv);
-        const uint64_t ap = s_ap;
-        const uint64_t f = 2 * ap + c, pun = 2 * ap + 1 - c;
-        st_blk(out + f, blk_xor(ld_blk(out + f), blk_xor(dec, S[c])));
-        s_ap = pun;
-        if (last) {
-          const Blk dec2 = blk_xor(ldg_blk(mcur + uint64_t(l + 1) * a.t + tree), mcv);
-          st_blk(out + pun, blk_xor(ld_blk(out + pun), blk_xor(dec2, S[1 - c])));
+      if (lane == 0) {
+        if (SEND && !sot) {
+          // ot_msg_0/1 of level l (spcot_sender.h:66-84), host layout [t][h]
+          st_blk(a.lsum + of, S[0]);
+          st_blk(a.rsum + of, S[1]);
+          if (last)  // secret_sum = XOR(masked leaves) ^ delta (spcot_sender.h:49-58)
+            st_blk(a.ss_out + tree, blk_xor(mask_lsb(blk_xor(S[0], S[1])), a.delta));
+        } else if (SEND) {
+          const Blk b0 = ldg_blk(a.base0 + os), b1 = ldg_blk(a.base1 + os);
+          st_blk(a.m0 + os, blk_xor(b0, S[0]));
+          st_blk(a.m1 + os, blk_xor(b1, S[1]));
+          if (last) {  // extra row that carries delta (silent/sender.cu:97-102)
+            st_blk(a.m0 + os + a.t, blk_xor(blk_xor(b0, S[1]), a.delta));
+            st_blk(a.m1 + os + a.t, blk_xor(blk_xor(b1, S[0]), a.delta));
+          }
+        } else if (!sot) {
+          // spcot_recver.h:71-95: b = 0 -> fill the even child, puncture the odd.
+          const uint64_t f = 2 * ap + bit, pun = 2 * ap + 1 - bit;
+          // The node at f currently holds X (garbage, derived from the unknown
+          // punctured parent).  S_b includes X, so X ^ S_b ^ m is the XOR of
+          // the other same-side nodes with m: the sender's node.
+          const Blk fix = blk_xor(bit ? S[1] : S[0], x0);
+          if (!last) {
+            st_blk(out + f, blk_xor(ld_blk(out + f), fix));
+          } else {
+            // Leaves are stored masked.  Filled leaf (masked) = X' ^ mask(fix).
+            st_blk(out + f, blk_xor(ld_blk(out + f), mask_lsb(fix)));
+            // Punctured leaf = XOR of all other masked leaves ^ secret_sum
+            // (spcot_recver.h:53-64) = mask(S0 ^ S1 ^ fix) ^ G' ^ ss, with G'
+            // the masked garbage leaf at `pun` (its term cancels).
+            const Blk g = ld_blk(out + pun);
+            Blk r = blk_xor(mask_lsb(blk_xor(blk_xor(S[0], S[1]), fix)), g);
+            r = blk_xor(r, ldg_blk(a.ss_in + tree));
+            st_blk(out + pun, r);
+          }
+          ap = pun;
+        } else {  // SOT_RECV (silent/recver.cu:98-115, 143-155)
+          const uint64_t f = 2 * ap + bit, pun = 2 * ap + 1 - bit;
+          st_blk(out + f, blk_xor(ld_blk(out + f), blk_xor(x0, bit ? S[1] : S[0])));
+          if (last) {
+            const Blk dec2 = blk_xor(ldg_blk((bit ? a.m1_in : a.m0_in) + os + a.t), ldg_blk(a.mc + os));
+            st_blk(out + pun, blk_xor(ld_blk(out + pun), blk_xor(dec2, bit ? S[0] : S[1])));
+          }
+          ap = pun;
         }
       }
     }
-    if (!kSend) __syncthreads();
+    if (!SEND) group_sync<G>(group);
   }
 }
 
-// One CTA per tree of a single instance.
-template <int MODE>
+// Trees of a single instance: every group takes trees group, group + groups,
+// ... (persistent: the table is staged once per CTA, and a group's slot of the
+// scratch stays in L2 from tree to tree).
+template <int MODE, int G>
 __global__ void __launch_bounds__(kPprfThreads, 3) pprf_tree_kernel(PprfArgs a) {
-  extern __shared__ __align__(16) uint32_t smem_tab[];
-  __shared__ PprfSmem sm;
+  const int per_cta = blockDim.x / G;
   stage_table(smem_tab, a.t0);
-  const TabRef T{reinterpret_cast<const char *>(smem_tab), uint32_t(threadIdx.x & 31) * 4u};
-  const uint64_t tree = blockIdx.x;
-  pprf_tree<MODE>(a, tree, a.scratch + (tree << a.h), T, sm);
+  __syncthreads();
+  const int group = threadIdx.x / G;
+  // groups of one CTA take trees far apart, so that few trees spread over CTAs
+  const uint64_t id = uint64_t(group) * gridDim.x + blockIdx.x, groups = uint64_t(gridDim.x) * per_cta;
+  for (uint64_t tree = id; tree < a.t; tree += groups) {
+    pprf_tree<MODE == FERRET_SEND || MODE == SOT_SEND, G>(a, MODE == SOT_SEND || MODE == SOT_RECV, tree,
+                                                          a.scratch + (id << a.h), group, threadIdx.x % G);
+    group_sync<G>(group);  // the next tree's writes to the shared state
+  }
+}
+
+// Threads per tree for `trees` trees (the deepest of depth h) on `ctas` resident
+// CTAs.  Shallow levels leave most of a large group idle, so with enough trees
+// to fill the chip several smaller groups share a CTA.  Measured on B200
+// (Ferret sender, 256 / 128 / 64 threads): 64 trees of depth 10 22.5 / 24.3 /
+// 30.5 us, 300 34.6 / 34.5 / 38.7, 918 of depth 9 49 / 43 / 45, 1,280 of depth 13
+// 475 / 470 / 483, 1,500 of depth 10 107 / 107 / 92, 4,971 of depth 11 549 / 516 /
+// 464, 5,000 of depth 9 221 / 211 / 162 (one CTA per tree and launch before: 277).
+inline int pprf_group_size(uint64_t trees, int h, uint64_t ctas) {
+  return trees <= ctas ? 256 : trees <= 3 * ctas || h > 12 ? 128 : 64;
 }
 
 }  // namespace

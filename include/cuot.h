@@ -61,7 +61,9 @@ int cuot_ctx_reserve(cuot_ctx *ctx, uint64_t bytes);
 uint64_t cuot_ctx_scratch_bytes(const cuot_ctx *ctx);
 /* Tuning knobs of the single-instance calls made on this context (the
  * autotuner in cuot_b200/autotune.py sets them from its measurements):
- *   CUOT_TUNE_PPRF_THREADS  threads per tree CTA, 128 or 256 (default 256)
+ *   CUOT_TUNE_PPRF_THREADS  threads per tree CTA, 128 or 256 (default 256; a
+ *                           256-thread CTA expands one, two or four trees
+ *                           at a time, by their number and depth)
  *   CUOT_TUNE_QC_PLANES     planes per QC pass, 0 = automatic (512 MiB of
  *                           intermediate)
  *   CUOT_TUNE_QC_BACKEND    transform of the exact QC encode: 0 automatic
