@@ -116,8 +116,11 @@ __device__ __forceinline__ Lane lane_of(int id, int W) {
 // DFTs over k1 of one k2 and one coefficient class i0, then the three-point
 // ones of one q1; the 243 pairs of every lane change hands in shared memory.
 constexpr int kExchangeBytes = 243 * 2 * 32 * 4;
+// (CTAs per SM: three leave the other passes 72 registers for their 54 words and
+// fewer loads in flight, 34-46 us at 2^20 against 31-41 with two; the first
+// pass has 27 words, 27 us against 30)
 template <int L, PassKind KIND>
-__global__ void __launch_bounds__(288) tern_pass27(PassArgs a) {
+__global__ void __launch_bounds__(288, pass_first(KIND) ? 3 : 2) tern_pass27(PassArgs a) {
   constexpr int B = tern_block(L);
   const int W = KIND == kFirst ? 4 : KIND == kFirstBits ? 1 : a.W;
   extern __shared__ uint32_t X[];  // [q1][k2][coefficient][word][lane]
