@@ -25,6 +25,8 @@
 // threads, level by level, took as long as the leaves).
 // Bound by the lookups' wavefronts: 32 x 4 per 32 leaves and SM, 145 us for
 // 2,507 trees of depth 12.  Measured there 675 -> 196 us (64 trees of depth 10: 48 -> 13).
+#include <atomic>
+
 #include "ctx.cuh"
 
 namespace cuot {
@@ -126,6 +128,7 @@ __device__ __forceinline__ uint4 xor4(uint4 a, uint4 b) {
   return make_uint4(a.x ^ b.x, a.y ^ b.y, a.z ^ b.z, a.w ^ b.w);
 }
 
+template <bool CHAINED>
 __global__ void __launch_bounds__(kChiThreads) chi_sum_kernel(const uint4 *__restrict__ leaves, int h,
                                                               const uint4 *__restrict__ seeds,
                                                               uint4 *__restrict__ out) {
@@ -134,7 +137,9 @@ __global__ void __launch_bounds__(kChiThreads) chi_sum_kernel(const uint4 *__res
   __shared__ uint4 R[4];
   const int tree = blockIdx.x, j = threadIdx.x, lane = j & 31, warp = j >> 5;
   const int64_t L = int64_t(1) << h, Q = L / kChiThreads;  // leaves per thread (0: some threads have one)
-  const uint4 *lv = leaves + tree * L;
+  const uint32_t zero = chain_begin<CHAINED>();
+  const uint4 *lv = leaves + tree * L + zero;
+  seeds += zero;
   const U128 s = u128(__ldg(&seeds[tree])), s4 = gsqr(gsqr(s));
   uint4 acc = make_uint4(0, 0, 0, 0);
   if (Q > 1) {
@@ -199,18 +204,22 @@ int cuot_ferret_chi_sum(cuot_ctx *ctx, const cuot_block *leaves_d, uint64_t t, i
   if (t < 1 || t > 0x7fffffffull) return fail(CUOT_EINVAL, "t=%llu out of range", (unsigned long long)t);
   if (h < 1 || h > 30) return fail(CUOT_EINVAL, "h=%d out of range [1,30]", h);
   DeviceGuard g(ctx);
-  static bool attr_set[64] = {false};
-  if (ctx->device < 64 && !attr_set[ctx->device]) {
-    if (cudaFuncSetAttribute(chi_sum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kChiTableBytes) !=
-        cudaSuccess) {
+  static std::atomic<bool> attr_set[64];
+  const int dev = ctx->device;
+  if (dev >= 64 || !attr_set[dev].load()) {
+    constexpr auto kAttr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    if (cudaFuncSetAttribute(chi_sum_kernel<false>, kAttr, kChiTableBytes) != cudaSuccess ||
+        cudaFuncSetAttribute(chi_sum_kernel<true>, kAttr, kChiTableBytes) != cudaSuccess) {
       cudaGetLastError();
       return fail(CUOT_ECUDA, "chi kernel attribute failed");
     }
-    attr_set[ctx->device] = true;
+    if (dev < 64) attr_set[dev].store(true);
   }
-  chi_sum_kernel<<<dim3((unsigned)t), kChiThreads, kChiTableBytes, static_cast<cudaStream_t>(stream)>>>(
-      reinterpret_cast<const uint4 *>(leaves_d), h, reinterpret_cast<const uint4 *>(seeds_d),
-      reinterpret_cast<uint4 *>(out_d));
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const bool chained = chain_launches(t << h, st);
+  launch_as(chained, chained ? chi_sum_kernel<true> : chi_sum_kernel<false>, dim3((unsigned)t), dim3(kChiThreads),
+            kChiTableBytes, st, reinterpret_cast<const uint4 *>(leaves_d), h, reinterpret_cast<const uint4 *>(seeds_d),
+            reinterpret_cast<uint4 *>(out_d));
   return launch_status();
 }
 

@@ -29,17 +29,18 @@ __global__ void __launch_bounds__(kLpnThreads) lpn_kernel(LpnArgs a) {
 }
 
 // d = 10: five lanes per group (lpn_split6), persistent CTAs.
-template <LpnRoles ROLES>
+template <LpnRoles ROLES, bool CHAINED>
 __global__ void __launch_bounds__(kLpnThreads, 3) lpn_split_kernel(LpnArgs a) {
   extern __shared__ __align__(16) uint32_t smem_tab[];
   stage_table(smem_tab, a.t0);
   __syncthreads();
+  const uint32_t zero = chain_begin<CHAINED>();
   const TabRef T{reinterpret_cast<const char *>(smem_tab), uint32_t(threadIdx.x & 31) * 4u};
   const int64_t warps = int64_t(gridDim.x) * (kLpnThreads / 32), end = a.g0 + a.ngroups;
   const int64_t warp = int64_t(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-  for (int64_t g = a.g0 + 6 * warp; g < end; g += 6 * warps) lpn_split6<ROLES>(a, T, g, end);
+  for (int64_t g = a.g0 + 6 * warp + zero; g < end; g += 6 * warps) lpn_split6<ROLES>(a, T, g, end);
   if (blockIdx.x == gridDim.x - 1)
-    for (int64_t j = threadIdx.x; j < a.ntail; j += kLpnThreads) lpn_row1(a, T, a.j0 + j);
+    for (int64_t j = threadIdx.x + zero; j < a.ntail; j += kLpnThreads) lpn_row1(a, T, a.j0 + j);
 }
 
 __global__ void __launch_bounds__(256) lpn_interleave_kernel(LpnArgs a) {
@@ -100,15 +101,21 @@ int launch_any(cuot_ctx *ctx, const LpnArgs &a, cudaStream_t st) {
   return launch_status();
 }
 
-template <LpnRoles ROLES>
-int launch_split(cuot_ctx *ctx, const LpnArgs &a, cudaStream_t st) {
-  CUOT_TRY(set_smem(lpn_split_kernel<ROLES>));
+template <LpnRoles ROLES, bool CHAINED>
+int launch_split_as(cuot_ctx *ctx, const LpnArgs &a, cudaStream_t st) {
+  CUOT_TRY(set_smem(lpn_split_kernel<ROLES, CHAINED>));
   int per_sm = 0, sms = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lpn_split_kernel<ROLES>, kLpnThreads, kTableBytes);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lpn_split_kernel<ROLES, CHAINED>, kLpnThreads, kTableBytes);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
   const int64_t tasks = (a.ngroups + 5) / 6, cap = int64_t(per_sm < 1 ? 1 : per_sm) * sms;
-  lpn_split_kernel<ROLES><<<unsigned(tasks < 1 ? 1 : tasks < cap ? tasks : cap), kLpnThreads, kTableBytes, st>>>(a);
+  launch_as(CHAINED, lpn_split_kernel<ROLES, CHAINED>, dim3(unsigned(tasks < 1 ? 1 : tasks < cap ? tasks : cap)),
+            dim3(kLpnThreads), kTableBytes, st, a);
   return launch_status();
+}
+template <LpnRoles ROLES>
+int launch_split(cuot_ctx *ctx, const LpnArgs &a, cudaStream_t st) {
+  return chain_launches(uint64_t(a.ngroups) * 4, st) ? launch_split_as<ROLES, true>(ctx, a, st)
+                                                     : launch_split_as<ROLES, false>(ctx, a, st);
 }
 
 // Both roles, d = 10.  From kInterleaveRows rows on, kk and kk2 are first copied

@@ -61,7 +61,7 @@ int setup_current_device(DeviceState **out) {
       return setup_error("cudaGetSymbolAddress(scratch)", e);
     if ((e = cudaGetSymbolAddress(reinterpret_cast<void **>(&s.t0), g_noalloc_t0)) != cudaSuccess)
       return setup_error("cudaGetSymbolAddress(table)", e);
-    if ((e = cudaFuncSetAttribute(pprf_tree_kernel<FERRET_SEND, kPprfThreads>,
+    if ((e = cudaFuncSetAttribute(pprf_tree_kernel<FERRET_SEND, kPprfThreads, false>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   pprf_smem_bytes<kPprfThreads>())) != cudaSuccess)
       return setup_error("cudaFuncSetAttribute", e);
@@ -102,7 +102,7 @@ extern "C" int cuot_ferret_pprf_sender_noalloc(const cuot_block *roots_d, uint64
   a.lsum = reinterpret_cast<Blk *>(lsum_d);
   a.rsum = reinterpret_cast<Blk *>(rsum_d);
   a.ss_out = reinterpret_cast<Blk *>(secret_sum_d);
-  pprf_tree_kernel<FERRET_SEND, kPprfThreads>
+  pprf_tree_kernel<FERRET_SEND, kPprfThreads, false>
       <<<dim3(unsigned(t)), kPprfThreads, pprf_smem_bytes<kPprfThreads>(), static_cast<cudaStream_t>(stream)>>>(a);
   return launch_status();
 }

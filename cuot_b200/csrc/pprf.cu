@@ -33,17 +33,17 @@ int pprf_init_device() {
 }
 
 // Resident CTAs of the tree kernel on ctx's device, with its shared memory set.
-template <int MODE, int G>
+template <int MODE, int G, bool CHAINED>
 static int pprf_capacity(const cuot_ctx *ctx, uint64_t *cap) {
   static std::atomic<int> known[64];
   const int dev = ctx->device;
   int c = dev < 64 ? known[dev].load() : 0;
   if (!c) {
     int per_sm = 0, sms = 0;
-    cudaError_t e = cudaFuncSetAttribute(pprf_tree_kernel<MODE, G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(pprf_tree_kernel<MODE, G, CHAINED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          pprf_smem_bytes<G>());
     if (e == cudaSuccess)
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pprf_tree_kernel<MODE, G>, kPprfThreads,
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pprf_tree_kernel<MODE, G, CHAINED>, kPprfThreads,
                                                         pprf_smem_bytes<G>());
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) {
@@ -57,25 +57,32 @@ static int pprf_capacity(const cuot_ctx *ctx, uint64_t *cap) {
   return CUOT_OK;
 }
 
-template <int MODE, int G>
-static int launch_groups(cuot_ctx *ctx, PprfArgs &a, int threads, cudaStream_t st) {
+template <int MODE, int G, bool CHAINED>
+static int launch_on(cuot_ctx *ctx, PprfArgs &a, int threads, cudaStream_t st) {
   uint64_t cap = 0;
-  CUOT_TRY((pprf_capacity<MODE, G>(ctx, &cap)));
+  CUOT_TRY((pprf_capacity<MODE, G, CHAINED>(ctx, &cap)));
   // fewer trees than groups: one tree per CTA as far as the CTAs go
   const uint64_t grid = a.t < cap ? a.t : cap, groups = grid * (threads / G);
   a.t0 = ctx->t0_d;
   void *scr = nullptr;
   CUOT_TRY(scratch(ctx, ((a.t < groups ? a.t : groups) << a.h) * sizeof(Blk), &scr));
   a.scratch = static_cast<Blk *>(scr);
-  pprf_tree_kernel<MODE, G><<<unsigned(grid), threads, pprf_smem_bytes<G>(), st>>>(a);
+  launch_as(CHAINED, pprf_tree_kernel<MODE, G, CHAINED>, dim3(unsigned(grid)), dim3(threads),
+            pprf_smem_bytes<G>(), st, a);
   return launch_status();
+}
+
+template <int MODE, int G>
+static int launch_groups(cuot_ctx *ctx, PprfArgs &a, int threads, cudaStream_t st) {
+  return chain_launches(a.t << a.h, st) ? launch_on<MODE, G, true>(ctx, a, threads, st)
+                                        : launch_on<MODE, G, false>(ctx, a, threads, st);
 }
 
 template <int MODE>
 static int launch_pprf(cuot_ctx *ctx, PprfArgs &a, cudaStream_t st) {
   if (ctx->pprf_threads == 128) return launch_groups<MODE, 128>(ctx, a, 128, st);
   uint64_t cap = 0;
-  CUOT_TRY((pprf_capacity<MODE, 256>(ctx, &cap)));
+  CUOT_TRY((pprf_capacity<MODE, 256, false>(ctx, &cap)));
   switch (pprf_group_size(a.t, a.h, cap)) {
     case 256: return launch_groups<MODE, 256>(ctx, a, kPprfThreads, st);
     case 128: return launch_groups<MODE, 128>(ctx, a, kPprfThreads, st);

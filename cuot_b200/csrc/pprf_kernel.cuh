@@ -219,15 +219,16 @@ __device__ __forceinline__ void pprf_tree(const PprfArgs &a, bool sot, uint64_t 
 // Trees of a single instance: every group takes trees group, group + groups,
 // ... (persistent: the table is staged once per CTA, and a group's slot of the
 // scratch stays in L2 from tree to tree).
-template <int MODE, int G>
+template <int MODE, int G, bool CHAINED>
 __global__ void __launch_bounds__(kPprfThreads, 3) pprf_tree_kernel(PprfArgs a) {
   const int per_cta = blockDim.x / G;
   stage_table(smem_tab, a.t0);
   __syncthreads();
+  const uint32_t zero = chain_begin<CHAINED>();
   const int group = threadIdx.x / G;
   // groups of one CTA take trees far apart, so that few trees spread over CTAs
   const uint64_t id = uint64_t(group) * gridDim.x + blockIdx.x, groups = uint64_t(gridDim.x) * per_cta;
-  for (uint64_t tree = id; tree < a.t; tree += groups) {
+  for (uint64_t tree = id + zero; tree < a.t; tree += groups) {
     pprf_tree<MODE == FERRET_SEND || MODE == SOT_SEND, G>(a, MODE == SOT_SEND || MODE == SOT_RECV, tree,
                                                           a.scratch + (id << a.h), group, threadIdx.x % G);
     group_sync<G>(group);  // the next tree's writes to the shared state

@@ -816,10 +816,9 @@ static int default_batch(uint64_t n, int nplanes) {
 
 // ---- backend selection -------------------------------------------------------
 // Transform of the dual LPN of n = 2^e: the ternary transform (qc_tern.cu)
-// for 2^16 .. 2^22, the fp64 FFT (qc_fft.cu) for other n up to 2^22 (below
-// 2^16 the ternary transform's six launches cost more: 42 against 35 us at
-// 2^14, 53 against 47 at 2^15, but 60 against 65 at 2^16 and 394 against 727
-// at 2^20) and whenever the context asks for it or records its margin, GF(2)
+// for 2^14 .. 2^22, the fp64 FFT (qc_fft.cu) for smaller n (at 2^14 the two are
+// close, 33 against 35 us; at 2^16 49 against 65, at 2^20 387 against 727) and
+// up to 2^22 whenever the context asks for it or records its margin, GF(2)
 // Karatsuba over it (qc_kara.cu) for 2^23 and 2^24, the NTT above and whenever
 // the context asks for it.  Plane encodes (cuot_qc_encode and
 // cuot_qc_plan_encode) take the FFT or the NTT.

@@ -1,4 +1,4 @@
-// qc_tern.cu -- exact quasi-cyclic dual LPN of n = 2^e blocks, 16 <= e <= 22,
+// qc_tern.cu -- exact quasi-cyclic dual LPN of n = 2^e blocks, 14 <= e <= 22,
 // by the ternary transform of qc_tern.cuh: out = a * in mod (x^n - 1) for all
 // 128 bit planes at once, with blocks read and written as they are (a block
 // is the 128 planes' bits of one coefficient, so no bit transpose is needed)
@@ -13,8 +13,8 @@
 //   tern_pass27 / pass9    inverse passes
 //   tern_final             pieces -> coefficients mod x^n - 1 (XORed with xor_in)
 // Measured on B200, one dual LPN through a plan, the fp64 FFT path against this:
-// n = 2^16 65 / 60 us, 2^17 102 / 83, 2^18 184 / 107, 2^19 371 / 189, 2^20 727
-// / 394, 2^21 1542 / 974, 2^22 3346 / 2000.
+// n = 2^14 35 / 33 us, 2^15 47 / 38, 2^16 65 / 49, 2^17 102 / 69, 2^18 184 / 92,
+// 2^19 371 / 186, 2^20 727 / 387, 2^21 1542 / 976, 2^22 3346 / 2003.
 #include "ctx.cuh"
 #include "qc_tern.cuh"
 
@@ -119,7 +119,7 @@ constexpr int kExchangeBytes = 243 * 2 * 32 * 4;
 // (CTAs per SM: three leave the other passes 72 registers for their 54 words and
 // fewer loads in flight, 34-46 us at 2^20 against 31-41 with two; the first
 // pass has 27 words, 27 us against 30)
-template <int L, PassKind KIND>
+template <int L, PassKind KIND, bool CHAINED>
 __global__ void __launch_bounds__(288, pass_first(KIND) ? 3 : 2) tern_pass27(PassArgs a) {
   constexpr int B = tern_block(L);
   const int W = KIND == kFirst ? 4 : KIND == kFirstBits ? 1 : a.W;
@@ -135,8 +135,9 @@ __global__ void __launch_bounds__(288, pass_first(KIND) ? 3 : 2) tern_pass27(Pas
   const uint64_t group = uint64_t(tern_points(s)) * tern_element(L);
   const uint64_t at = uint64_t(blockIdx.z) * a.job_words + uint64_t(w) * group;
   __syncthreads();
+  const uint32_t zero = chain_begin<CHAINED>();
   {
-    const uint32_t *src = pass_first(KIND) ? a.jobs.in[blockIdx.z] : a.src + at;
+    const uint32_t *src = pass_first(KIND) ? a.jobs.in[blockIdx.z] + zero : a.src + at + zero;
     const int k2 = warp / 3, i0 = warp % 3;
     G4 f[9][3];
     if (ln.on) {
@@ -186,7 +187,7 @@ __global__ void __launch_bounds__(288, pass_first(KIND) ? 3 : 2) tern_pass27(Pas
 }
 
 // Radix 9 or 3: a thread holds three blocks' coefficients of all pieces.
-template <int L, int RAD, PassKind KIND>
+template <int L, int RAD, PassKind KIND, bool CHAINED>
 __global__ void __launch_bounds__(128, 5) tern_pass9(PassArgs a) {  // 5: all 54 loads in flight (at 80 registers 150 us a pass at 2^22, at 96 125)
   constexpr int B = tern_block(L);
   __shared__ RotEntry tab[kRotEntries];
@@ -197,10 +198,11 @@ __global__ void __launch_bounds__(128, 5) tern_pass9(PassArgs a) {  // 5: all 54
   const int id = blockIdx.y * 128 + threadIdx.x, i0 = id / (a.W * B);
   const Lane ln = lane_of<L, KIND>(id % (a.W * B), a.W);
   __syncthreads();
+  const uint32_t zero = chain_begin<CHAINED>();
   if (!ln.on || i0 >= 3) return;
   const uint64_t at = uint64_t(blockIdx.z) * a.job_words + uint64_t(ln.w) * tern_points(s) * tern_element(L);
   G4 f[RAD][3];
-  load_slots<L, RAD, RAD, KIND>(a, b, sigmas, a.src + at, tab, 0, 1, i0, ln.r, ln.w, f);
+  load_slots<L, RAD, RAD, KIND>(a, b, sigmas, a.src + at + zero, tab, 0, 1, i0, ln.r, ln.w, f);
   dft<RAD>(f);
   uint32_t *o = a.dst + at + b.first * tern_element(L) + i0 * B + ln.r;
   const int step = b.step * tern_element(L);
@@ -251,15 +253,16 @@ __device__ __forceinline__ void inner_forward(const uint32_t *x, uint32_t *V, in
   __syncthreads();
 }
 
-template <class S>
+template <class S, bool CHAINED>
 __global__ void __launch_bounds__(inner_threads<S>(), inner_blocks<S>()) tern_inner(uint32_t *buf, uint64_t job_words,
                                                                                    TernJobs jobs) {
   extern __shared__ uint32_t V[];
   constexpr int NT = inner_threads<S>();
   const int tid = threadIdx.x;
-  uint32_t *x = buf + uint64_t(blockIdx.z) * job_words +
+  const uint32_t zero = chain_begin<CHAINED>();
+  uint32_t *x = buf + zero + uint64_t(blockIdx.z) * job_words +
                 (uint64_t(blockIdx.y) * gridDim.x + blockIdx.x) * tern_element(S::L);
-  const uint32_t *cs = jobs.consts[blockIdx.z] + uint64_t(blockIdx.x) * kLeafWords * S::LEAVES;
+  const uint32_t *cs = jobs.consts[blockIdx.z] + zero + uint64_t(blockIdx.x) * kLeafWords * S::LEAVES;
   const Task2 t2 = task2<S>(tid);
   uint32_t next[kLeafWords] = {};
   {
@@ -309,14 +312,15 @@ __global__ void __launch_bounds__(inner_threads<S>(), inner_blocks<S>()) tern_in
 }
 
 // The leaf constants of a point of the transform of `a`.
-template <class S>
+template <class S, bool CHAINED>
 __global__ void __launch_bounds__(192) tern_consts(const uint32_t *buf, uint32_t *consts) {
   extern __shared__ uint32_t V[];
   const int tid = threadIdx.x;
   const Task2 t2 = task2<S>(tid);
+  const uint32_t zero = chain_begin<CHAINED>();
   {
     G4 f[3][S::G];
-    inner_forward<S, 192>(buf + uint64_t(blockIdx.x) * tern_element(S::L), V, tid, t2, f);
+    inner_forward<S, 192>(buf + zero + uint64_t(blockIdx.x) * tern_element(S::L), V, tid, t2, f);
     if (tid < S::TASK2) {
 #pragma unroll
       for (int q = 0; q < 3; q++)
@@ -351,17 +355,18 @@ __global__ void __launch_bounds__(192) tern_consts(const uint32_t *buf, uint32_t
 
 // A thread per coefficient: the word groups' coefficients of a warp are each
 // contiguous, and its blocks are written whole.
-template <int E>
+template <int E, bool CHAINED>
 __global__ void __launch_bounds__(256) tern_final(const uint32_t *buf, uint64_t job_words, TernJobs jobs) {
   constexpr TernShape s = tern_shape(E);
   const uint32_t j = blockIdx.x * 256 + threadIdx.x;
-  const uint32_t *b = buf + uint64_t(blockIdx.z) * job_words;
+  const uint32_t zero = chain_begin<CHAINED>();
+  const uint32_t *b = buf + zero + uint64_t(blockIdx.z) * job_words;
   constexpr uint64_t group = uint64_t(tern_points(s)) * tern_element(s.L);
   uint4 v = make_uint4(tern_coefficient<E>(b, j), tern_coefficient<E>(b + group, j), tern_coefficient<E>(b + 2 * group, j),
                        tern_coefficient<E>(b + 3 * group, j));
   const uint4 *xi = reinterpret_cast<const uint4 *>(jobs.xor_in[blockIdx.z]);
   if (xi) {
-    const uint4 x = xi[j];
+    const uint4 x = xi[j + zero];
     v = make_uint4(v.x ^ x.x, v.y ^ x.y, v.z ^ x.z, v.w ^ x.w);
   }
   reinterpret_cast<uint4 *>(jobs.out[blockIdx.z])[j] = v;
@@ -379,90 +384,105 @@ int set_smem(F fn, int bytes) {
   cudaGetLastError();
   return fail(CUOT_ECUDA, "QC shared-memory attribute failed: %s", cudaGetErrorString(e));
 }
-template <int L, PassKind KIND>
-int pass27(const PassArgs &a, int njobs, cudaStream_t st) {
-  CUOT_TRY(set_smem(tern_pass27<L, KIND>, kExchangeBytes));
-  const dim3 grid(tern_points(tern_shape(a.e)) / 27, (a.W * tern_block(L) + 31) / 32, njobs);
-  tern_pass27<L, KIND><<<grid, 288, kExchangeBytes, st>>>(a);
+
+// One call's launches: njobs side by side on st, chained or not.
+struct Run {
+  int njobs;
+  bool chained;
+  cudaStream_t st;
+};
+template <int L, PassKind KIND, bool C>
+int pass27(const Run &r, const PassArgs &a) {
+  CUOT_TRY(set_smem(tern_pass27<L, KIND, C>, kExchangeBytes));
+  const dim3 grid(tern_points(tern_shape(a.e)) / 27, (a.W * tern_block(L) + 31) / 32, r.njobs);
+  launch_as(C, tern_pass27<L, KIND, C>, grid, dim3(288), kExchangeBytes, r.st, a);
   return CUOT_OK;
 }
-template <int L, int RAD, PassKind KIND>
-int pass9(const PassArgs &a, int njobs, cudaStream_t st) {
-  const dim3 grid(tern_points(tern_shape(a.e)) / RAD, (3 * a.W * tern_block(L) + 127) / 128, njobs);
-  tern_pass9<L, RAD, KIND><<<grid, 128, 0, st>>>(a);
+template <int L, int RAD, PassKind KIND, bool C>
+int pass9(const Run &r, const PassArgs &a) {
+  const dim3 grid(tern_points(tern_shape(a.e)) / RAD, (3 * a.W * tern_block(L) + 127) / 128, r.njobs);
+  launch_as(C, tern_pass9<L, RAD, KIND, C>, grid, dim3(128), 0, r.st, a);
   return CUOT_OK;
 }
 // Pass a.pass of the transform (KIND kForward: of the passes after the first).
-template <int L>
-int pass_of(const PassArgs &a, PassKind kind, int njobs, cudaStream_t st) {
+template <int L, bool C>
+int pass_of(const Run &r, const PassArgs &a, PassKind kind) {
   const int rad = tern_radix(tern_shape(a.e).m, a.pass);
   switch (kind) {
-    case kFirst: return pass27<L, kFirst>(a, njobs, st);
-    case kFirstBits: return pass27<L, kFirstBits>(a, njobs, st);
-    case kLastInverse: return pass27<L, kLastInverse>(a, njobs, st);
+    case kFirst: return pass27<L, kFirst, C>(r, a);
+    case kFirstBits: return pass27<L, kFirstBits, C>(r, a);
+    case kLastInverse: return pass27<L, kLastInverse, C>(r, a);
     case kForward:
-      return rad == 27  ? pass27<L, kForward>(a, njobs, st)
-             : rad == 9 ? pass9<L, 9, kForward>(a, njobs, st)
-                        : pass9<L, 3, kForward>(a, njobs, st);
+      return rad == 27  ? pass27<L, kForward, C>(r, a)
+             : rad == 9 ? pass9<L, 9, kForward, C>(r, a)
+                        : pass9<L, 3, kForward, C>(r, a);
     default:
-      return rad == 27  ? pass27<L, kInverse>(a, njobs, st)
-             : rad == 9 ? pass9<L, 9, kInverse>(a, njobs, st)
-                        : pass9<L, 3, kInverse>(a, njobs, st);
+      return rad == 27  ? pass27<L, kInverse, C>(r, a)
+             : rad == 9 ? pass9<L, 9, kInverse, C>(r, a)
+                        : pass9<L, 3, kInverse, C>(r, a);
   }
 }
-int pass(const PassArgs &a, PassKind kind, int njobs, cudaStream_t st) {
-  switch (tern_shape(a.e).L) {
-    case 243: return pass_of<243>(a, kind, njobs, st);
-    case 729: return pass_of<729>(a, kind, njobs, st);
-    case 1458: return pass_of<1458>(a, kind, njobs, st);
-    default: return pass_of<2187>(a, kind, njobs, st);
-  }
+template <class S, bool C>
+int inner_of(const Run &r, int P, uint32_t *buf, uint64_t job_words, const TernJobs &jobs) {
+  CUOT_TRY(set_smem(tern_inner<S, C>, S::WORDS * 4));
+  launch_as(C, tern_inner<S, C>, dim3(P, 4, r.njobs), dim3(inner_threads<S>()), S::WORDS * 4, r.st, buf, job_words, jobs);
+  return CUOT_OK;
 }
-// Input -> values at the points; *buf: where they are (one of the two halves).
-int forward(int e, PassKind kind, const TernJobs &jobs, uint32_t *half[2], uint64_t job_words, int njobs, int *at,
-            cudaStream_t st) {
-  const int W = kind == kFirstBits ? 1 : 4, passes = tern_passes(tern_shape(e).m);
-  PassArgs a{e, 0, W, nullptr, half[0], job_words, jobs};
-  CUOT_TRY(pass(a, kind, njobs, st));
+template <class S, bool C>
+int consts_of(const Run &r, int P, const uint32_t *buf, uint32_t *consts) {
+  constexpr int smem = (S::BASE + S::NE * S::DIAGS) * 4;
+  CUOT_TRY(set_smem(tern_consts<S, C>, smem));
+  launch_as(C, tern_consts<S, C>, dim3(P), dim3(192), smem, r.st, buf, consts);
+  return CUOT_OK;
+}
+// The sizes that are ever chained (kChainBlocks) have L = 243 or 729.
+#define TERN_DISPATCH(L_, F, ...)                                                         \
+  switch (L_) {                                                                           \
+    case 243: return r.chained ? F<TERN_##F(243, 27), true> __VA_ARGS__                   \
+                               : F<TERN_##F(243, 27), false> __VA_ARGS__;                 \
+    case 729: return r.chained ? F<TERN_##F(729, 27), true> __VA_ARGS__                   \
+                               : F<TERN_##F(729, 27), false> __VA_ARGS__;                 \
+    case 1458: return F<TERN_##F(1458, 54), false> __VA_ARGS__;                           \
+    default: return F<TERN_##F(2187, 81), false> __VA_ARGS__;                             \
+  }
+#define TERN_pass_of(L, LP) L
+#define TERN_inner_of(L, LP) Inner<L, LP>
+#define TERN_consts_of(L, LP) Inner<L, LP>
+int pass(const Run &r, const PassArgs &a, PassKind kind) {
+  TERN_DISPATCH(tern_shape(a.e).L, pass_of, (r, a, kind))
+}
+int inner(const Run &r, int e, uint32_t *buf, uint64_t job_words, const TernJobs &jobs) {
+  const int P = tern_points(tern_shape(e));
+  TERN_DISPATCH(tern_shape(e).L, inner_of, (r, P, buf, job_words, jobs))
+}
+int consts(const Run &r, int e, const uint32_t *buf, uint32_t *out) {
+  const int P = tern_points(tern_shape(e));
+  TERN_DISPATCH(tern_shape(e).L, consts_of, (r, P, buf, out))
+}
+#undef TERN_pass_of
+#undef TERN_inner_of
+#undef TERN_consts_of
+#undef TERN_DISPATCH
+
+template <int E>
+void final_of(const Run &r, const uint32_t *buf, uint64_t job_words, const TernJobs &jobs) {
+  constexpr bool kMayChain = (1ull << E) <= kChainBlocks;
+  launch_as(kMayChain && r.chained, kMayChain && r.chained ? tern_final<E, kMayChain> : tern_final<E, false>,
+            dim3((1u << E) / 256, 1, r.njobs), dim3(256), 0, r.st, buf, job_words, jobs);
+}
+
+// Input -> values at the points; *at: the half they are in.
+int forward(const Run &r, int e, PassKind kind, const TernJobs &jobs, uint32_t *half[2], uint64_t job_words, int *at) {
+  const int passes = tern_passes(tern_shape(e).m);
+  PassArgs a{e, 0, kind == kFirstBits ? 1 : 4, nullptr, half[0], job_words, jobs};
+  CUOT_TRY(pass(r, a, kind));
   for (a.pass = 1; a.pass < passes; a.pass++) {
     a.src = half[(a.pass - 1) & 1];
     a.dst = half[a.pass & 1];
-    CUOT_TRY(pass(a, kForward, njobs, st));
+    CUOT_TRY(pass(r, a, kForward));
   }
   *at = (passes - 1) & 1;
   return CUOT_OK;
-}
-
-template <class S>
-int inner_launch(int P, uint32_t *buf, uint64_t job_words, const TernJobs &jobs, int njobs, cudaStream_t st) {
-  CUOT_TRY(set_smem(tern_inner<S>, S::WORDS * 4));
-  tern_inner<S><<<dim3(P, 4, njobs), inner_threads<S>(), S::WORDS * 4, st>>>(buf, job_words, jobs);
-  return CUOT_OK;
-}
-template <class S>
-int consts_launch(int P, const uint32_t *buf, uint32_t *consts, cudaStream_t st) {
-  constexpr int smem = (S::BASE + S::NE * S::DIAGS) * 4;
-  CUOT_TRY(set_smem(tern_consts<S>, smem));
-  tern_consts<S><<<P, 192, smem, st>>>(buf, consts);
-  return CUOT_OK;
-}
-int inner(const TernShape &s, uint32_t *buf, uint64_t job_words, const TernJobs &jobs, int njobs, cudaStream_t st) {
-  const int P = tern_points(s);
-  switch (s.L) {
-    case 243: return inner_launch<Inner<243, 27>>(P, buf, job_words, jobs, njobs, st);
-    case 729: return inner_launch<Inner<729, 27>>(P, buf, job_words, jobs, njobs, st);
-    case 1458: return inner_launch<Inner<1458, 54>>(P, buf, job_words, jobs, njobs, st);
-    default: return inner_launch<Inner<2187, 81>>(P, buf, job_words, jobs, njobs, st);
-  }
-}
-int consts(const TernShape &s, const uint32_t *buf, uint32_t *out, cudaStream_t st) {
-  const int P = tern_points(s);
-  switch (s.L) {
-    case 243: return consts_launch<Inner<243, 27>>(P, buf, out, st);
-    case 729: return consts_launch<Inner<729, 27>>(P, buf, out, st);
-    case 1458: return consts_launch<Inner<1458, 54>>(P, buf, out, st);
-    default: return consts_launch<Inner<2187, 81>>(P, buf, out, st);
-  }
 }
 
 }  // namespace
@@ -479,11 +499,12 @@ uint64_t tern_job_bytes(int e) { return 2 * group_words(e) * 16; }
 
 int tern_build_ahat(int e, const uint64_t *a_d, void *scratch, void *ahat, cudaStream_t st) {
   uint32_t *half[2] = {static_cast<uint32_t *>(scratch), static_cast<uint32_t *>(scratch) + group_words(e)};
+  const Run r{1, chain_launches(1ull << e, st), st};
   TernJobs jobs{};
   jobs.in[0] = reinterpret_cast<const uint32_t *>(a_d);
   int at = 0;
-  CUOT_TRY(forward(e, kFirstBits, jobs, half, 0, 1, &at, st));
-  CUOT_TRY(consts(tern_shape(e), half[at], static_cast<uint32_t *>(ahat), st));
+  CUOT_TRY(forward(r, e, kFirstBits, jobs, half, 0, &at));
+  CUOT_TRY(consts(r, e, half[at], static_cast<uint32_t *>(ahat)));
   return launch_status(1 + tern_passes(tern_shape(e).m));
 }
 
@@ -493,6 +514,7 @@ int tern_dual(int e, const TernJob *job, int njobs, void *scratch, cudaStream_t 
   const uint64_t job_words = group_words(e) * 4;
   uint32_t *half[2] = {static_cast<uint32_t *>(scratch), static_cast<uint32_t *>(scratch) + njobs * job_words};
   const int passes = tern_passes(s.m);
+  const Run r{njobs, chain_launches(uint64_t(njobs) << e, st), st};
   TernJobs jobs{};
   for (int j = 0; j < njobs; j++) {
     jobs.in[j] = reinterpret_cast<const uint32_t *>(job[j].in);
@@ -501,24 +523,20 @@ int tern_dual(int e, const TernJob *job, int njobs, void *scratch, cudaStream_t 
     jobs.consts[j] = static_cast<const uint32_t *>(job[j].ahat);
   }
   int at = 0;
-  CUOT_TRY(forward(e, kFirst, jobs, half, job_words, njobs, &at, st));
-  CUOT_TRY(inner(s, half[at], job_words, jobs, njobs, st));
+  CUOT_TRY(forward(r, e, kFirst, jobs, half, job_words, &at));
+  CUOT_TRY(inner(r, e, half[at], job_words, jobs));
   PassArgs a{e, 0, 4, nullptr, nullptr, job_words, jobs};
   for (a.pass = passes - 1; a.pass >= 0; a.pass--, at ^= 1) {
     a.src = half[at];
     a.dst = half[at ^ 1];
     // a single coset's pieces (y^m = 1) need no rotation in the end
-    CUOT_TRY(pass(a, a.pass || s.cosets == 1 ? kInverse : kLastInverse, njobs, st));
+    CUOT_TRY(pass(r, a, a.pass || s.cosets == 1 ? kInverse : kLastInverse));
   }
-  const uint32_t *buf = half[at];
-  const dim3 grid((1u << e) / 256, 1, njobs);
   switch (e) {
-#define TERN_FINAL(E)                                          \
-  case E:                                                      \
-    tern_final<E><<<grid, 256, 0, st>>>(buf, job_words, jobs); \
-    break;
-    TERN_FINAL(16) TERN_FINAL(17) TERN_FINAL(18) TERN_FINAL(19)
-    TERN_FINAL(20) TERN_FINAL(21) TERN_FINAL(22)
+#define TERN_FINAL(E) \
+  case E: final_of<E>(r, half[at], job_words, jobs); break;
+    TERN_FINAL(14) TERN_FINAL(15) TERN_FINAL(16) TERN_FINAL(17) TERN_FINAL(18)
+    TERN_FINAL(19) TERN_FINAL(20) TERN_FINAL(21) TERN_FINAL(22)
 #undef TERN_FINAL
   }
   return launch_status(2 * passes + 2);

@@ -39,9 +39,11 @@ struct TernShape {
   int L, Lp;      // ring sizes: R_L (outer), R_Lp (inner); T = L / Lp points per half
   int m, cosets;  // 1: C (y^m = 1); 2: F
 };
-constexpr int kTernMinE = 16, kTernMaxE = 22;
+constexpr int kTernMinE = 14, kTernMaxE = 22;
 constexpr TernShape tern_shape(int e) {
-  return e == 16   ? TernShape{243, 27, 729, 1}
+  return e == 14   ? TernShape{243, 27, 81, 2}
+         : e == 15 ? TernShape{243, 27, 243, 2}
+         : e == 16 ? TernShape{243, 27, 729, 1}
          : e == 17 ? TernShape{729, 27, 243, 2}
          : e == 18 ? TernShape{729, 27, 729, 1}
          : e == 19 ? TernShape{729, 27, 729, 2}
@@ -61,7 +63,7 @@ constexpr bool tern_shape_ok(int e) {
   return (s.cosets == 2 ? 2 : 1) * s.m >= 2 * tern_pieces(s, e) - 1 && tern_pieces(s, e) <= s.m &&
          s.L % (s.cosets == 2 ? s.m : s.m / 3) == 0;
 }
-static_assert(tern_shape_ok(16) && tern_shape_ok(17) && tern_shape_ok(18) &&
+static_assert(tern_shape_ok(14) && tern_shape_ok(15) && tern_shape_ok(16) && tern_shape_ok(17) && tern_shape_ok(18) &&
                   tern_shape_ok(19) && tern_shape_ok(20) && tern_shape_ok(21) && tern_shape_ok(22),
               "points must determine the product and their roots of unity must lie in R_L");
 

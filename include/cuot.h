@@ -67,7 +67,7 @@ uint64_t cuot_ctx_scratch_bytes(const cuot_ctx *ctx);
  *   CUOT_TUNE_QC_PLANES     planes per QC pass, 0 = automatic (512 MiB of
  *                           intermediate)
  *   CUOT_TUNE_QC_BACKEND    transform of the exact QC encode: 0 automatic
- *                           (dual LPNs of 2^16 <= n <= 2^22 by the ternary
+ *                           (dual LPNs of 2^14 <= n <= 2^22 by the ternary
  *                           GF(2) transform; otherwise as 2), 1 the NTT
  *                           everywhere, 2 the fp64 FFT for n <= 2^22, dual
  *                           LPNs at 2^23 and 2^24 as GF(2) Karatsuba over
@@ -303,7 +303,7 @@ int cuot_ferret_chi_sum(cuot_ctx *ctx, const cuot_block *leaves_d, uint64_t t,
  * consecutive) becomes a * plane_r mod (x^n - 1) over GF(2), exactly
  * (replaces the float cuFFT path of QuasiCyclic::encode_dense,
  * quasi_cyclic.cu:118-128).  n a power of two in [2^10, 2^25].  The
- * product is a transform over GF(2)[x] itself for dual LPNs of 2^16 <= n <=
+ * product is a transform over GF(2)[x] itself for dual LPNs of 2^14 <= n <=
  * 2^22; an fp64 FFT carrying four planes per transform for plane encodes and
  * other dual LPNs of n <= 2^22 (exact: the rounding error of the convolution
  * stays below 1/2), GF(2) Karatsuba over that FFT for dual LPNs at 2^23 and

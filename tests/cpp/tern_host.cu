@@ -216,6 +216,8 @@ static void dual(const uint64_t *a, const uint32_t *in, uint32_t *out) {
 
 extern "C" int tern_host_dual(int e, const uint64_t *a, const uint32_t *in, uint32_t *out) {
   switch (e) {
+    case 14: dual<14, Inner<243, 27>>(a, in, out); break;
+    case 15: dual<15, Inner<243, 27>>(a, in, out); break;
     case 16: dual<16, Inner<243, 27>>(a, in, out); break;
     case 17: dual<17, Inner<729, 27>>(a, in, out); break;
     case 18: dual<18, Inner<729, 27>>(a, in, out); break;

@@ -14,7 +14,7 @@ import oracle
 from tests.util import rng_blocks, to_dev, to_host
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-SIZES = range(16, 23)
+SIZES = range(14, 23)
 
 
 @pytest.fixture(scope="module")
@@ -99,9 +99,9 @@ def test_dual_lpn_equals_fft(e):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("e,count", [(16, 9), (17, 4), (18, 3), (20, 2)])
+@pytest.mark.parametrize("e,count", [(14, 3), (15, 9), (16, 9), (17, 4), (18, 3), (20, 2)])
 def test_batched_jobs_equal_plain(e, count):
-    """Several instances of one size share launches (e = 16: 18 jobs, more than
+    """Several instances of one size share launches (e = 15, 16: 18 jobs, more than
     one launch holds); each equals its own plan's dual LPN, and a margin-
     recording context, which keeps to the FFT, agrees."""
     torch = pytest.importorskip("torch")
@@ -128,3 +128,65 @@ def test_batched_jobs_equal_plain(e, count):
         ctx.close()
     for (v, w), (v2, w2) in zip(*outs):
         assert torch.equal(v, v2) and torch.equal(w, w2)
+
+
+@pytest.mark.gpu
+def test_chained_launches_keep_the_order():
+    """Small calls back to back on one stream (their kernels are chained), on two
+    streams joined by events, and captured into a graph: every call sees the
+    results of the one before."""
+    import cuot_b200
+    torch = pytest.importorskip("torch")
+    t, h = 16, 10
+    n = t << h
+    rng = np.random.default_rng(99)
+    ctxs = [cuot_b200.Context(0), cuot_b200.Context(0)]
+    a = to_dev(rng.integers(0, 1 << 63, n // 64, dtype=np.int64))
+    roots = [to_dev(rng_blocks(rng, t)) for _ in range(4)]
+    kk, seed, delta = to_dev(rng_blocks(rng, 300)), bytes(range(16)), bytes(range(1, 17))
+    e = lambda m: torch.empty((m, 16), dtype=torch.uint8, device="cuda")
+    plans = [c.qc_plan(a, n) for c in ctxs]
+
+    def chain(i, ctx, plan, v, s, sync):
+        ls, rs, ss, out = e(t * h), e(t * h), e(t), e(t)
+        for f in (lambda: ctx.ferret_pprf_sender(roots[i], h, delta, v, ls, rs, ss, stream=s),
+                  lambda: ctx.lpn_primal(seed, kk, v, stream=s), lambda: plan.dual_lpn(v, stream=s),
+                  lambda: plan.dual_lpn(v, stream=s), lambda: ctx.lpn_primal(seed, kk, v, stream=s),
+                  lambda: ctx.ferret_chi_sum(v, h, ss, out, stream=s)):
+            f()
+            if sync:
+                torch.cuda.synchronize()
+        return out
+
+    v = [e(n) for _ in range(2)]
+    main = torch.cuda.current_stream()
+    want = []
+    for i in range(4):
+        o = chain(i, ctxs[0], plans[0], v[0], main, True)
+        want.append((v[0].clone(), o.clone()))
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for rep in range(3):
+        got = []
+        for i in range(4):  # alternate streams, each step after the one before
+            s = side if i % 2 else main
+            s.wait_stream(main if i % 2 else side)
+            with torch.cuda.stream(s):
+                o = chain(i, ctxs[i % 2], plans[i % 2], v[0], s, False)
+                got.append((v[0].clone(), o))
+        main.wait_stream(side)
+        torch.cuda.synchronize()
+        for (x, y), (x2, y2) in zip(want, got):
+            assert torch.equal(x, x2) and torch.equal(y, y2), rep
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        o = chain(1, ctxs[0], plans[0], v[1], torch.cuda.current_stream(), False)
+    for _ in range(3):
+        v[1].zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(v[1], want[1][0]) and torch.equal(o, want[1][1])
+    del plans
+    torch.cuda.synchronize()
+    for c in ctxs:
+        c.close()
