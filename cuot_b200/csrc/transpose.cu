@@ -8,6 +8,11 @@
 //     tile (tr_blocks_to_planes128, tr_planes128_to_blocks);
 //   blocks -> any multiple of 32 planes, and up to 128 planes -> blocks:
 //     padded shared tile (stride 33 words), 4-byte plane-row accesses.
+//   any multiple of 8 blocks <-> 128 planes whose rows then start at any byte
+//     (tr_blocks_to_ragged, tr_ragged_to_blocks): the same tiles, plane rows
+//     accessed in aligned 4-byte words put together by funnel shifts (1,290,680
+//     blocks: 80 -> 15 us to planes and 25 -> 13 back, with the byte-granular
+//     kernel before; every byte of a plane row was a store of its own).
 // All move 32x32 bit tiles with a five-stage warp-shuffle transpose (one word
 // per lane).  Any other shape, or a pointer not aligned for the fast path's
 // accesses, uses a byte-granular 8x8 kernel.
@@ -157,6 +162,111 @@ __global__ void __launch_bounds__(kTrThreads) tr_planes128_to_blocks(const uint4
   }
 }
 
+// blocks -> 128 planes, rows % 8 == 0.  out: 128 rows of rows / 8 bytes, any
+// alignment.  A warp writes a plane's 128 bytes of the CTA: lane j the aligned
+// word that holds bytes 4j - m .. 4j - m + 3 of them (m: the row's misalignment);
+// the bytes at both ends are left to byte stores, as is the last tile.
+__global__ void __launch_bounds__(kTrThreads) tr_blocks_to_ragged(const uint4 *__restrict__ in, uint64_t rows,
+                                                                  uint8_t *__restrict__ out) {
+  __shared__ uint32_t st[128][kTrG + 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const TrLane tl = tr_lane(lane);
+  const uint64_t g0 = uint64_t(blockIdx.x) * kTrG;
+  constexpr int kPer = kTrG / (kTrThreads / 32);
+  uint4 v[kPer];
+#pragma unroll
+  for (int j = 0; j < kPer; j++) {
+    const uint64_t row = (g0 + warp * kPer + j) * 32 + lane;
+    v[j] = row < rows ? __ldcs(in + row) : make_uint4(0, 0, 0, 0);
+  }
+#pragma unroll
+  for (int j = 0; j < kPer; j++) {
+    const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+#pragma unroll
+    for (int q = 0; q < 4; q++) st[q * 32 + lane][warp * kPer + j] = warp_transpose32(w[q], tl);
+  }
+  __syncthreads();
+  const uint64_t row_bytes = rows / 8, left = row_bytes - g0 * 4;
+  if (left >= 4 * kTrG) {  // whole tile: 31 or 32 aligned words per plane, then the planes' ends
+#pragma unroll 4
+    for (int p = warp; p < 128; p += kTrThreads / 32) {
+      uint8_t *o = out + uint64_t(p) * row_bytes + g0 * 4;
+      const int m = int(reinterpret_cast<uintptr_t>(o) & 3);
+      const uint32_t x = __funnelshift_l(lane ? st[p][lane - 1] : 0u, st[p][lane], 8 * m);
+      if (lane || !m) *reinterpret_cast<uint32_t *>(o + 4 * lane - m) = x;
+    }
+    const int p = warp + (kTrThreads / 32) * (lane & 15);
+    uint8_t *o = out + uint64_t(p) * row_bytes + g0 * 4;
+    const int m = int(reinterpret_cast<uintptr_t>(o) & 3);
+    if (m) {  // lanes 0..15 the first 4 - m bytes, 16..31 the last m
+      const uint32_t x = lane < 16 ? st[p][0] : st[p][kTrG - 1] >> (32 - 8 * m);
+      const int n = lane < 16 ? 4 - m : m, at = lane < 16 ? 0 : 4 * kTrG - m;
+#pragma unroll
+      for (int k = 0; k < 3; k++)
+        if (k < n) o[at + k] = uint8_t(x >> (8 * k));
+    }
+    return;
+  }
+  const int nb = int(left);
+  for (int p = warp; p < 128; p += kTrThreads / 32) {
+    uint8_t *o = out + uint64_t(p) * row_bytes + g0 * 4;
+    for (int b = lane; b < nb; b += 32) o[b] = uint8_t(st[p][b / 4] >> (8 * (b & 3)));
+  }
+}
+
+// 128 planes -> blocks, ncols % 8 == 0.  in: 128 rows of row_bytes bytes, any
+// alignment, of which the first ncols / 8 are read, in aligned words put
+// together by funnel shifts (the first and the last tiles byte by byte).
+__global__ void __launch_bounds__(kTrThreads) tr_ragged_to_blocks(const uint8_t *__restrict__ in, uint64_t ncols,
+                                                                  uint64_t row_bytes, uint4 *__restrict__ out) {
+  __shared__ uint32_t st[128][kTrG + 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const TrLane tl = tr_lane(lane);
+  const uint64_t g0 = uint64_t(blockIdx.x) * kTrG;
+  const uint64_t left = ncols / 8 - g0 * 4;
+  const int nb = left < uint64_t(4 * kTrG) ? int(left) : 4 * kTrG;
+  const uint64_t base = g0 * 4;
+  constexpr int kPer = 128 / (kTrThreads / 32);
+  // Words that start before plane 0's row or end after plane 127's last byte
+  // may lie outside the input: the first tile and the last two read bytes.
+  if (base >= 4 && base + 4 * kTrG + 8 <= row_bytes) {
+    auto word = [&](int p, int j) {
+      const uint8_t *r = in + uint64_t(p) * row_bytes + base;
+      return __ldcs(reinterpret_cast<const uint32_t *>(r - (reinterpret_cast<uintptr_t>(r) & 3)) + j);
+    };
+    uint32_t x[kPer];
+#pragma unroll
+    for (int i = 0; i < kPer; i++) x[i] = word(warp + i * (kTrThreads / 32), lane);
+    const uint32_t ends = word(warp + (lane % kPer) * (kTrThreads / 32), 32);
+#pragma unroll
+    for (int i = 0; i < kPer; i++) {
+      const int p = warp + i * (kTrThreads / 32);
+      const int m = int(reinterpret_cast<uintptr_t>(in + uint64_t(p) * row_bytes + base) & 3);
+      const uint32_t next = __shfl_down_sync(0xffffffffu, x[i], 1), last = __shfl_sync(0xffffffffu, ends, i);
+      st[p][lane] = __funnelshift_r(x[i], lane == 31 ? last : next, 8 * m);
+    }
+  } else {
+    for (int i = 0; i < kPer; i++) {
+      const int p = warp + i * (kTrThreads / 32);
+      const uint8_t *r = in + uint64_t(p) * row_bytes + base;
+      uint32_t v = 0;
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        if (4 * lane + k < nb) v |= uint32_t(__ldg(r + 4 * lane + k)) << (8 * k);
+      st[p][lane] = v;
+    }
+  }
+  __syncthreads();
+  for (int gg = warp; gg < kTrG; gg += kTrThreads / 32) {
+    const uint64_t row = (g0 + gg) * 32 + lane;
+    if ((g0 + gg) * 32 >= ncols) break;
+    uint32_t w[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) w[q] = warp_transpose32(st[q * 32 + lane][gg], tl);
+    if (row < ncols) out[row] = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}
+
 constexpr int kTrGroups = 32;       // row groups of 32 rows per CTA (128 B of each plane row)
 constexpr int kTrStride = kTrGroups + 1;
 
@@ -288,6 +398,21 @@ int transpose_launch(const void *in, uint64_t rows, uint64_t row_bytes, uint64_t
     if (grid > 0x7fffffffull) return fail(CUOT_EINVAL, "too many columns");
     tr_planes128_to_blocks<<<unsigned(grid), kTrThreads, 0, st>>>(static_cast<const uint4 *>(in), ncols,
                                                                    row_bytes / 16, static_cast<uint4 *>(out));
+    return launch_status();
+  }
+  const bool all_planes = row_bytes == 16 && col_lo == 0 && ncols == 128 && aligned(in, 16);
+  if (all_planes && (rows % 32 || !aligned(out, 4))) {
+    const uint64_t grid = (rows + 32 * kTrG - 1) / (32 * kTrG);
+    if (grid > 0x7fffffffull) return fail(CUOT_EINVAL, "too many rows");
+    tr_blocks_to_ragged<<<unsigned(grid), kTrThreads, 0, st>>>(static_cast<const uint4 *>(in), rows,
+                                                                static_cast<uint8_t *>(out));
+    return launch_status();
+  }
+  if (rows == 128 && col_lo == 0 && aligned(out, 16) && (ncols % 32 || row_bytes % 4 || !aligned(in, 4))) {
+    const uint64_t grid = (ncols + 32 * kTrG - 1) / (32 * kTrG);
+    if (grid > 0x7fffffffull) return fail(CUOT_EINVAL, "too many columns");
+    tr_ragged_to_blocks<<<unsigned(grid), kTrThreads, 0, st>>>(static_cast<const uint8_t *>(in), ncols, row_bytes,
+                                                                static_cast<uint4 *>(out));
     return launch_status();
   }
   if (row_bytes == 16 && rows % 32 == 0 && col_lo % 32 == 0 && ncols % 32 == 0 && ncols > 0 &&
