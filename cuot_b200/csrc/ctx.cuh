@@ -9,6 +9,7 @@ struct cuot_ctx {
   uint64_t scratch_bytes;
   void *qc_tables[32];     // NTT twiddle tables per log2(n) (qc.cu)
   void *qcf_tables[32];    // FFT twiddle tables per log2(n) (qc_fft.cu)
+  void *tern_aux[32];      // second stream of the ternary transform per log2(n) (qc.cu)
   int pprf_threads;        // threads per tree CTA (128 or 256)
   int qc_planes_per_pass;  // 0: automatic
   int qc_backend;          // CUOT_TUNE_QC_BACKEND value: 0 automatic, 1 NTT, 2 FFT
@@ -124,7 +125,13 @@ int tern_build_ahat(int e, const uint64_t *a_d, void *scratch, void *ahat, cudaS
 // Up to kTernMaxJobs dual LPNs of one size side by side; scratch holds
 // tern_job_bytes(e) for each.
 constexpr int kTernMaxJobs = 16;
-int tern_dual(int e, const TernJob *jobs, int njobs, void *scratch, cudaStream_t st);
+// aux: second stream to share the work with (joined again before the call
+// returns), or null.
+struct TernAux {
+  cudaStream_t stream;
+  cudaEvent_t ev[2];  // fork, join
+};
+int tern_dual(int e, const TernJob *jobs, int njobs, void *scratch, TernAux *aux, cudaStream_t st);
 int transpose_launch(const void *in, uint64_t rows, uint64_t row_bytes, uint64_t col_lo,
                      uint64_t col_hi, void *out, cudaStream_t st);
 }  // namespace cuot

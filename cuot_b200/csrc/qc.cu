@@ -683,12 +683,26 @@ static int get_tables(cuot_ctx *ctx, int e, QcTables **out) {
   return CUOT_OK;
 }
 
+// Smallest work that two streams share (2^18: 93 us with them, 92 without).
+constexpr int kTernAuxMinE = 19;
+static void free_aux(TernAux *a) {
+  if (!a) return;
+  if (a->stream) cudaStreamDestroy(a->stream);
+  for (cudaEvent_t e : a->ev)
+    if (e) cudaEventDestroy(e);
+  delete a;
+}
+
 void qc_free_ctx_tables(cuot_ctx *ctx) {
   for (int e = 0; e < 32; e++) {
     free_tables(static_cast<QcTables *>(ctx->qc_tables[e]));
     ctx->qc_tables[e] = nullptr;
   }
   qcf_free_ctx_tables(ctx);
+  for (void *&p : ctx->tern_aux) {
+    free_aux(static_cast<TernAux *>(p));
+    p = nullptr;
+  }
 }
 
 static int col_smem(const QcTables *t) {
@@ -817,7 +831,7 @@ static int default_batch(uint64_t n, int nplanes) {
 // ---- backend selection -------------------------------------------------------
 // Transform of the dual LPN of n = 2^e: the ternary transform (qc_tern.cu)
 // for 2^14 .. 2^22, the fp64 FFT (qc_fft.cu) for smaller n (at 2^14 the two are
-// close, 33 against 35 us; at 2^16 49 against 65, at 2^20 387 against 727) and
+// close, 33 against 35 us; at 2^16 49 against 65, at 2^20 375 against 727) and
 // up to 2^22 whenever the context asks for it or records its margin, GF(2)
 // Karatsuba over it (qc_kara.cu) for 2^23 and 2^24, the NTT above and whenever
 // the context asks for it.  Plane encodes (cuot_qc_encode and
@@ -884,6 +898,33 @@ static uint64_t dual_scratch_bytes(const cuot_ctx *ctx, QcKind k, int e, int bat
 static uint64_t dual_y_offset(QcKind k, int e, bool r2) {
   if (k == kQcKara) return qck_scratch_bytes(e);
   return (r2 ? 32ull : 16ull) << e;
+}
+
+// The second stream of the ternary dual LPNs of n = 2^e on ctx, for sizes that
+// gain from one; null for others, and while the context keeps its encodes on
+// one stream.  Created with a plan or batch, or on the first call that is not
+// being captured (capturing: null until then).
+static int tern_aux(cuot_ctx *ctx, int e, int njobs, cudaStream_t st, TernAux **out) {
+  *out = nullptr;
+  if (ctx->qc_streams != 2 || (uint64_t(njobs) << e) < (1ull << kTernAuxMinE)) return CUOT_OK;
+  if (!ctx->tern_aux[e]) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+      cudaGetLastError();
+      return CUOT_OK;
+    }
+    TernAux *a = new TernAux{};
+    if (cudaStreamCreateWithFlags(&a->stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&a->ev[0], cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&a->ev[1], cudaEventDisableTiming) != cudaSuccess) {
+      cudaGetLastError();
+      free_aux(a);
+      return fail(CUOT_ECUDA, "QC stream / event creation failed");
+    }
+    ctx->tern_aux[e] = a;
+  }
+  *out = static_cast<TernAux *>(ctx->tern_aux[e]);
+  return CUOT_OK;
 }
 
 struct QcEngine {
@@ -953,7 +994,9 @@ static int eng_dual(cuot_ctx *ctx, const QcEngine &g, int e, const void *ahat, c
   const cuot_block *xor_in = r2 ? in : nullptr;
   if (g.kind == kQcTern) {
     const TernJob job{src, xor_in, out, ahat};
-    return tern_dual(e, &job, 1, scr, st);
+    TernAux *aux;
+    CUOT_TRY(tern_aux(ctx, e, 1, st, &aux));
+    return tern_dual(e, &job, 1, scr, aux, st);
   }
   void *Y = scr + dual_y_offset(g.kind, e, r2);
   if (g.kind == kQcKara) return qck_dual_lpn(g.f, e, ahat, src, xor_in, out, scr, Y, leaf_batch(ctx), st);
@@ -980,6 +1023,8 @@ int qc_kind(const cuot_ctx *ctx, int e) { return dual_kind(ctx, e); }
 
 int qc_prepare(cuot_ctx *ctx, int kind, int e) {
   QcEngine g;
+  TernAux *aux;
+  if (kind == kQcTern) CUOT_TRY(tern_aux(ctx, e, kTernMaxJobs, nullptr, &aux));
   return engine(ctx, e, QcKind(kind), false, &g);
 }
 
@@ -1077,7 +1122,9 @@ int qc_encode_jobs(cuot_ctx *ctx, int kind, int e, cuot_block *const *io, int nj
       TernJob jobs[kTernMaxJobs];
       const int nj = njobs - j0 < per ? njobs - j0 : per;
       for (int j = 0; j < nj; j++) jobs[j] = TernJob{io[j0 + j], nullptr, io[j0 + j], ahats[j0 + j]};
-      CUOT_TRY(tern_dual(e, jobs, nj, Y, st));
+      TernAux *aux;
+      CUOT_TRY(tern_aux(ctx, e, nj, st, &aux));
+      CUOT_TRY(tern_dual(e, jobs, nj, Y, aux, st));
     }
     return CUOT_OK;
   }
@@ -1152,6 +1199,8 @@ int cuot_qc_plan_create(cuot_ctx *ctx, const uint64_t *a_d, uint64_t n, void *st
   cuot_qc_plan *pl = new cuot_qc_plan{ctx, e, n, dual_kind(ctx, e), nullptr, 0};
   QcEngine g;
   int st = engine(ctx, e, pl->kind, true, &g);
+  TernAux *aux;
+  if (st == CUOT_OK && pl->kind == kQcTern) st = tern_aux(ctx, e, 1, static_cast<cudaStream_t>(stream), &aux);
   if (st == CUOT_OK) st = dev_alloc(&pl->ahat, ahat_bytes(pl->kind, e, true));
   void *scr = nullptr;
   if (st == CUOT_OK) st = scratch(ctx, ahat_scratch_bytes(pl->kind, e), &scr);

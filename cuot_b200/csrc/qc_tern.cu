@@ -14,7 +14,7 @@
 //   tern_final             pieces -> coefficients mod x^n - 1 (XORed with xor_in)
 // Measured on B200, one dual LPN through a plan, the fp64 FFT path against this:
 // n = 2^14 35 / 33 us, 2^15 47 / 38, 2^16 65 / 49, 2^17 102 / 69, 2^18 184 / 92,
-// 2^19 371 / 186, 2^20 727 / 387, 2^21 1542 / 976, 2^22 3346 / 2003.
+// 2^19 371 / 169, 2^20 727 / 375, 2^21 1542 / 928, 2^22 3346 / 1946.
 #include "ctx.cuh"
 #include "qc_tern.cuh"
 
@@ -385,9 +385,9 @@ int set_smem(F fn, int bytes) {
   return fail(CUOT_ECUDA, "QC shared-memory attribute failed: %s", cudaGetErrorString(e));
 }
 
-// One call's launches: njobs side by side on st, chained or not.
+// One call's launches: njobs side by side on st, chained or not; W word groups.
 struct Run {
-  int njobs;
+  int njobs, W;
   bool chained;
   cudaStream_t st;
 };
@@ -425,7 +425,7 @@ int pass_of(const Run &r, const PassArgs &a, PassKind kind) {
 template <class S, bool C>
 int inner_of(const Run &r, int P, uint32_t *buf, uint64_t job_words, const TernJobs &jobs) {
   CUOT_TRY(set_smem(tern_inner<S, C>, S::WORDS * 4));
-  launch_as(C, tern_inner<S, C>, dim3(P, 4, r.njobs), dim3(inner_threads<S>()), S::WORDS * 4, r.st, buf, job_words, jobs);
+  launch_as(C, tern_inner<S, C>, dim3(P, r.W, r.njobs), dim3(inner_threads<S>()), S::WORDS * 4, r.st, buf, job_words, jobs);
   return CUOT_OK;
 }
 template <class S, bool C>
@@ -471,17 +471,26 @@ void final_of(const Run &r, const uint32_t *buf, uint64_t job_words, const TernJ
             dim3((1u << E) / 256, 1, r.njobs), dim3(256), 0, r.st, buf, job_words, jobs);
 }
 
-// Input -> values at the points; *at: the half they are in.
-int forward(const Run &r, int e, PassKind kind, const TernJobs &jobs, uint32_t *half[2], uint64_t job_words, int *at) {
-  const int passes = tern_passes(tern_shape(e).m);
-  PassArgs a{e, 0, kind == kFirstBits ? 1 : 4, nullptr, half[0], job_words, jobs};
-  CUOT_TRY(pass(r, a, kind));
-  for (a.pass = 1; a.pass < passes; a.pass++) {
-    a.src = half[(a.pass - 1) & 1];
-    a.dst = half[a.pass & 1];
+// Passes first.. of the transform in half[0] (forward; the result's half in *at),
+// or back to pass 0.
+int passes_on(const Run &r, int e, int from, uint32_t *const half[2], uint64_t job_words, int *at) {
+  PassArgs a{e, 0, r.W, nullptr, nullptr, job_words, TernJobs{}};
+  for (a.pass = from; a.pass < tern_passes(tern_shape(e).m); a.pass++, *at ^= 1) {
+    a.src = half[*at];
+    a.dst = half[*at ^ 1];
     CUOT_TRY(pass(r, a, kForward));
   }
-  *at = (passes - 1) & 1;
+  return CUOT_OK;
+}
+int passes_back(const Run &r, int e, uint32_t *const half[2], uint64_t job_words, int *at) {
+  const TernShape s = tern_shape(e);
+  PassArgs a{e, 0, r.W, nullptr, nullptr, job_words, TernJobs{}};
+  for (a.pass = tern_passes(s.m) - 1; a.pass >= 0; a.pass--, *at ^= 1) {
+    a.src = half[*at];
+    a.dst = half[*at ^ 1];
+    // a single coset's pieces (y^m = 1) need no rotation in the end
+    CUOT_TRY(pass(r, a, a.pass || s.cosets == 1 ? kInverse : kLastInverse));
+  }
   return CUOT_OK;
 }
 
@@ -499,22 +508,23 @@ uint64_t tern_job_bytes(int e) { return 2 * group_words(e) * 16; }
 
 int tern_build_ahat(int e, const uint64_t *a_d, void *scratch, void *ahat, cudaStream_t st) {
   uint32_t *half[2] = {static_cast<uint32_t *>(scratch), static_cast<uint32_t *>(scratch) + group_words(e)};
-  const Run r{1, chain_launches(1ull << e, st), st};
-  TernJobs jobs{};
-  jobs.in[0] = reinterpret_cast<const uint32_t *>(a_d);
+  const Run r{1, 1, chain_launches(1ull << e, st), st};
+  PassArgs a{e, 0, 1, nullptr, half[0], 0, TernJobs{}};
+  a.jobs.in[0] = reinterpret_cast<const uint32_t *>(a_d);
   int at = 0;
-  CUOT_TRY(forward(r, e, kFirstBits, jobs, half, 0, &at));
+  CUOT_TRY(pass(r, a, kFirstBits));
+  CUOT_TRY(passes_on(r, e, 1, half, 0, &at));
   CUOT_TRY(consts(r, e, half[at], static_cast<uint32_t *>(ahat)));
   return launch_status(1 + tern_passes(tern_shape(e).m));
 }
 
-int tern_dual(int e, const TernJob *job, int njobs, void *scratch, cudaStream_t st) {
+int tern_dual(int e, const TernJob *job, int njobs, void *scratch, TernAux *aux, cudaStream_t st) {
   const TernShape s = tern_shape(e);
   if (njobs > kTernMaxJobs) return fail(CUOT_EINVAL, "%d dual LPNs in one launch (at most %d)", njobs, kTernMaxJobs);
-  const uint64_t job_words = group_words(e) * 4;
+  const uint64_t group = group_words(e), job_words = group * 4;
   uint32_t *half[2] = {static_cast<uint32_t *>(scratch), static_cast<uint32_t *>(scratch) + njobs * job_words};
   const int passes = tern_passes(s.m);
-  const Run r{njobs, chain_launches(uint64_t(njobs) << e, st), st};
+  Run r{njobs, 4, chain_launches(uint64_t(njobs) << e, st), st};
   TernJobs jobs{};
   for (int j = 0; j < njobs; j++) {
     jobs.in[j] = reinterpret_cast<const uint32_t *>(job[j].in);
@@ -522,15 +532,34 @@ int tern_dual(int e, const TernJob *job, int njobs, void *scratch, cudaStream_t 
     jobs.out[j] = reinterpret_cast<uint32_t *>(job[j].out);
     jobs.consts[j] = static_cast<const uint32_t *>(job[j].ahat);
   }
-  int at = 0;
-  CUOT_TRY(forward(r, e, kFirst, jobs, half, job_words, &at));
-  CUOT_TRY(inner(r, e, half[at], job_words, jobs));
-  PassArgs a{e, 0, 4, nullptr, nullptr, job_words, jobs};
-  for (a.pass = passes - 1; a.pass >= 0; a.pass--, at ^= 1) {
-    a.src = half[at];
-    a.dst = half[at ^ 1];
-    // a single coset's pieces (y^m = 1) need no rotation in the end
-    CUOT_TRY(pass(r, a, a.pass || s.cosets == 1 ? kInverse : kLastInverse));
+  CUOT_TRY(pass(r, PassArgs{e, 0, 4, nullptr, half[0], job_words, jobs}, kFirst));
+  int at = 0, launches = 2 * passes + 2;
+  if (aux) {
+    // The word groups are independent from here to the end: they alternate
+    // between two streams, so that one's kernels fill the other's wave tails
+    // and its passes (memory) run beside inner products (integer pipe).  Two
+    // groups at a time while a group's kernels are small (2^19: 187 us on one
+    // stream, 169 with pairs, 189 one by one; 2^20 386, 375, 377), one by one
+    // above (2^21 976, 940, 928; 2^22 2006, 1973, 1946).
+    r.W = e > 20 ? 1 : 2;
+    if (cudaEventRecord(aux->ev[0], st) != cudaSuccess || cudaStreamWaitEvent(aux->stream, aux->ev[0], 0) != cudaSuccess)
+      return launch_status(1);
+    for (int w = 0; w < 4; w += r.W) {
+      r.st = (w / r.W) & 1 ? aux->stream : st;
+      uint32_t *part[2] = {half[0] + w * group, half[1] + w * group};
+      at = 0;
+      CUOT_TRY(passes_on(r, e, 1, part, job_words, &at));
+      CUOT_TRY(inner(r, e, part[at], job_words, jobs));
+      CUOT_TRY(passes_back(r, e, part, job_words, &at));
+    }
+    r.st = st;
+    if (cudaEventRecord(aux->ev[1], aux->stream) != cudaSuccess || cudaStreamWaitEvent(st, aux->ev[1], 0) != cudaSuccess)
+      return launch_status(1);
+    launches += (4 / r.W - 1) * 2 * passes;
+  } else {
+    CUOT_TRY(passes_on(r, e, 1, half, job_words, &at));
+    CUOT_TRY(inner(r, e, half[at], job_words, jobs));
+    CUOT_TRY(passes_back(r, e, half, job_words, &at));
   }
   switch (e) {
 #define TERN_FINAL(E) \
@@ -539,7 +568,7 @@ int tern_dual(int e, const TernJob *job, int njobs, void *scratch, cudaStream_t 
     TERN_FINAL(19) TERN_FINAL(20) TERN_FINAL(21) TERN_FINAL(22)
 #undef TERN_FINAL
   }
-  return launch_status(2 * passes + 2);
+  return launch_status(launches);
 }
 
 }  // namespace cuot

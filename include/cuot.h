@@ -74,9 +74,10 @@ uint64_t cuot_ctx_scratch_bytes(const cuot_ctx *ctx);
  *                           2^22 FFTs, the NTT mod 469762049 above.  Plans
  *                           and batches keep the backend they were created
  *                           with; set it before creating them.
- *   CUOT_TUNE_QC_STREAMS    streams of one FFT encode, 1 or 2 (default 2:
- *                           groups of about 32 MiB of intermediate alternate
- *                           between the caller's stream and a second stream
+ *   CUOT_TUNE_QC_STREAMS    streams of one encode, 1 or 2 (default 2: an FFT's
+ *                           groups of about 32 MiB of intermediate, or the
+ *                           plane groups of a ternary transform of n >= 2^19,
+ *                           alternate between the caller's stream and a second stream
  *                           of the context, joined back before the call
  *                           returns).  1 keeps all work on the caller's
  *                           stream, for callers that already overlap several

@@ -190,3 +190,52 @@ def test_chained_launches_keep_the_order():
     torch.cuda.synchronize()
     for c in ctxs:
         c.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("e", [16, 19, 21])
+@pytest.mark.parametrize("streams", [1, 2])
+def test_captured_and_streamed(e, streams):
+    """Plans on one and two streams, one-shot and captured (also as a context's
+    first call of the size), with work on the caller's stream before and after."""
+    import cuot_b200
+    torch = pytest.importorskip("torch")
+    n = 1 << e
+    rng = np.random.default_rng(70 + e)
+    x = rng_blocks(rng, n)
+    a = to_dev(rng.integers(0, 1 << 63, n // 64, dtype=np.int64))
+    fft = _ctx(2)
+    want = to_dev(x)
+    fft.sot_dual_lpn(a, want, n)
+    want ^= 0x5A
+    ctx = _ctx()
+    ctx.set_tuning(ctx.TUNE_QC_STREAMS, streams)
+    ctx.reserve(1 << 30)
+    src, d = to_dev(x), torch.empty((n, 16), dtype=torch.uint8, device="cuda")
+    g = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g):
+        d.copy_(src)
+        ctx.sot_dual_lpn(a, d, n)
+        d.bitwise_xor_(0x5A)
+    plan = ctx.qc_plan(a, n)
+    g2 = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g2):
+        d.copy_(src)
+        plan.dual_lpn(d)
+        d.bitwise_xor_(0x5A)
+    for run in (g.replay, g2.replay, g.replay):
+        d.zero_()
+        run()
+        torch.cuda.synchronize()
+        assert torch.equal(d, want)
+    for _ in range(3):
+        d.copy_(src)
+        plan.dual_lpn(d)
+        d.bitwise_xor_(0x5A)
+    torch.cuda.synchronize()
+    assert torch.equal(d, want)
+    del plan
+    torch.cuda.synchronize()
+    ctx.close()
+    fft.close()
