@@ -78,6 +78,13 @@ __device__ __forceinline__ void group_sync(int group) {
   asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "n"(G) : "memory");
 }
 
+// XOR of a block value over the lanes of `mask` (all that call), in each of them.
+__device__ __forceinline__ Blk mask_xor(uint32_t mask, Blk v) {
+#pragma unroll
+  for (int i = 0; i < 4; i++) v.w[i] = __reduce_xor_sync(mask, v.w[i]);
+  return v;
+}
+
 // Expands tree `tree` of the instance described by `a` with a group of G
 // threads (tid: thread of the group).  slot: 2^h blocks for the ping-pong of the
 // levels above G nodes; smaller ones stay in shared memory, where a level costs
@@ -102,22 +109,84 @@ __device__ __forceinline__ void pprf_tree(const PprfArgs &a, bool sot, uint64_t 
   const uint64_t W = 1ull << h;
   Blk *const leaves = a.leaves + tree * W;
   Blk root{{0, 0, 0, 0}};
-  if (SEND) root = ldg_blk(a.roots + tree);
-  uint64_t ap = 0;  // receivers' path (first thread)
+  uint32_t bits = 0;  // receivers: choice bit of level l in bit l (h <= 30)
+  if (SEND) {
+    root = ldg_blk(a.roots + tree);
+  } else {
+    const bool c = lane < h && a.choice[sot ? uint64_t(lane) * a.t + tree : tree * h + lane];
+    bits = __ballot_sync(0xffffffffu, c);
+  }
+  uint64_t ap = 0;  // receivers' path
+  // Senders' outputs of level l from its left and right sums (one thread).
+  const auto send_sums = [&](int l, bool last, const Blk(&S)[2]) {
+    const uint64_t of = tree * h + l, os = uint64_t(l) * a.t + tree;
+    if (!sot) {
+      // ot_msg_0/1 of level l (spcot_sender.h:66-84), host layout [t][h]
+      st_blk(a.lsum + of, S[0]);
+      st_blk(a.rsum + of, S[1]);
+      if (last)  // secret_sum = XOR(masked leaves) ^ delta (spcot_sender.h:49-58)
+        st_blk(a.ss_out + tree, blk_xor(mask_lsb(blk_xor(S[0], S[1])), a.delta));
+    } else {
+      const Blk b0 = ldg_blk(a.base0 + os), b1 = ldg_blk(a.base1 + os);
+      st_blk(a.m0 + os, blk_xor(b0, S[0]));
+      st_blk(a.m1 + os, blk_xor(b1, S[1]));
+      if (last) {  // extra row that carries delta (silent/sender.cu:97-102)
+        st_blk(a.m0 + os + a.t, blk_xor(blk_xor(b0, S[1]), a.delta));
+        st_blk(a.m1 + os + a.t, blk_xor(blk_xor(b1, S[0]), a.delta));
+      }
+    }
+  };
 
   for (int l = 0; l < h; l++) {
     const bool last = (l == h - 1);
     const uint32_t np = 1u << l;  // h <= 30
     const Blk *in = np <= unsigned(G) ? sm.level(l) : (h - l) & 1 ? slot : leaves;
     Blk *out = !last && 2 * np <= unsigned(G) ? sm.level(l + 1) : (h - l) & 1 ? leaves : slot;
-    // receivers: the level's choice and message, on their way during the AES
-    Blk x0{{0, 0, 0, 0}};
-    int bit = 0;
-    const uint64_t of = tree * h + l, os = uint64_t(l) * a.t + tree;
-    if (!SEND && tid == 0) {
-      bit = a.choice[sot ? os : of] ? 1 : 0;
-      x0 = ldg_blk(a.mc + (sot ? os : of));
-      if (sot) x0 = blk_xor(x0, ldg_blk((bit ? a.m1_in : a.m0_in) + os));
+    // receivers: the level's message (and its mask), on the way during the AES
+    Blk x0{{0, 0, 0, 0}}, x1{{0, 0, 0, 0}};
+    const int bit = (bits >> l) & 1;
+    const uint64_t os = uint64_t(l) * a.t + tree;
+    const bool quick = np <= 32 && !last;
+    if (!SEND && (quick ? warp == bit && lane == int(ap) : tid == 0)) {
+      x0 = ldg_blk(a.mc + (sot ? os : tree * h + l));
+      if (sot) x1 = ldg_blk((bit ? a.m1_in : a.m0_in) + os);
+    }
+    // (without it the loading thread ran on by itself: 479 -> 679 us for 1,280 trees
+    // of depth 13)
+    if (!SEND) __syncwarp();
+    if (quick) {
+      // The chain of levels is what a small call waits for: about 2,000 cycles each
+      // here when one thread made both children (1,590 of issue and latency for the
+      // two AES) and one warp then finished the sums (570).  So a warp per side, a node
+      // per lane (1,100), and no sums on the chain: the senders' last warp adds up the
+      // children in shared memory while the others go on, and the receivers' sum of
+      // side `bit` is in one warp, whose lane `ap` has the node to mend.  16 trees of
+      // depth 10: Ferret 18.4 / 19.8 -> 16.9 / 18.2 us (sender / receiver), SOT
+      // 20.0 / 22.1 -> 17.1 / 18.7; 5,000 of depth 9: 163 / 169 -> 148 / 152.
+      if (warp < 2 && lane < int(np)) {
+        const Blk p = (l == 0) ? root : ld_blk(in + lane);
+        uint32_t x[4] = {p.w[0], p.w[1], p.w[2], p.w[3]};
+        aes_enc(T, x, c_ggm_rk[warp]);
+        Blk c{{x[0] ^ p.w[0], x[1] ^ p.w[1], x[2] ^ p.w[2], x[3] ^ p.w[3]}};
+        if (!SEND && warp == bit) {
+          const Blk s = mask_xor(uint32_t((1ull << np) - 1), c);
+          if (lane == int(ap)) c = blk_xor(blk_xor(c, s), blk_xor(x0, x1));
+        }
+        st_blk(out + 2 * lane + warp, c);
+      }
+      ap = 2 * ap + 1 - bit;
+      group_sync<G>(group);
+      if (SEND && warp == G / 32 - 1) {
+        Blk S[2] = {Blk{{0, 0, 0, 0}}, Blk{{0, 0, 0, 0}}};
+        if (lane < int(np)) {
+          S[0] = ld_blk(out + 2 * lane);
+          S[1] = ld_blk(out + 2 * lane + 1);
+        }
+        S[0] = warp_xor(S[0]);
+        S[1] = warp_xor(S[1]);
+        if (lane == 0) send_sums(l, last, S);
+      }
+      continue;
     }
     const uint32_t keep = last && !sot ? ~1u : ~0u;  // Ferret leaves: emp-ot `& one`
     Blk accL{{0, 0, 0, 0}}, accR{{0, 0, 0, 0}};
@@ -166,20 +235,8 @@ __device__ __forceinline__ void pprf_tree(const PprfArgs &a, bool sot, uint64_t 
         for (int i = 0; i < 4; i++) S[1].w[i] = __shfl_down_sync(0xffffffffu, v.w[i], 16);
       }
       if (lane == 0) {
-        if (SEND && !sot) {
-          // ot_msg_0/1 of level l (spcot_sender.h:66-84), host layout [t][h]
-          st_blk(a.lsum + of, S[0]);
-          st_blk(a.rsum + of, S[1]);
-          if (last)  // secret_sum = XOR(masked leaves) ^ delta (spcot_sender.h:49-58)
-            st_blk(a.ss_out + tree, blk_xor(mask_lsb(blk_xor(S[0], S[1])), a.delta));
-        } else if (SEND) {
-          const Blk b0 = ldg_blk(a.base0 + os), b1 = ldg_blk(a.base1 + os);
-          st_blk(a.m0 + os, blk_xor(b0, S[0]));
-          st_blk(a.m1 + os, blk_xor(b1, S[1]));
-          if (last) {  // extra row that carries delta (silent/sender.cu:97-102)
-            st_blk(a.m0 + os + a.t, blk_xor(blk_xor(b0, S[1]), a.delta));
-            st_blk(a.m1 + os + a.t, blk_xor(blk_xor(b1, S[0]), a.delta));
-          }
+        if (SEND) {
+          send_sums(l, last, S);
         } else if (!sot) {
           // spcot_recver.h:71-95: b = 0 -> fill the even child, puncture the odd.
           const uint64_t f = 2 * ap + bit, pun = 2 * ap + 1 - bit;
@@ -203,7 +260,7 @@ __device__ __forceinline__ void pprf_tree(const PprfArgs &a, bool sot, uint64_t 
           ap = pun;
         } else {  // SOT_RECV (silent/recver.cu:98-115, 143-155)
           const uint64_t f = 2 * ap + bit, pun = 2 * ap + 1 - bit;
-          st_blk(out + f, blk_xor(ld_blk(out + f), blk_xor(x0, bit ? S[1] : S[0])));
+          st_blk(out + f, blk_xor(ld_blk(out + f), blk_xor(blk_xor(x0, x1), bit ? S[1] : S[0])));
           if (last) {
             const Blk dec2 = blk_xor(ldg_blk((bit ? a.m1_in : a.m0_in) + os + a.t), ldg_blk(a.mc + os));
             st_blk(out + pun, blk_xor(ld_blk(out + pun), blk_xor(dec2, bit ? S[0] : S[1])));
@@ -238,10 +295,10 @@ __global__ void __launch_bounds__(kPprfThreads, 3) pprf_tree_kernel(PprfArgs a) 
 // Threads per tree for `trees` trees (the deepest of depth h) on `ctas` resident
 // CTAs.  Shallow levels leave most of a large group idle, so with enough trees
 // to fill the chip several smaller groups share a CTA.  Measured on B200
-// (Ferret sender, 256 / 128 / 64 threads): 64 trees of depth 10 22.5 / 24.3 /
-// 30.5 us, 300 34.6 / 34.5 / 38.7, 918 of depth 9 49 / 43 / 45, 1,280 of depth 13
-// 475 / 470 / 483, 1,500 of depth 10 107 / 107 / 92, 4,971 of depth 11 549 / 516 /
-// 464, 5,000 of depth 9 221 / 211 / 162 (one CTA per tree and launch before: 277).
+// (Ferret sender, 256 / 128 / 64 threads): 64 trees of depth 10 17.4 / 17.6 /
+// 24.6 us, 300 33.5 / 32.9 / 39.2, 918 of depth 9 45 / 41 / 41, 1,280 of depth 13
+// 463 / 468 / 485, 1,500 of depth 10 102 / 99 / 90, 4,971 of depth 11 519 / 490 /
+// 458, 5,000 of depth 9 203 / 194 / 148 (one CTA per tree and launch before: 277).
 inline int pprf_group_size(uint64_t trees, int h, uint64_t ctas) {
   return trees <= ctas ? 256 : trees <= 3 * ctas || h > 12 ? 128 : 64;
 }
