@@ -468,152 +468,132 @@ __global__ void prg_make_counters(Blk *b, uint64_t nb, uint64_t off) {
   }
 }
 
-// Sparse encode: out = XOR_i rot(a, pos_i).  Grid: x over output words (256
-// consecutive words per CTA, so the reads of `a` coalesce), y over chunks of
-// kSparseChunk positions staged in shared memory; each thread XORs its
-// chunk's partial into out (zeroed by the caller) with one 64-bit atomic.
-// r2 (rate-1/2 noise of 2n positions): positions p < n contribute x^p
-// itself, positions p in [n, 2n) contribute rot(a, p - n).
-constexpr int kSparseChunk = 256;
-__global__ void __launch_bounds__(256) qc_sparse(const uint64_t *__restrict__ a, const uint64_t *__restrict__ pos,
-                                                 int weight, uint64_t n, uint64_t *__restrict__ out, int r2) {
-  __shared__ uint64_t sp[kSparseChunk];
-  const uint64_t nw = n / 64;
-  const int i0 = blockIdx.y * kSparseChunk;
-  const int cnt = min(kSparseChunk, weight - i0);
-  for (int i = threadIdx.x; i < cnt; i += blockDim.x) sp[i] = __ldg(&pos[i0 + i]);
-  __syncthreads();
-  const uint64_t w = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (w >= nw) return;
-  uint64_t acc = 0;
+// Sparse encode: out = XOR_i rot(a, pos_i).  A CTA makes 32 V output words; its NW
+// warps take every NW-th position each, so that a word's chain of loads is short,
+// and add up through shared memory.  One CTA per word tile stores its words;
+// several (grid y: few words and many positions) XOR them into the zeroed
+// output.  Positions >= n contribute nothing.  R2 (rate-1/2 noise of 2n
+// positions): positions p < n contribute x^p itself, positions p in [n, 2n)
+// contribute rot(a, p - n).
+//
+// Bound by the L1 wavefronts of the unaligned word loads (about six per 32 words
+// and position) for many positions, by latency for few.  `a` comes from L2 and
+// L1: staging the positions' common window in shared memory, with one CTA per 256
+// words, left most of the chip idle below n = 2^20 and recomputed a 64-bit
+// modulus per staged word.  Measured on B200, that form against this one, one
+// position per tree of 2^h: n = 2^17, h = 11 14.7 / 8.7 us, 2^20 and 12 17.9 / 10.3,
+// 2^22 and 14 42 / 19, 2^24 and 14 491 / 183, 2^26 and 14 7,649 / 2,646; 5,000
+// random positions at 2^20 150 / 68.
+template <bool R2, int V, int NW, bool CHAINED>
+__global__ void __launch_bounds__(32 * NW) qc_sparse(const uint64_t *a, const uint64_t *pos, int weight, uint64_t n,
+                                                     uint64_t *out) {
+  __shared__ uint64_t red[NW][32 * V];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t zero = chain_begin<CHAINED>();
+  a += zero;
+  pos += zero;
+  const uint64_t nw = n / 64, t0 = uint64_t(blockIdx.x) * (32 * V), t1 = t0 + 32 * V;
+  uint64_t acc[V];
+#pragma unroll
+  for (int k = 0; k < V; k++) acc[k] = 0;
+  constexpr int kStep = 32 * NW;  // positions of the CTA at a time
+  for (int b = blockIdx.y * kStep; b < weight; b += gridDim.y * kStep) {
+    const int i = b + lane * NW + warp;
+    const uint64_t p_l = i < weight ? __ldg(&pos[i]) : ~0ull;
+    const int left = weight - b - warp, cnt = left <= 0 ? 0 : (left + NW - 1) / NW, n_j = cnt < 32 ? cnt : 32;
 #pragma unroll 4
-  for (int i = 0; i < cnt; i++) {
-    uint64_t p = sp[i];
-    if (r2) {
-      if (p < n) {
-        if ((p >> 6) == w) acc ^= 1ull << (p & 63);
+    for (int j = 0; j < n_j; j++) {
+      uint64_t p = __shfl_sync(0xffffffffu, p_l, j);
+      if (R2) {
+        if (p < n) {  // x^p
+          const uint64_t w = p >> 6;
+          if (w >= t0 && w < t1)
+#pragma unroll
+            for (int k = 0; k < V; k++)
+              if (w == t0 + 32 * k + lane) acc[k] ^= 1ull << (p & 63);
+          continue;
+        }
+        p -= n;
+      }
+      if (p >= n) continue;
+      const uint64_t ws = p >> 6;
+      const int bs = int(p & 63);
+      // bit (64w + b) of rot(a, p) = bit (64w + b - p) mod n of a
+      if (t1 <= nw && (t0 > ws || t1 <= ws)) {  // a whole tile that does not wrap around in `a`
+        const uint64_t *src = a + (t0 > ws ? t0 - ws : t0 + nw - ws) + lane;
+        // 64 shifted bits come from three 32-bit words: an 8-byte load and a 4-byte one
+        if (bs < 32) {
+#pragma unroll
+          for (int k = 0; k < V; k++) {
+            const uint64_t c = __ldg(src + 32 * k);
+            const uint32_t d = __ldg(reinterpret_cast<const uint32_t *>(src + 32 * k) - 1);
+            acc[k] ^= uint64_t(__funnelshift_l(uint32_t(c), uint32_t(c >> 32), bs)) << 32 |
+                      __funnelshift_l(d, uint32_t(c), bs);
+          }
+        } else {
+#pragma unroll
+          for (int k = 0; k < V; k++) {
+            const uint32_t c = __ldg(reinterpret_cast<const uint32_t *>(src + 32 * k));
+            const uint64_t d = __ldg(src + 32 * k - 1);
+            acc[k] ^= uint64_t(__funnelshift_l(uint32_t(d >> 32), c, bs)) << 32 |
+                      __funnelshift_l(uint32_t(d), uint32_t(d >> 32), bs);  // (shifts by bs mod 32)
+          }
+        }
         continue;
       }
-      p -= n;
-    }
-    if (p >= n) continue;
-    const uint64_t ws = p >> 6, bs = p & 63;
-    // bit (64w + b) of rot(a, p) = bit (64w + b - p) mod n of a
-    const uint64_t src = w >= ws ? w - ws : w + nw - ws;
-    uint64_t v = __ldg(&a[src]) << bs;
-    if (bs) v |= __ldg(&a[src ? src - 1 : nw - 1]) >> (64 - bs);
-    acc ^= v;
-  }
-  if (acc) atomicXor(reinterpret_cast<unsigned long long *>(out + w), (unsigned long long)acc);
-}
-
-// Window form of the sparse encode (r2 = 0, fewer than 2^31 output words).
-// Positions listed in tree order (one punctured leaf per GGM tree of 2^h
-// leaves) lie close together, so the 257-word windows of `a` that a chunk's
-// positions rotate into the CTA's 256 output words overlap almost entirely:
-// the CTA stages their union (span + 257 words, span = the chunk's largest
-// minus smallest word shift) in shared memory once, and every (word,
-// position) pair then reads shared memory instead of L2.  A chunk whose
-// positions spread wider than kSparseWin (any order is accepted) takes the
-// global-memory loop of qc_sparse.  Positions >= n contribute nothing, as
-// there.
-constexpr int kSparseWin = 4608;  // words of `a` (36 KiB)
-__global__ void __launch_bounds__(256) qc_sparse_win(const uint64_t *__restrict__ a, const uint64_t *__restrict__ pos,
-                                                     int weight, int chunk, uint64_t n, uint64_t *__restrict__ out) {
-  __shared__ uint64_t win[kSparseWin];
-  __shared__ uint32_t sws[kSparseChunk];  // word shift, or ~0u for a position >= n
-  __shared__ uint8_t sbs[kSparseChunk];   // bit shift
-  __shared__ unsigned long long wmin, wmax;
-  const uint64_t nw = n / 64;
-  const int i0 = blockIdx.y * chunk;
-  const int cnt = min(chunk, weight - i0);
-  if (threadIdx.x == 0) {
-    wmin = ~0ull;
-    wmax = 0;
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
-    const uint64_t p = __ldg(&pos[i0 + i]);
-    if (p < n) {
-      sws[i] = uint32_t(p >> 6);
-      sbs[i] = uint8_t(p & 63);
-      atomicMin(&wmin, (unsigned long long)(p >> 6));
-      atomicMax(&wmax, (unsigned long long)(p >> 6));
-    } else {
-      sws[i] = ~0u;
-    }
-  }
-  __syncthreads();
-  if (wmin > wmax) return;  // no position below n in this chunk (the same for every thread)
-  const uint64_t span = wmax - wmin;
-  const uint64_t w = uint64_t(blockIdx.x) * 256 + threadIdx.x;
-  uint64_t acc = 0;
-  if (span + 257 <= uint64_t(kSparseWin)) {
-    // win[j] = a[(W0 - wmax - 1 + j) mod nw], W0 = the CTA's first output word;
-    // word w = W0 + t under word shift ws needs a[w - ws] = win[t + wmax - ws + 1]
-    // and its lower neighbour win[t + wmax - ws], both inside [0, span + 257)
-    const uint64_t start = (uint64_t(blockIdx.x) * 256 + nw - wmax - 1) % nw;
-    const int len = int(span) + 257;
-    for (int j = threadIdx.x; j < len; j += blockDim.x) win[j] = __ldg(&a[(start + uint64_t(j)) % nw]);
-    __syncthreads();
-    if (w < nw) {
-      const int t1 = int(threadIdx.x) + int(wmax) + 1;
-#pragma unroll 4
-      for (int i = 0; i < cnt; i++) {
-        const uint32_t ws = sws[i];
-        if (ws == ~0u) continue;
-        const int bs = sbs[i];
-        const int idx = t1 - int(ws);
-        uint64_t v = win[idx] << bs;
-        if (bs) v |= win[idx - 1] >> (64 - bs);
-        acc ^= v;
+#pragma unroll
+      for (int k = 0; k < V; k++) {
+        const uint64_t w = t0 + 32 * k + lane;
+        if (w >= nw) continue;
+        const uint64_t at = w >= ws ? w - ws : w + nw - ws;
+        acc[k] ^= (__ldg(&a[at]) << bs) ^ (__ldg(&a[at ? at - 1 : nw - 1]) >> 1 >> (63 - bs));
       }
     }
-  } else if (w < nw) {
-    for (int i = 0; i < cnt; i++) {
-      const uint32_t ws32 = sws[i];
-      if (ws32 == ~0u) continue;
-      const uint64_t ws = ws32;
-      const int bs = sbs[i];
-      const uint64_t src = w >= ws ? w - ws : w + nw - ws;
-      uint64_t v = __ldg(&a[src]) << bs;
-      if (bs) v |= __ldg(&a[src ? src - 1 : nw - 1]) >> (64 - bs);
-      acc ^= v;
-    }
   }
-  if (w < nw && acc) atomicXor(reinterpret_cast<unsigned long long *>(out + w), (unsigned long long)acc);
+#pragma unroll
+  for (int k = 0; k < V; k++) red[warp][32 * k + lane] = acc[k];
+  __syncthreads();
+  for (int t = threadIdx.x; t < 32 * V; t += 32 * NW) {
+    uint64_t x = 0;
+#pragma unroll
+    for (int k = 0; k < NW; k++) x ^= red[k][t];
+    const uint64_t w = uint64_t(blockIdx.x) * (32 * V) + t;
+    if (w >= n / 64) continue;
+    if (gridDim.y == 1)
+      out[w] = x;
+    else if (x)
+      atomicXor(reinterpret_cast<unsigned long long *>(out + w), (unsigned long long)x);
+  }
+}
+
+template <int V, int NW, bool CHAINED>
+static int launch_sparse_as(const uint64_t *a_d, const uint64_t *pos_d, int weight, uint64_t n, uint64_t *out_d,
+                            int r2, cudaStream_t st) {
+  const uint64_t gx = (n / 64 + 32 * V - 1) / (32 * V);
+  // 64 positions per warp at least, and no more CTAs than fill the chip several times
+  const uint64_t most = (uint64_t(weight) + 1023) / 1024, fill = (2048 + gx - 1) / gx;
+  const uint64_t gy = most < fill ? most : fill;
+  if (gy > 1 && cudaMemsetAsync(out_d, 0, n / 8, st) != cudaSuccess) return launch_status(0);
+  launch_as(CHAINED, r2 ? qc_sparse<true, V, NW, CHAINED> : qc_sparse<false, V, NW, CHAINED>,
+            dim3(unsigned(gx), unsigned(gy)), dim3(32 * NW), 0, st, a_d, pos_d, weight, n, out_d);
+  return launch_status();
 }
 
 static int launch_sparse(const uint64_t *a_d, const uint64_t *pos_d, int weight, uint64_t n, uint64_t *out_d,
                          int r2, cudaStream_t st) {
-  if (cudaMemsetAsync(out_d, 0, n / 8, st) != cudaSuccess) return launch_status(0);
-  if (weight == 0) return launch_status(0);
-  const uint64_t nw = n / 64;
-  const unsigned gx = unsigned((nw + 255) / 256);
-  const bool win = !r2 && nw < (1ull << 31);
-  // Window chunk: in tree order (one position in each run of n / weight
-  // bits) `chunk` consecutive positions span less than chunk * n / weight
-  // bits, i.e. chunk * nw / weight words; the chunk is chosen so that this
-  // fits kSparseWin - 257 (a multiple of 32 in [32, kSparseChunk]).
-  int chunk = kSparseChunk;
-  if (win) {
-    const uint64_t sp = nw / uint64_t(weight) > 1 ? nw / uint64_t(weight) : 1;
-    const uint64_t c = uint64_t(kSparseWin - 257) / sp;
-    chunk = c >= uint64_t(kSparseChunk) ? kSparseChunk : c < 32 ? 32 : int(c / 32 * 32);
+  if (weight == 0) {
+    if (cudaMemsetAsync(out_d, 0, n / 8, st) != cudaSuccess) return launch_status(0);
+    return launch_status(0);
   }
-  // at most 65,535 chunks per launch (grid y)
-  const int per_launch = 65535 * chunk;
-  int launches = 0;
-  for (int off = 0; off < weight; off += per_launch) {
-    const int wpart = weight - off < per_launch ? weight - off : per_launch;
-    const dim3 grid(gx, unsigned((wpart + chunk - 1) / chunk));
-    if (win)
-      qc_sparse_win<<<grid, 256, 0, st>>>(a_d, pos_d + off, wpart, chunk, n, out_d);
-    else
-      qc_sparse<<<grid, 256, 0, st>>>(a_d, pos_d + off, wpart, n, out_d, r2);
-    launches++;
-  }
-  return launch_status(launches);
+  const bool chained = chain_launches(n, st);
+  // Few words: small tiles, or most SMs stay idle (n = 2^10 with 20,000 positions
+  // 17 against 25 us).  From 2^16 on the wide tile is as fast or faster: it loads a
+  // position's words independently (2^17 with 2^17 positions 189 against 490).
+  if (n / 64 <= 512)
+    return chained ? launch_sparse_as<1, 16, true>(a_d, pos_d, weight, n, out_d, r2, st)
+                   : launch_sparse_as<1, 16, false>(a_d, pos_d, weight, n, out_d, r2, st);
+  return chained ? launch_sparse_as<4, 16, true>(a_d, pos_d, weight, n, out_d, r2, st)
+                 : launch_sparse_as<4, 16, false>(a_d, pos_d, weight, n, out_d, r2, st);
 }
 
 // ---------------------------------------------------------------------------
