@@ -75,14 +75,22 @@ constexpr int kTrG = 32;
 constexpr int kTrCh = kTrG / 4;                   // 16-byte chunks per plane row
 constexpr int kTrCpw = kTrCh / (kTrThreads / 32);  // chunks per warp
 static_assert(kTrCpw >= 1 && kTrCh >= 8, "tile shape");
+// The 128-plane kernels are chained up to 16 times the general limit, 2^22 blocks:
+// their few waves of CTAs then start while the kernel before drains (to planes and
+// back, 2^21 blocks: 27.1 -> 25.0 us, 2^22 47.7 -> 46.4, 2^24 no difference).
+// Bound by the two trips through memory, and by the last wave (8 CTAs per SM, 1.7
+// waves at 2^21).
+constexpr uint64_t kTrChain = 16;
 
 // blocks -> planes, all 128 planes.  in: rows x 16 bytes (rows % 128 == 0).
 // out: 128 rows of rows / 8 bytes.
+template <bool CHAINED>
 __global__ void __launch_bounds__(kTrThreads) tr_blocks_to_planes128(const uint4 *__restrict__ in, uint64_t rows,
                                                                      uint4 *__restrict__ out) {
   __shared__ uint4 st[128 * kTrCh];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const TrLane tl = tr_lane(lane);
+  in += chain_begin<CHAINED>();
   const uint64_t ngroups = rows / 32;
   const uint64_t g0 = uint64_t(blockIdx.x) * kTrG;
   const int gvalid = int(ngroups - g0 < uint64_t(kTrG) ? ngroups - g0 : uint64_t(kTrG));  // multiple of 4
@@ -121,11 +129,13 @@ __global__ void __launch_bounds__(kTrThreads) tr_blocks_to_planes128(const uint4
 // planes -> blocks, 128 planes.  in: 128 rows of in_row4 16-byte words, of
 // which the first ncols / 128 are read (ncols % 128 == 0).  out: ncols rows of
 // 16 bytes.
+template <bool CHAINED>
 __global__ void __launch_bounds__(kTrThreads) tr_planes128_to_blocks(const uint4 *__restrict__ in, uint64_t ncols,
                                                                      uint64_t in_row4, uint4 *__restrict__ out) {
   __shared__ uint4 st[128 * kTrCh];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const TrLane tl = tr_lane(lane);
+  in += chain_begin<CHAINED>();
   const uint64_t ngroups = ncols / 32;
   const uint64_t g0 = uint64_t(blockIdx.x) * kTrG;
   const int gvalid = int(ngroups - g0 < uint64_t(kTrG) ? ngroups - g0 : uint64_t(kTrG));  // multiple of 4
@@ -388,16 +398,18 @@ int transpose_launch(const void *in, uint64_t rows, uint64_t row_bytes, uint64_t
   if (row_bytes == 16 && rows % 128 == 0 && col_lo == 0 && ncols == 128 && aligned(in, 16) && aligned(out, 16)) {
     const uint64_t grid = (rows / 32 + kTrG - 1) / kTrG;
     if (grid > 0x7fffffffull) return fail(CUOT_EINVAL, "too many rows");
-    tr_blocks_to_planes128<<<unsigned(grid), kTrThreads, 0, st>>>(static_cast<const uint4 *>(in), rows,
-                                                                   static_cast<uint4 *>(out));
+    const bool chained = chain_launches(rows / kTrChain, st);
+    launch_as(chained, chained ? tr_blocks_to_planes128<true> : tr_blocks_to_planes128<false>, dim3(unsigned(grid)),
+              dim3(kTrThreads), 0, st, static_cast<const uint4 *>(in), rows, static_cast<uint4 *>(out));
     return launch_status();
   }
   if (rows == 128 && col_lo == 0 && ncols % 128 == 0 && ncols <= row_bytes * 8 && row_bytes % 16 == 0 &&
       aligned(in, 16) && aligned(out, 16)) {
     const uint64_t grid = (ncols / 32 + kTrG - 1) / kTrG;
     if (grid > 0x7fffffffull) return fail(CUOT_EINVAL, "too many columns");
-    tr_planes128_to_blocks<<<unsigned(grid), kTrThreads, 0, st>>>(static_cast<const uint4 *>(in), ncols,
-                                                                   row_bytes / 16, static_cast<uint4 *>(out));
+    const bool chained = chain_launches(ncols / kTrChain, st);
+    launch_as(chained, chained ? tr_planes128_to_blocks<true> : tr_planes128_to_blocks<false>, dim3(unsigned(grid)),
+              dim3(kTrThreads), 0, st, static_cast<const uint4 *>(in), ncols, row_bytes / 16, static_cast<uint4 *>(out));
     return launch_status();
   }
   const bool all_planes = row_bytes == 16 && col_lo == 0 && ncols == 128 && aligned(in, 16);
