@@ -288,6 +288,7 @@ NCU_TRAFFIC_PER_STEP = {
 
 QC_FFT_MAX_LOG_N = 22  # the fp64 FFT encodes n <= 2^22 (exactness bound)
 QC_KARA_MAX_LOG_N = 24  # dual LPNs up to 2^24: GF(2) Karatsuba over 2^22 FFTs; the NTT above
+QC_TERN_LOG_N = (14, 22)  # dual LPNs that take the ternary GF(2) transform (backend auto)
 
 
 def qc_leaves(lg: int) -> int:
@@ -300,6 +301,11 @@ def qc_leaves(lg: int) -> int:
     return 0
 QC_BACKENDS = {"auto": 0, "ntt": 1, "fft": 2}
 _qc_backend = 0
+
+
+def qc_ternary(lg: int) -> bool:
+    """Whether a dual LPN of n = 2^lg runs on the ternary transform."""
+    return _qc_backend == 0 and QC_TERN_LOG_N[0] <= lg <= QC_TERN_LOG_N[1]
 
 
 def new_context(cuot_b200, device: int):
@@ -345,6 +351,20 @@ def qc_transform_report(ns, ms: float, fp64_peak: float | None = None) -> dict:
             out["fp64_peak_method"] = ("cuot_measure_fp64_tflops: 8 independent FMA chains per thread, 2048 "
                                        "threads per SM, best of 5 launches of ~9 ms, 2 flops per FMA")
     return out
+
+
+def qc_report(ns, ms: float, measure_fp64) -> dict:
+    """The encode's report for the transforms that run: sizes of the ternary
+    transform do bit logic (no fp64 work to rate), others as
+    qc_transform_report.  measure_fp64: called for the fp64 peak if needed."""
+    other = [n for n in ns if not qc_ternary(n.bit_length() - 1)]
+    if len(other) == len(ns):
+        return qc_transform_report(ns, ms, measure_fp64())
+    return {"backend": "ternary GF(2) transform (2^14 <= n <= 2^22) / fft below / karatsuba over 2^22 ffts (2^23, "
+                       "2^24) / ntt (larger n)",
+            "stage_ms": ms, "ternary_coefficients": sum(2 * n for n in ns) - sum(2 * n for n in other),
+            **qc_transform_work(other),
+            "model": "ternary: coefficients of both roles, 128 planes each; the stage time covers all sizes"}
 
 
 def fp64_roofline(qct: dict) -> dict | None:
@@ -1012,8 +1032,8 @@ def run_batch(args):
                               "2,757 per COT for smaller FFT sizes; 4,066 per COT for NTT sizes "
                               "(profiles/qc_ntt_sot_n20.md)"},
         "aes_roofline": aes,
-        "qc_transform": qc_transform_report([i.n for i in insts if i.kind != KIND_FERRET], stages["sot_encode"],
-                                            ctx.measure_fp64_tflops()),
+        "qc_transform": qc_report([i.n for i in insts if i.kind != KIND_FERRET], stages["sot_encode"],
+                                  ctx.measure_fp64_tflops),
         "e2e": {"value": world * cots / (e2e_ms / 1e3), "unit": "COTs/s", "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h, "ms_per_step": e2e_ms,
                 "method": "steps back to back through Batch.run with two device input/output sets; each "
@@ -1398,7 +1418,7 @@ def run_ours(args):
     if inst.spec["kind"] == "sot":
         out["transpose"] = transpose_roofline(inst, flush, peaks, peak_kind)
     if inst.spec["kind"] == "sot":
-        out["qc_transform"] = qc_transform_report([inst.n], lpn_ms, inst.sctx.measure_fp64_tflops())
+        out["qc_transform"] = qc_report([inst.n], lpn_ms, inst.sctx.measure_fp64_tflops)
         if dom == "dual_lpn" and fp64_roofline(out["qc_transform"]):
             out["roofline"]["fp64"] = fp64_roofline(out["qc_transform"])
     if rank == 0 and world == 1:
@@ -1439,8 +1459,8 @@ def main():
                     help="batched mix: one chain (default), the Ferret branch beside the SOT chain, or every SOT "
                          "size on its own stream too")
     ap.add_argument("--qc-backend", default="auto", choices=sorted(QC_BACKENDS),
-                    help="transform of the exact QC encode (auto: fp64 FFT for n <= 2^22, Karatsuba over it for "
-                         "dual LPNs at 2^23 and 2^24, NTT above)")
+                    help="transform of the exact QC encode (auto: dual LPNs by the ternary GF(2) transform from "
+                         "2^14 to 2^22, the fp64 FFT below, Karatsuba over it at 2^23 and 2^24, NTT above)")
     args = ap.parse_args()
     global _qc_backend
     _qc_backend = QC_BACKENDS[args.qc_backend]
