@@ -123,17 +123,19 @@ int launch_split(cuot_ctx *ctx, const LpnArgs &a, cudaStream_t st) {
 // copy, 10,485,760 rows 1197 -> 927; at 131,072 rows the 3 us that the gathers
 // would save are the copy's launch).  Not while `st` is captured: the arena may
 // neither grow then nor, as far as this call goes, stay where it is until the
-// graph runs.
+// graph runs.  Nor if an arena is there and would have to grow for it (a caller's
+// graph may hold the old one), or none can be had: the plain form needs no scratch.
 constexpr int64_t kInterleaveRows = 1 << 18;
 int launch_dual(cuot_ctx *ctx, LpnArgs a, cudaStream_t st) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  const uint64_t bytes = uint64_t(a.k) * 32;
+  void *scr = nullptr;
   if (a.ngroups * 4 < kInterleaveRows || a.k > a.ngroups || cudaStreamIsCapturing(st, &cap) != cudaSuccess ||
-      cap != cudaStreamCaptureStatusNone) {
+      cap != cudaStreamCaptureStatusNone || (ctx->scratch && ctx->scratch_bytes < bytes) ||
+      scratch(ctx, bytes, &scr) != CUOT_OK) {
     cudaGetLastError();
     return launch_split<kTwoRoles>(ctx, a, st);
   }
-  void *scr = nullptr;
-  CUOT_TRY(scratch(ctx, uint64_t(a.k) * 32, &scr));
   a.kk12 = static_cast<Blk *>(scr);
   const int64_t grid = (a.k + 255) / 256;
   lpn_interleave_kernel<<<unsigned(grid < 148 * 8 ? grid : 148 * 8), 256, 0, st>>>(a);

@@ -54,6 +54,23 @@ def test_both_roles(n, k, captured):
     ctx.close()
 
 
+def test_both_roles_keep_a_smaller_arena():
+    """The context's scratch is too small for the interleaved copy: it stays (a graph may hold it)."""
+    import cuot_b200
+    ctx = cuot_b200.Context(0)
+    n, k, t, h = (1 << 18) + 8, 65536, 3, 9
+    rng = np.random.default_rng(3)
+    roots, out = to_dev(rng_blocks(rng, t)), [torch.empty((m, 16), dtype=torch.uint8, device="cuda")
+                                              for m in (t << h, t * h, t * h, t)]
+    ctx.ferret_pprf_sender(roots, h, bytes(16), *out)
+    seed, kk, e = rng_blocks(rng, 1)[0], rng_blocks(rng, 2 * k).reshape(2, k, 16), rng_blocks(rng, 2 * n).reshape(2, n, 16)
+    de = [to_dev(x) for x in e]
+    ctx.lpn_primal_dual(seed, to_dev(kk[0]), to_dev(kk[1]), de[0], de[1])
+    for r in range(2):
+        assert np.array_equal(to_host(de[r]), oracle.lpn_primal(seed, kk[r], e[r], threads=8)), r
+    ctx.close()
+
+
 @pytest.mark.parametrize("rows", [0, 4, 1000])
 def test_batched_tasks(ctx, rows):
     from cuot_b200.batch import KIND_FERRET, Batch, Instance
