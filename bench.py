@@ -274,17 +274,19 @@ class Instance:
 # kernel and one to three launches per capture (ncu starts every launch with
 # cold caches, so intermediate that steady state keeps in L2 is counted):
 # ferret_b13: the dual-role LPN launch (profiles/pprf_lpn_ferret_b13.md);
-# sot_n20: gather, 16 launches of each transform pass and scatter per role
+# sot_n20_fft: gather, 16 launches of each transform pass and scatter per role
 # (profiles/qc_fft_sot_n20.md); sot_n20_ntt: the same workload on the NTT
 # backend, which scales the SOT encodes of NTT sizes (profiles/qc_ntt_sot_n20.md);
-# sot_n22: 32 transforms of 251.8 MB per role plus gather and scatter
+# sot_n22_fft: 32 transforms of 251.8 MB per role plus gather and scatter
 # (profiles/qc_fft_sot_n22.md).
 NCU_TRAFFIC_PER_STEP = {
     "ferret_b13:lpn": 631.83e6,
-    "sot_n20:dual_lpn": 2 * (16.79e6 + 16 * 88.24e6 + 16.86e6),
+    "sot_n20_fft:dual_lpn": 2 * (16.79e6 + 16 * 88.24e6 + 16.86e6),
     "sot_n20_ntt:dual_lpn": 2 * (509.60e6 + 1024.36e6 + 563.98e6 + 33.58e6),
-    "sot_n22:dual_lpn": 2 * (32 * 251.75e6 + 84.17e6 + 82.25e6),
+    "sot_n22_fft:dual_lpn": 2 * (32 * 251.75e6 + 84.17e6 + 82.25e6),
 }
+# The same for one ternary dual LPN of n = 2^key (profiles/qc_ternary.md).
+NCU_TERNARY_TRAFFIC = {16: 33.85e6, 17: 65.45e6, 18: 99.05e6, 19: 203.32e6, 20: 497.11e6, 21: 2013.97e6, 22: 4921.76e6}
 
 QC_FFT_MAX_LOG_N = 22  # the fp64 FFT encodes n <= 2^22 (exactness bound)
 QC_KARA_MAX_LOG_N = 24  # dual LPNs up to 2^24: GF(2) Karatsuba over 2^22 FFTs; the NTT above
@@ -977,21 +979,25 @@ def run_batch(args):
     peaks, peak_kind = measured_peaks()
     achieved = alg[dom] / (stages[dom] / 1e3) / 1e9
     # traffic: the batch is too large for a multi-metric ncu capture; the SOT
-    # encode runs the same kernels as the single-instance sot_n20 / sot_n22
-    # lines (FFT up to 2^22, Karatsuba over 2^22 FFTs at 2^23 and 2^24, NTT
+    # encode runs the same kernels as the single-instance lines (ternary from
+    # 2^14 to 2^22, FFT below, Karatsuba over 2^22 FFTs at 2^23 and 2^24, NTT
     # above), whose captured DRAM bytes per COT (both roles) scale it: the
     # 2^22 capture for the 1024 x 4096 split of 2^22 (and the Karatsuba
     # leaves), the 2^20 capture below; other stages have no capture (null)
     traffic = None
     if dom == "sot_encode":
-        fft_cot = NCU_TRAFFIC_PER_STEP["sot_n20:dual_lpn"] / (1 << 20)  # FFT dual LPN, both roles
-        fft22_cot = NCU_TRAFFIC_PER_STEP["sot_n22:dual_lpn"] / (1 << 22)
+        fft_cot = NCU_TRAFFIC_PER_STEP["sot_n20_fft:dual_lpn"] / (1 << 20)  # FFT dual LPN, both roles
+        fft22_cot = NCU_TRAFFIC_PER_STEP["sot_n22_fft:dual_lpn"] / (1 << 22)
         ntt_cot = NCU_TRAFFIC_PER_STEP["sot_n20_ntt:dual_lpn"] / (1 << 20)
         traffic = 0.0
         for i in insts:
             if i.kind == KIND_FERRET:
                 continue
             lg = i.n.bit_length() - 1
+            if qc_ternary(lg):
+                traffic += 2 * NCU_TERNARY_TRAFFIC[max(e for e in NCU_TERNARY_TRAFFIC if e <= max(lg, 16))] * (
+                    i.n / (1 << max(e for e in NCU_TERNARY_TRAFFIC if e <= max(lg, 16))))
+                continue
             leaves = qc_leaves(lg)
             per = fft22_cot if lg >= QC_FFT_MAX_LOG_N else fft_cot
             traffic += per * leaves * min(i.n, 1 << QC_FFT_MAX_LOG_N) if leaves else i.n * ntt_cot
@@ -1026,10 +1032,10 @@ def run_batch(args):
                      "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)",
                      "algorithmic_bytes_per_step": alg[dom],
                      "basis": "stage totals per step (both roles); traffic scaled from one-kernel ncu "
-                              "captures of the single-instance lines (cold cache per kernel): n = 2^22 "
-                              "(profiles/qc_fft_sot_n22.md) 3,921 DRAM bytes per COT for the 2^22 instances "
-                              "and, 3^L times, the Karatsuba leaves; n = 2^20 (profiles/qc_fft_sot_n20.md) "
-                              "2,757 per COT for smaller FFT sizes; 4,066 per COT for NTT sizes "
+                              "captures of single dual LPNs (cold cache per kernel): ternary sizes "
+                              "profiles/qc_ternary.md; FFT sizes 3,921 DRAM bytes per COT at n = 2^22 "
+                              "(profiles/qc_fft_sot_n22.md; 3^L times for the Karatsuba sizes), 2,757 below "
+                              "(profiles/qc_fft_sot_n20.md); 4,066 per COT for NTT sizes "
                               "(profiles/qc_ntt_sot_n20.md)"},
         "aes_roofline": aes,
         "qc_transform": qc_report([i.n for i in insts if i.kind != KIND_FERRET], stages["sot_encode"],
@@ -1393,7 +1399,10 @@ def run_ours(args):
     dom = max(stages, key=lambda s: stages[s][0])
     dms, dbytes = stages[dom]
     achieved = dbytes / (dms / 1e3) / 1e9
-    traffic = NCU_TRAFFIC_PER_STEP.get(f"{args.workload}:{dom}")
+    traffic = NCU_TRAFFIC_PER_STEP.get(f"{args.workload}{'' if args.qc_backend == 'auto' else '_' + args.qc_backend}:{dom}"
+                                       if dom == "dual_lpn" else f"{args.workload}:{dom}")
+    if dom == "dual_lpn" and not inst.r2 and qc_ternary(n.bit_length() - 1):
+        traffic = 2 * NCU_TERNARY_TRAFFIC.get(n.bit_length() - 1, 0) or None
     out = {
         "metric": metric_name(args.workload),
         "value": value, "unit": "COTs/s", "n_gpus": world, "steps": args.steps, "warmup": args.warmup,

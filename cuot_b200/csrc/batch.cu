@@ -21,11 +21,10 @@
 // stream of its own beside the SOT branch; CUOT_BATCH_FORK_SIZES also puts
 // each transform size on its own stream (sizes that share per-size FFT
 // state, qc_lane, on one).  Measured on B200 (the 64-instance mix of
-// log2 n in [16, 22], 10 graph replays each): one chain 86.1 ms, Ferret
-// beside SOT 88.7 ms, sizes side by side 97.3 ms.  Every part already fills
-// the GPU; run together, the persistent PPRF / LPN CTAs take SMs and
-// shared memory from the FFT passes, and the sizes' transform passes evict
-// each other's intermediate from L2.
+// log2 n in [16, 22], 10 graph replays each): one chain 48.5 ms, Ferret
+// beside SOT 48.3 ms, sizes side by side 48.9 ms (86.1, 88.7 and 97.3 ms when
+// the encodes were FFTs, whose intermediates evicted each other from L2).  Every
+// part already fills the GPU.
 // The whole program is captured into a CUDA graph on the first run.
 // Spin-free: work queues are atomic counters, reset by a memset node.
 #include <algorithm>
