@@ -80,8 +80,9 @@ def tune_batch(ctx, instances, table: TuningTable | None = None, reps: int = 2, 
     if hit:
         return hit["config"], hit.get("results", {})
     if candidates is None:
+        # rows 0: from the batch's rows (the default; a fixed count starves a small batch)
         candidates = [dict(pprf_threads=p, ctas_per_sm=c, lpn_rows_per_task=r)
-                      for p, c, r in itertools.product((128, 256), (2, 3), (16384, 65536))]
+                      for p, c, r in itertools.product((128, 256), (2, 3), (0, 16384, 65536))]
     stream = torch.cuda.Stream()
     results = {}
     best, best_ms = None, float("inf")
