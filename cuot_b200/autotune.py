@@ -3,7 +3,7 @@
 Measures candidate configurations on the caller's own shapes with CUDA
 events and keeps the fastest, persisted as a JSON table keyed by
 (kind, n, depth) for single instances and by the batch's shape signature for
-batches.  Knobs:
+batches, each with the version of the launch rules it was measured on.  Knobs:
   pprf_threads        threads per tree CTA (128 / 256)
   ctas_per_sm         persistent-grid CTAs per SM of the batched PPRF / LPN
   lpn_rows_per_task   LPN work-queue granularity (the LPN tile)
@@ -20,6 +20,11 @@ import os
 
 DEFAULT_TABLE = os.environ.get("CUOT_TUNING_TABLE",
                                os.path.join(os.path.expanduser("~"), ".cache", "cuot_b200", "tuning.json"))
+
+# Part of every key: raised whenever kernels or launch rules change what the
+# knobs cost, so that winners measured on earlier ones are measured again.
+# 2: grouped PPRF, LPN task size from the batch's rows, ternary dual LPN.
+RULES = 2
 
 
 class TuningTable:
@@ -48,12 +53,12 @@ class TuningTable:
 
 
 def shape_key(kind: int, n: int, h: int) -> str:
-    return f"{'sot' if kind == 1 else 'ferret'}:{n}:{h}"
+    return f"v{RULES}:{'sot' if kind == 1 else 'ferret'}:{n}:{h}"
 
 
 def batch_key(instances) -> str:
     sig = sorted((i.kind, i.n, i.h) for i in instances)
-    return "batch:" + hashlib.sha256(json.dumps(sig).encode()).hexdigest()[:16]
+    return f"v{RULES}:batch:" + hashlib.sha256(json.dumps(sig).encode()).hexdigest()[:16]
 
 
 def _time(fn, stream, reps: int) -> float:

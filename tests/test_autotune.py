@@ -41,3 +41,17 @@ def test_batch_may_keep_the_library_defaults(fakes, tmp_path):
     fakes(lambda cfg: 1.0 if cfg == default else 2.0)
     best, _ = autotune.tune_batch(None, [inst()], table=autotune.TuningTable(str(tmp_path / "t.json")))
     assert best == default
+
+
+def test_winners_of_earlier_launch_rules_are_measured_again(fakes, tmp_path):
+    import hashlib
+    import json
+    fakes(lambda cfg: 1.0 if cfg["pprf_threads"] == 256 else 2.0)
+    table, old = autotune.TuningTable(str(tmp_path / "t.json")), {"config": dict(pprf_threads=128), "ms": 3.0}
+    i = inst()
+    sig = json.dumps([[i.kind, i.n, i.h]])  # keys without a version
+    table.put("batch:" + hashlib.sha256(sig.encode()).hexdigest()[:16], old)
+    table.put(f"ferret:{i.n}:{i.h}", old)
+    best, _ = autotune.tune_batch(None, [i], table=table)
+    assert best["pprf_threads"] == 256 and table.get(autotune.batch_key([i]))["config"] == best
+    assert table.get(autotune.shape_key(i.kind, i.n, i.h)) is None
