@@ -630,7 +630,7 @@ int cuot_batch_create(cuot_ctx *ctx, const cuot_batch_item *items, int count,
     if ((st = qc_prepare(ctx, c.kind, c.e))) return cleanup(st);
     if ((st = balloc(b, &c.planes, qc_layout_bytes(c.kind, c.e, int(2 * c.items.size()))))) return cleanup(st);
     int pb = b->cfg.qc_planes_per_pass > 0 ? b->cfg.qc_planes_per_pass
-                                           : qc_default_batch(n, int(256 * c.items.size()));
+                                           : qc_default_batch(c.kind, n, int(256 * c.items.size()));
     pb = std::min(pb, int(256 * c.items.size()));
     c.batch = pb;
     if ((st = balloc(b, &c.Y, qc_y_bytes(ctx, c.kind, c.e, pb)))) return cleanup(st);

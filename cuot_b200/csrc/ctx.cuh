@@ -61,7 +61,8 @@ uint64_t qc_layout_bytes(int kind, int e, int njobs);
 // a_j (host arrays).  layout: qc_layout_bytes; Y: qc_y_bytes(batch).
 int qc_encode_jobs(cuot_ctx *ctx, int kind, int e, cuot_block *const *io, int njobs, const void *const *ahats,
                    void *layout, void *Y, int batch, cudaStream_t st);
-int qc_default_batch(uint64_t n, int nplanes);
+// Planes per pass when the caller leaves them to the library.
+int qc_default_batch(int kind, uint64_t n, int nplanes);
 // FP64 FFT backend of the QC encode (qc_fft.cu): n = 2^e, 10 <= e <= kQcfMaxE.
 constexpr int kQcfMaxE = 22;
 // n = 2^22 packs centred planes against `a` or its complement (whichever is
@@ -120,10 +121,11 @@ struct TernJob {
 bool tern_supported(int e);
 uint64_t tern_ahat_bytes(int e);   // leaf constants of `a`
 uint64_t tern_build_bytes(int e);  // scratch of tern_build_ahat
-uint64_t tern_job_bytes(int e);    // scratch per job of a launch
+// Scratch per job of a launch that takes `groups` groups of 32 planes at a time (1, 2 or 4).
+uint64_t tern_job_bytes(int e, int groups);
 int tern_build_ahat(int e, const uint64_t *a_d, void *scratch, void *ahat, cudaStream_t st);
 // Up to kTernMaxJobs dual LPNs of one size side by side; scratch holds
-// tern_job_bytes(e) for each.
+// tern_job_bytes(e, groups) for each.
 constexpr int kTernMaxJobs = 16;
 // aux: second stream to share the work with (joined again before the call
 // returns), or null.
@@ -131,7 +133,7 @@ struct TernAux {
   cudaStream_t stream;
   cudaEvent_t ev[2];  // fork, join
 };
-int tern_dual(int e, const TernJob *jobs, int njobs, void *scratch, TernAux *aux, cudaStream_t st);
+int tern_dual(int e, const TernJob *jobs, int njobs, int groups, void *scratch, TernAux *aux, cudaStream_t st);
 int transpose_launch(const void *in, uint64_t rows, uint64_t row_bytes, uint64_t col_lo,
                      uint64_t col_hi, void *out, cudaStream_t st);
 }  // namespace cuot

@@ -818,16 +818,20 @@ static int default_batch(uint64_t n, int nplanes) {
 // cuot_qc_plan_encode) take the FFT or the NTT.
 enum QcKind { kQcNtt = 0, kQcFft = 1, kQcKara = 2, kQcTern = 3 };
 
-static QcKind dual_kind(const cuot_ctx *ctx, int e) {
+// planes: planes per pass that the caller bounds its calls to (0: none).  The
+// ternary transform's 32 at a time need up to 68n bytes, an FFT pass 16n + 4n planes.
+constexpr int kTernMinPlanes = 16;
+static QcKind dual_kind(const cuot_ctx *ctx, int e, int planes) {
   if (ctx->qc_backend == 1) return kQcNtt;
-  if (ctx->qc_backend == 0 && !ctx->qcf_margin && tern_supported(e)) return kQcTern;
+  if (ctx->qc_backend == 0 && !ctx->qcf_margin && tern_supported(e) && (planes <= 0 || planes >= kTernMinPlanes))
+    return kQcTern;
   if (qcf_supported(e)) return kQcFft;
   if (qck_supported(e)) return kQcKara;
   return kQcNtt;
 }
 
 static bool planes_by_fft(QcKind k) { return k == kQcFft || k == kQcTern; }
-static QcKind plane_kind(const cuot_ctx *ctx, int e) { return planes_by_fft(dual_kind(ctx, e)) ? kQcFft : kQcNtt; }
+static QcKind plane_kind(const cuot_ctx *ctx, int e) { return planes_by_fft(dual_kind(ctx, e, 0)) ? kQcFft : kQcNtt; }
 
 // Intermediate bytes of a pass over `batch` planes: 4 bytes per plane and
 // coefficient for both transforms (the FFT packs 4 planes in 16 bytes, in
@@ -867,11 +871,14 @@ static uint64_t ahat_scratch_bytes(QcKind k, int e) {
   return 4ull << e;
 }
 
+// Groups of 32 planes that a ternary dual LPN takes at a time for a pass of `batch` planes.
+static int tern_groups_at_once(int batch) { return batch >= 128 ? 4 : batch >= 64 ? 2 : 1; }
+
 // Scratch of a dual LPN (rate 1, or rate 1/2 with r2): the planes / tile
 // words (and the 2n-bit planes of the rate-1/2 form) or the Karatsuba
 // split blocks, then the pass intermediate; the ternary transform's values.
 static uint64_t dual_scratch_bytes(const cuot_ctx *ctx, QcKind k, int e, int batch, bool r2) {
-  if (k == kQcTern) return tern_job_bytes(e);
+  if (k == kQcTern) return tern_job_bytes(e, tern_groups_at_once(batch));
   if (k == kQcKara) return qck_scratch_bytes(e) + y_bytes(true, kQcfMaxE, leaf_batch(ctx));
   return ((r2 ? 32ull : 16ull) << e) + y_bytes(k == kQcFft, e, batch);
 }
@@ -976,7 +983,7 @@ static int eng_dual(cuot_ctx *ctx, const QcEngine &g, int e, const void *ahat, c
     const TernJob job{src, xor_in, out, ahat};
     TernAux *aux;
     CUOT_TRY(tern_aux(ctx, e, 1, st, &aux));
-    return tern_dual(e, &job, 1, scr, aux, st);
+    return tern_dual(e, &job, 1, tern_groups_at_once(batch), scr, aux, st);
   }
   void *Y = scr + dual_y_offset(g.kind, e, r2);
   if (g.kind == kQcKara) return qck_dual_lpn(g.f, e, ahat, src, xor_in, out, scr, Y, leaf_batch(ctx), st);
@@ -999,7 +1006,7 @@ static int eng_dual(cuot_ctx *ctx, const QcEngine &g, int e, const void *ahat, c
 }
 
 // ---- helpers for the batched engine (batch.cu) ----------------------------
-int qc_kind(const cuot_ctx *ctx, int e) { return dual_kind(ctx, e); }
+int qc_kind(const cuot_ctx *ctx, int e) { return dual_kind(ctx, e, 0); }
 
 int qc_prepare(cuot_ctx *ctx, int kind, int e) {
   QcEngine g;
@@ -1021,9 +1028,10 @@ uint64_t qc_layout_bytes(int kind, int e, int njobs) {
 }
 
 // Dual LPNs per launch of the ternary transform for a batch of `batch`
-// planes: as many as leave its values (tern_job_bytes each) in L2.
+// planes: as many as leave its values (tern_job_bytes each) in L2; one for a
+// batch below 128 planes, which takes fewer word groups at a time instead.
 static int tern_jobs_per_launch(int e, int batch) {
-  const uint64_t fit = (80ull << 20) / tern_job_bytes(e);
+  const uint64_t fit = (80ull << 20) / tern_job_bytes(e, 4);
   uint64_t jobs = uint64_t(batch > 128 ? batch / 128 : 1);
   if (jobs > kTernMaxJobs) jobs = kTernMaxJobs;
   return int(jobs < fit ? jobs : fit < 1 ? 1 : fit);
@@ -1032,7 +1040,7 @@ static int tern_jobs_per_launch(int e, int batch) {
 uint64_t qc_y_bytes(const cuot_ctx *ctx, int kind, int e, int batch) {
   const QcKind k = QcKind(kind);
   const uint64_t y = k == kQcKara   ? dual_scratch_bytes(ctx, k, e, batch, false)
-                     : k == kQcTern ? tern_jobs_per_launch(e, batch) * tern_job_bytes(e)
+                     : k == kQcTern ? tern_jobs_per_launch(e, batch) * tern_job_bytes(e, tern_groups_at_once(batch))
                                     : y_bytes(k == kQcFft, e, batch);
   const uint64_t a = ahat_scratch_bytes(k, e);
   return y > a ? y : a;
@@ -1104,7 +1112,7 @@ int qc_encode_jobs(cuot_ctx *ctx, int kind, int e, cuot_block *const *io, int nj
       for (int j = 0; j < nj; j++) jobs[j] = TernJob{io[j0 + j], nullptr, io[j0 + j], ahats[j0 + j]};
       TernAux *aux;
       CUOT_TRY(tern_aux(ctx, e, nj, st, &aux));
-      CUOT_TRY(tern_dual(e, jobs, nj, Y, aux, st));
+      CUOT_TRY(tern_dual(e, jobs, nj, tern_groups_at_once(batch), Y, aux, st));
     }
     return CUOT_OK;
   }
@@ -1118,17 +1126,20 @@ int qc_encode_jobs(cuot_ctx *ctx, int kind, int e, cuot_block *const *io, int nj
   return encode_jobs_ntt(g, e, io, njobs, ahats, static_cast<uint64_t *>(layout), Y, batch, st);
 }
 
-int qc_default_batch(uint64_t n, int nplanes) { return default_batch(n, nplanes); }
+int qc_default_batch(int kind, uint64_t n, int nplanes) {
+  const int b = default_batch(n, nplanes);
+  return kind == kQcTern && b < 128 ? 128 : b;  // a ternary dual LPN takes all its planes at once
+}
 
-static int one_shot_batch(const cuot_ctx *ctx, uint64_t n) {
-  const int batch = ctx->qc_planes_per_pass > 0 ? ctx->qc_planes_per_pass : default_batch(n, 128);
+static int one_shot_batch(const cuot_ctx *ctx, QcKind kind, uint64_t n) {
+  const int batch = ctx->qc_planes_per_pass > 0 ? ctx->qc_planes_per_pass : qc_default_batch(kind, n, 128);
   return batch > 128 ? 128 : batch;
 }
 
 // Scratch of cuot_sot_dual_lpn (r2: cuot_sot_dual_lpn_r2) at n = 2^e on ctx.
 uint64_t qc_one_shot_dual_bytes(const cuot_ctx *ctx, int e, bool r2) {
-  const QcKind kind = dual_kind(ctx, e);
-  const uint64_t ds = dual_scratch_bytes(ctx, kind, e, one_shot_batch(ctx, 1ull << e), r2);
+  const QcKind kind = dual_kind(ctx, e, ctx->qc_planes_per_pass);
+  const uint64_t ds = dual_scratch_bytes(ctx, kind, e, one_shot_batch(ctx, kind, 1ull << e), r2);
   const uint64_t as = ahat_scratch_bytes(kind, e);
   return ahat_bytes(kind, e, false) + (ds > as ? ds : as);
 }
@@ -1143,7 +1154,11 @@ struct cuot_qc_plan {
   uint64_t n;
   QcKind kind;
   void *ahat;
-  int batch;
+  int batch;  // planes per pass, 0: automatic
+  int planes_per_pass(int kind_, int nplanes) const {
+    const int b = batch > 0 ? batch : cuot::qc_default_batch(kind_, n, 128);
+    return b < nplanes ? b : nplanes;
+  }
 };
 
 extern "C" {
@@ -1176,7 +1191,7 @@ int cuot_qc_plan_create(cuot_ctx *ctx, const uint64_t *a_d, uint64_t n, void *st
   int e;
   CUOT_TRY(check_n(n, &e));
   DeviceGuard dg(ctx);
-  cuot_qc_plan *pl = new cuot_qc_plan{ctx, e, n, dual_kind(ctx, e), nullptr, 0};
+  cuot_qc_plan *pl = new cuot_qc_plan{ctx, e, n, dual_kind(ctx, e, ctx->qc_planes_per_pass), nullptr, 0};
   QcEngine g;
   int st = engine(ctx, e, pl->kind, true, &g);
   TernAux *aux;
@@ -1190,7 +1205,7 @@ int cuot_qc_plan_create(cuot_ctx *ctx, const uint64_t *a_d, uint64_t n, void *st
     delete pl;
     return st;
   }
-  pl->batch = ctx->qc_planes_per_pass > 0 ? ctx->qc_planes_per_pass : default_batch(n, 128);
+  pl->batch = ctx->qc_planes_per_pass;
   *out = pl;
   return CUOT_OK;
 }
@@ -1215,7 +1230,7 @@ int cuot_qc_plan_encode(cuot_qc_plan *pl, uint64_t *planes_io_d, int nplanes, vo
   DeviceGuard dg(ctx);
   QcEngine g;
   CUOT_TRY(engine(ctx, pl->e, pl->kind, true, &g));
-  const int batch = pl->batch < nplanes ? pl->batch : nplanes;
+  const int batch = pl->planes_per_pass(kQcFft, nplanes);
   void *scr;
   CUOT_TRY(scratch(ctx, y_bytes(planes_by_fft(pl->kind), pl->e, batch), &scr));
   return eng_encode(g, pl->e, pl->ahat, planes_io_d, planes_io_d, pl->n / 64, 0, nplanes, scr, batch,
@@ -1228,7 +1243,7 @@ int cuot_qc_plan_dual_lpn(cuot_qc_plan *pl, cuot_block *io_d, void *stream) {
   DeviceGuard dg(ctx);
   QcEngine g;
   CUOT_TRY(engine(ctx, pl->e, pl->kind, false, &g));
-  const int batch = pl->batch < 128 ? pl->batch : 128;
+  const int batch = pl->planes_per_pass(pl->kind, 128);
   void *scr;
   CUOT_TRY(scratch(ctx, dual_scratch_bytes(ctx, pl->kind, pl->e, batch, false), &scr));
   return eng_dual(ctx, g, pl->e, pl->ahat, io_d, io_d, false, static_cast<uint8_t *>(scr), batch,
@@ -1241,7 +1256,7 @@ int cuot_qc_plan_dual_lpn_r2(cuot_qc_plan *pl, const cuot_block *in_d, cuot_bloc
   DeviceGuard dg(ctx);
   QcEngine g;
   CUOT_TRY(engine(ctx, pl->e, pl->kind, false, &g));
-  const int batch = pl->batch < 128 ? pl->batch : 128;
+  const int batch = pl->planes_per_pass(pl->kind, 128);
   void *scr;
   CUOT_TRY(scratch(ctx, dual_scratch_bytes(ctx, pl->kind, pl->e, batch, true), &scr));
   return eng_dual(ctx, g, pl->e, pl->ahat, in_d, out_d, true, static_cast<uint8_t *>(scr), batch,
@@ -1276,9 +1291,9 @@ static int one_shot_dual(cuot_ctx *ctx, const uint64_t *a_d, const cuot_block *i
   CUOT_TRY(check_n(n, &e));
   DeviceGuard dg(ctx);
   QcEngine g;
-  const QcKind kind = dual_kind(ctx, e);
+  const QcKind kind = dual_kind(ctx, e, ctx->qc_planes_per_pass);
   CUOT_TRY(engine(ctx, e, kind, false, &g));
-  const int batch = one_shot_batch(ctx, n);
+  const int batch = one_shot_batch(ctx, kind, n);
   const uint64_t ab = ahat_bytes(kind, e, false);
   void *scr;
   CUOT_TRY(scratch(ctx, qc_one_shot_dual_bytes(ctx, e, r2), &scr));

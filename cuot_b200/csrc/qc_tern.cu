@@ -34,14 +34,14 @@ __constant__ TernSigmas c_sigmas = tern_sigmas();
 // What a pass reads and writes: src != dst, or the pieces of jobs.in first.
 struct PassArgs {
   int e, pass;
-  int W;  // word groups: 4, or 1 for the bits of `a`
+  int W;  // word groups: 4 or a caller's 2 or 1 (kFirstSome: jobs.in from the first of them), 1 for the bits of `a`
   const uint32_t *src;
   uint32_t *dst;
   uint64_t job_words;
   TernJobs jobs;
 };
-enum PassKind { kFirst, kFirstBits, kForward, kInverse, kLastInverse };
-constexpr bool pass_first(PassKind k) { return k == kFirst || k == kFirstBits; }
+enum PassKind { kFirst, kFirstSome, kFirstBits, kForward, kInverse, kLastInverse };
+constexpr bool pass_first(PassKind k) { return k == kFirst || k == kFirstSome || k == kFirstBits; }
 constexpr bool pass_inverse(PassKind k) { return k == kInverse || k == kLastInverse; }
 
 // Rotation table of a pass in shared memory, and the one of its rotated stores.
@@ -372,6 +372,20 @@ __global__ void __launch_bounds__(256) tern_final(const uint32_t *buf, uint64_t 
   reinterpret_cast<uint4 *>(jobs.out[blockIdx.z])[j] = v;
 }
 
+// The same for word groups w0 .. w0 + W - 1 (W = 1 or 2) of a dual LPN that takes them
+// in turn: a thread per coefficient and group.
+template <int E>
+__global__ void __launch_bounds__(256) tern_final_some(const uint32_t *buf, uint64_t job_words, TernJobs jobs, int W,
+                                                       int w0) {
+  constexpr TernShape s = tern_shape(E);
+  constexpr uint64_t group = uint64_t(tern_points(s)) * tern_element(s.L);
+  const uint32_t id = blockIdx.x * 256 + threadIdx.x, j = id / W, w = id % W;
+  uint32_t v = tern_coefficient<E>(buf + uint64_t(blockIdx.z) * job_words + w * group, j);
+  const uint64_t at = uint64_t(j) * 4 + w0 + w;
+  if (jobs.xor_in[blockIdx.z]) v ^= jobs.xor_in[blockIdx.z][at];
+  jobs.out[blockIdx.z][at] = v;
+}
+
 uint64_t group_words(int e) {
   const TernShape s = tern_shape(e);
   return uint64_t(tern_points(s)) * tern_element(s.L);
@@ -410,6 +424,7 @@ int pass_of(const Run &r, const PassArgs &a, PassKind kind) {
   const int rad = tern_radix(tern_shape(a.e).m, a.pass);
   switch (kind) {
     case kFirst: return pass27<L, kFirst, C>(r, a);
+    case kFirstSome: return pass27<L, kFirstSome, C>(r, a);
     case kFirstBits: return pass27<L, kFirstBits, C>(r, a);
     case kLastInverse: return pass27<L, kLastInverse, C>(r, a);
     case kForward:
@@ -464,8 +479,14 @@ int consts(const Run &r, int e, const uint32_t *buf, uint32_t *out) {
 #undef TERN_consts_of
 #undef TERN_DISPATCH
 
+// Word groups w0 .. w0 + W - 1.
 template <int E>
-void final_of(const Run &r, const uint32_t *buf, uint64_t job_words, const TernJobs &jobs) {
+void final_of(const Run &r, const uint32_t *buf, uint64_t job_words, const TernJobs &jobs, int W, int w0) {
+  if (W < 4) {
+    launch_as(false, tern_final_some<E>, dim3((1u << E) / 256 * W, 1, r.njobs), dim3(256), 0, r.st, buf, job_words,
+              jobs, W, w0);
+    return;
+  }
   constexpr bool kMayChain = (1ull << E) <= kChainBlocks;
   launch_as(kMayChain && r.chained, kMayChain && r.chained ? tern_final<E, kMayChain> : tern_final<E, false>,
             dim3((1u << E) / 256, 1, r.njobs), dim3(256), 0, r.st, buf, job_words, jobs);
@@ -504,7 +525,7 @@ uint64_t tern_ahat_bytes(int e) {
 }
 
 uint64_t tern_build_bytes(int e) { return 2 * group_words(e) * 4; }
-uint64_t tern_job_bytes(int e) { return 2 * group_words(e) * 16; }
+uint64_t tern_job_bytes(int e, int groups) { return 2 * group_words(e) * 4 * groups; }
 
 int tern_build_ahat(int e, const uint64_t *a_d, void *scratch, void *ahat, cudaStream_t st) {
   uint32_t *half[2] = {static_cast<uint32_t *>(scratch), static_cast<uint32_t *>(scratch) + group_words(e)};
@@ -518,33 +539,30 @@ int tern_build_ahat(int e, const uint64_t *a_d, void *scratch, void *ahat, cudaS
   return launch_status(1 + tern_passes(tern_shape(e).m));
 }
 
-int tern_dual(int e, const TernJob *job, int njobs, void *scratch, TernAux *aux, cudaStream_t st) {
+// Word groups w0 .. w0 + W - 1 of the dual LPNs `jobs`, in scratch.
+static int tern_groups(int e, const TernJobs &jobs, int njobs, int W, int w0, void *scratch, TernAux *aux,
+                       cudaStream_t st) {
   const TernShape s = tern_shape(e);
-  if (njobs > kTernMaxJobs) return fail(CUOT_EINVAL, "%d dual LPNs in one launch (at most %d)", njobs, kTernMaxJobs);
-  const uint64_t group = group_words(e), job_words = group * 4;
+  const uint64_t group = group_words(e), job_words = group * W;
   uint32_t *half[2] = {static_cast<uint32_t *>(scratch), static_cast<uint32_t *>(scratch) + njobs * job_words};
   const int passes = tern_passes(s.m);
-  Run r{njobs, 4, chain_launches(uint64_t(njobs) << e, st), st};
-  TernJobs jobs{};
-  for (int j = 0; j < njobs; j++) {
-    jobs.in[j] = reinterpret_cast<const uint32_t *>(job[j].in);
-    jobs.xor_in[j] = reinterpret_cast<const uint32_t *>(job[j].xor_in);
-    jobs.out[j] = reinterpret_cast<uint32_t *>(job[j].out);
-    jobs.consts[j] = static_cast<const uint32_t *>(job[j].ahat);
-  }
-  CUOT_TRY(pass(r, PassArgs{e, 0, 4, nullptr, half[0], job_words, jobs}, kFirst));
+  Run r{njobs, W, chain_launches(uint64_t(njobs) << e, st), st};
+  PassArgs first{e, 0, W, nullptr, half[0], job_words, jobs};
+  for (int j = 0; j < njobs; j++) first.jobs.in[j] += w0;
+  CUOT_TRY(pass(r, first, W == 4 ? kFirst : kFirstSome));
   int at = 0, launches = 2 * passes + 2;
-  if (aux) {
+  const int turn = e > 20 ? 1 : 2;
+  if (aux && turn < W) {
     // The word groups are independent from here to the end: they alternate
     // between two streams, so that one's kernels fill the other's wave tails
     // and its passes (memory) run beside inner products (integer pipe).  Two
     // groups at a time while a group's kernels are small (2^19: 187 us on one
     // stream, 169 with pairs, 189 one by one; 2^20 386, 375, 377), one by one
     // above (2^21 976, 940, 928; 2^22 2006, 1973, 1946).
-    r.W = e > 20 ? 1 : 2;
+    r.W = turn;
     if (cudaEventRecord(aux->ev[0], st) != cudaSuccess || cudaStreamWaitEvent(aux->stream, aux->ev[0], 0) != cudaSuccess)
       return launch_status(1);
-    for (int w = 0; w < 4; w += r.W) {
+    for (int w = 0; w < W; w += r.W) {
       r.st = (w / r.W) & 1 ? aux->stream : st;
       uint32_t *part[2] = {half[0] + w * group, half[1] + w * group};
       at = 0;
@@ -555,7 +573,7 @@ int tern_dual(int e, const TernJob *job, int njobs, void *scratch, TernAux *aux,
     r.st = st;
     if (cudaEventRecord(aux->ev[1], aux->stream) != cudaSuccess || cudaStreamWaitEvent(st, aux->ev[1], 0) != cudaSuccess)
       return launch_status(1);
-    launches += (4 / r.W - 1) * 2 * passes;
+    launches += (W / r.W - 1) * 2 * passes;
   } else {
     CUOT_TRY(passes_on(r, e, 1, half, job_words, &at));
     CUOT_TRY(inner(r, e, half[at], job_words, jobs));
@@ -563,12 +581,25 @@ int tern_dual(int e, const TernJob *job, int njobs, void *scratch, TernAux *aux,
   }
   switch (e) {
 #define TERN_FINAL(E) \
-  case E: final_of<E>(r, half[at], job_words, jobs); break;
+  case E: final_of<E>(r, half[at], job_words, jobs, W, w0); break;
     TERN_FINAL(14) TERN_FINAL(15) TERN_FINAL(16) TERN_FINAL(17) TERN_FINAL(18)
     TERN_FINAL(19) TERN_FINAL(20) TERN_FINAL(21) TERN_FINAL(22)
 #undef TERN_FINAL
   }
   return launch_status(launches);
+}
+
+int tern_dual(int e, const TernJob *job, int njobs, int groups, void *scratch, TernAux *aux, cudaStream_t st) {
+  if (njobs > kTernMaxJobs) return fail(CUOT_EINVAL, "%d dual LPNs in one launch (at most %d)", njobs, kTernMaxJobs);
+  TernJobs jobs{};
+  for (int j = 0; j < njobs; j++) {
+    jobs.in[j] = reinterpret_cast<const uint32_t *>(job[j].in);
+    jobs.xor_in[j] = reinterpret_cast<const uint32_t *>(job[j].xor_in);
+    jobs.out[j] = reinterpret_cast<uint32_t *>(job[j].out);
+    jobs.consts[j] = static_cast<const uint32_t *>(job[j].ahat);
+  }
+  for (int w0 = 0; w0 < 4; w0 += groups) CUOT_TRY(tern_groups(e, jobs, njobs, groups, w0, scratch, aux, st));
+  return CUOT_OK;
 }
 
 }  // namespace cuot

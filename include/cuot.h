@@ -65,7 +65,11 @@ uint64_t cuot_ctx_scratch_bytes(const cuot_ctx *ctx);
  *                           256-thread CTA expands one, two or four trees
  *                           at a time, by their number and depth)
  *   CUOT_TUNE_QC_PLANES     planes per QC pass, 0 = automatic (512 MiB of
- *                           intermediate)
+ *                           intermediate; a ternary dual LPN takes all 128).
+ *                           A ternary dual LPN takes whole groups of 32
+ *                           planes: one at a time below 64, two below 128
+ *                           (34n to 68n bytes of scratch per group); below 16
+ *                           single dual LPNs take the FFT
  *   CUOT_TUNE_QC_BACKEND    transform of the exact QC encode: 0 automatic
  *                           (dual LPNs of 2^14 <= n <= 2^22 by the ternary
  *                           GF(2) transform; otherwise as 2), 1 the NTT
@@ -346,7 +350,8 @@ int cuot_qc_encode_sparse_r2(cuot_ctx *ctx, const uint64_t *a_d,
  * the context (the first use of a size synchronises the device).
  * plan_encode / plan_dual_lpn do what cuot_qc_encode / cuot_sot_dual_lpn do
  * without re-transforming `a`.  set_batch bounds how many planes share one
- * intermediate pass (4 bytes per coefficient per plane of scratch). */
+ * intermediate pass (4 bytes per coefficient per plane of scratch; ternary
+ * dual LPNs as CUOT_TUNE_QC_PLANES says). */
 typedef struct cuot_qc_plan cuot_qc_plan;
 int cuot_qc_plan_create(cuot_ctx *ctx, const uint64_t *a_d, uint64_t n,
                         void *stream, cuot_qc_plan **out);
