@@ -847,15 +847,16 @@ static int leaf_batch(const cuot_ctx *ctx) {
   return ctx->qc_planes_per_pass > 0 ? ctx->qc_planes_per_pass : default_batch(1ull << kQcfMaxE, 128);
 }
 
-// The ternary transform's constants, padded so that an FFT A_hat can follow.
+// The ternary transform's constants, padded so that a plan's copy of `a` can follow.
 static uint64_t tern_ahat_span(int e) { return (tern_ahat_bytes(e) + 255) & ~255ull; }
 
 // Bytes of A_hat: NTT n Shoup pairs; FFT n complex doubles; ternary its leaf
-// constants; Karatsuba the 3^L leaf transforms.  With planes the last two are
-// followed by the FFT's / the NTT's A_hat for plane encodes.
+// constants; Karatsuba the 3^L leaf transforms.  With planes the last is
+// followed by the NTT's A_hat for plane encodes, and the ternary constants by `a`
+// itself (a plan makes the FFT's A_hat of it for its first plane encode).
 static uint64_t ahat_bytes(QcKind k, int e, bool with_planes) {
   if (k == kQcFft) return qcf_ahat_bytes(e);
-  if (k == kQcTern) return tern_ahat_span(e) + (with_planes ? qcf_ahat_bytes(e) : 0);
+  if (k == kQcTern) return tern_ahat_span(e) + (with_planes ? 1ull << e >> 3 : 0);
   if (k == kQcKara) return qck_ahat_bytes(e) + (with_planes ? 8ull << e : 0);
   return 8ull << e;
 }
@@ -863,7 +864,7 @@ static uint64_t ahat_bytes(QcKind k, int e, bool with_planes) {
 // Scratch of the A_hat build.
 static uint64_t ahat_scratch_bytes(QcKind k, int e) {
   if (k == kQcFft) return 16ull << e;
-  if (k == kQcTern) return tern_build_bytes(e) > (16ull << e) ? tern_build_bytes(e) : 16ull << e;
+  if (k == kQcTern) return tern_build_bytes(e);
   if (k == kQcKara) {
     const uint64_t kb = qck_bits_scratch_bytes(e) + (16ull << kQcfMaxE);
     return kb > (4ull << e) ? kb : (4ull << e);
@@ -946,8 +947,10 @@ static int eng_ahat(const QcEngine &g, int e, const uint64_t *a_d, void *scr, vo
   if (g.kind == kQcFft) return qcf_build_ahat(g.f, a_d, scr, ahat, st);
   if (g.kind == kQcTern) {
     CUOT_TRY(tern_build_ahat(e, a_d, scr, ahat, st));
-    if (!with_planes) return CUOT_OK;
-    return qcf_build_ahat(g.f, a_d, scr, static_cast<uint8_t *>(ahat) + tern_ahat_span(e), st);
+    if (with_planes && cudaMemcpyAsync(static_cast<uint8_t *>(ahat) + tern_ahat_span(e), a_d, 1ull << e >> 3,
+                                       cudaMemcpyDeviceToDevice, st) != cudaSuccess)
+      return launch_status(0);
+    return CUOT_OK;
   }
   if (g.kind == kQcKara) {
     const uint64_t bb = qck_bits_scratch_bytes(e);
@@ -959,11 +962,10 @@ static int eng_ahat(const QcEngine &g, int e, const uint64_t *a_d, void *scr, vo
 }
 
 // Planes p < nplanes: in + p * stride -> out + p * stride (64-bit words),
-// written or XORed into (accumulate).  A ternary (Karatsuba) plan encodes
-// planes with the FFT (NTT) A_hat stored after its constants (leaves).
+// written or XORed into (accumulate).  ahat: the FFT's for a ternary plan; a
+// Karatsuba plan encodes planes with the NTT A_hat stored after its leaves.
 static int eng_encode(const QcEngine &g, int e, const void *ahat, const uint64_t *in, uint64_t *out, uint64_t stride,
                       int accumulate, int nplanes, void *Y, int batch, cudaStream_t st) {
-  if (g.kind == kQcTern) ahat = static_cast<const uint8_t *>(ahat) + tern_ahat_span(e);
   if (planes_by_fft(g.kind))
     return qcf_encode(g.f, single_tab(ahat), in, out, stride, accumulate, nplanes, Y, batch, st);
   if (g.kind == kQcKara) ahat = static_cast<const uint8_t *>(ahat) + qck_ahat_bytes(e);
@@ -1155,11 +1157,38 @@ struct cuot_qc_plan {
   QcKind kind;
   void *ahat;
   int batch;  // planes per pass, 0: automatic
+  void *plane_ahat;  // ternary: the FFT's A_hat, once planes have been encoded
+  bool planes_ready;
   int planes_per_pass(int kind_, int nplanes) const {
     const int b = batch > 0 ? batch : cuot::qc_default_batch(kind_, n, 128);
     return b < nplanes ? b : nplanes;
   }
 };
+
+// A_hat of plane encodes.  A ternary plan makes the FFT's when the first planes
+// come (made with every plan, it was half of the plan's memory and of the time to
+// create one at 2^22, and the dual LPN never reads it).  Captured first calls
+// are legal: the allocation is no part of the graph, the transform is, and the next
+// call that is not captured makes it again for those after.
+static int plane_ahat(cuot_qc_plan *pl, const QcEngine &g, void *scr, cudaStream_t st, const void **out) {
+  *out = pl->ahat;
+  if (pl->kind != kQcTern) return CUOT_OK;
+  if (!pl->plane_ahat) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const int rc = dev_alloc(&pl->plane_ahat, qcf_ahat_bytes(pl->e));
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    CUOT_TRY(rc);
+  }
+  *out = pl->plane_ahat;
+  if (pl->planes_ready) return CUOT_OK;
+  const uint8_t *bits = static_cast<const uint8_t *>(pl->ahat) + tern_ahat_span(pl->e);
+  CUOT_TRY(qcf_build_ahat(g.f, reinterpret_cast<const uint64_t *>(bits), scr, pl->plane_ahat, st));
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) return launch_status(0);
+  pl->planes_ready = cap == cudaStreamCaptureStatusNone;
+  return CUOT_OK;
+}
 
 extern "C" {
 
@@ -1191,7 +1220,7 @@ int cuot_qc_plan_create(cuot_ctx *ctx, const uint64_t *a_d, uint64_t n, void *st
   int e;
   CUOT_TRY(check_n(n, &e));
   DeviceGuard dg(ctx);
-  cuot_qc_plan *pl = new cuot_qc_plan{ctx, e, n, dual_kind(ctx, e, ctx->qc_planes_per_pass), nullptr, 0};
+  cuot_qc_plan *pl = new cuot_qc_plan{ctx, e, n, dual_kind(ctx, e, ctx->qc_planes_per_pass), nullptr, 0, nullptr, false};
   QcEngine g;
   int st = engine(ctx, e, pl->kind, true, &g);
   TernAux *aux;
@@ -1214,6 +1243,7 @@ int cuot_qc_plan_destroy(cuot_qc_plan *pl) {
   if (!pl) return CUOT_OK;
   DeviceGuard g(pl->ctx);
   cudaFree(pl->ahat);
+  cudaFree(pl->plane_ahat);
   delete pl;
   return CUOT_OK;
 }
@@ -1231,9 +1261,14 @@ int cuot_qc_plan_encode(cuot_qc_plan *pl, uint64_t *planes_io_d, int nplanes, vo
   QcEngine g;
   CUOT_TRY(engine(ctx, pl->e, pl->kind, true, &g));
   const int batch = pl->planes_per_pass(kQcFft, nplanes);
+  uint64_t bytes = y_bytes(planes_by_fft(pl->kind), pl->e, batch);
+  const uint64_t build = ahat_scratch_bytes(kQcFft, pl->e);
+  if (pl->kind == kQcTern && !pl->planes_ready && bytes < build) bytes = build;  // (the arena has it since plan_create)
   void *scr;
-  CUOT_TRY(scratch(ctx, y_bytes(planes_by_fft(pl->kind), pl->e, batch), &scr));
-  return eng_encode(g, pl->e, pl->ahat, planes_io_d, planes_io_d, pl->n / 64, 0, nplanes, scr, batch,
+  CUOT_TRY(scratch(ctx, bytes, &scr));
+  const void *ahat;
+  CUOT_TRY(plane_ahat(pl, g, scr, static_cast<cudaStream_t>(stream), &ahat));
+  return eng_encode(g, pl->e, ahat, planes_io_d, planes_io_d, pl->n / 64, 0, nplanes, scr, batch,
                     static_cast<cudaStream_t>(stream));
 }
 

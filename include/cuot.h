@@ -349,7 +349,9 @@ int cuot_qc_encode_sparse_r2(cuot_ctx *ctx, const uint64_t *a_d,
  * the transform in its own device buffer; the twiddle tables are cached in
  * the context (the first use of a size synchronises the device).
  * plan_encode / plan_dual_lpn do what cuot_qc_encode / cuot_sot_dual_lpn do
- * without re-transforming `a`.  set_batch bounds how many planes share one
+ * without re-transforming `a` (a plan of 2^14 to 2^22 keeps `a` itself too and
+ * makes the FFT's transform of it on the first plan_encode: 16n bytes, one
+ * cudaMalloc).  set_batch bounds how many planes share one
  * intermediate pass (4 bytes per coefficient per plane of scratch; ternary
  * dual LPNs as CUOT_TUNE_QC_PLANES says). */
 typedef struct cuot_qc_plan cuot_qc_plan;
