@@ -119,6 +119,7 @@ int cuot_ctx_destroy(cuot_ctx *c) {
     qc_free_ctx_tables(c);
     if (c->qcf_margin) cudaFree(c->qcf_margin);
     if (c->scratch) cudaFree(c->scratch);
+    if (c->pool) cudaMemPoolDestroy(c->pool);
     if (c->t0_d) cudaFree(c->t0_d);
   }
   delete c;

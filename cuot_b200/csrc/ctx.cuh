@@ -7,6 +7,7 @@ struct cuot_ctx {
   uint32_t *t0_d;          // T0 table (256 words) for staging into shared memory
   void *scratch;           // grow-only scratch arena
   uint64_t scratch_bytes;
+  cudaMemPool_t pool;      // stream-ordered memory of single calls (lpn.cu), or null
   void *qc_tables[32];     // NTT twiddle tables per log2(n) (qc.cu)
   void *qcf_tables[32];    // FFT twiddle tables per log2(n) (qc_fft.cu)
   void *tern_aux[32];      // second stream of the ternary transform per log2(n) (qc.cu)

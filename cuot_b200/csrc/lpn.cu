@@ -10,6 +10,8 @@
 // The index AES runs in the same kernel as the gather, so the n*d index
 // matrix never touches HBM (cuOT materialises it, dev_layer.cu:171-173).
 // kk (k blocks) is read through the read-only path and stays L2-resident.
+#include <mutex>
+
 #include "lpn_kernel.cuh"
 
 namespace cuot {
@@ -118,29 +120,70 @@ int launch_split(cuot_ctx *ctx, const LpnArgs &a, cudaStream_t st) {
                                                      : launch_split_as<ROLES, false>(ctx, a, st);
 }
 
+// Memory of its own for one call on `st`, given back to the context's pool in stream
+// order: no other call's arena, captured graph or stream holds it.  Null if there is
+// none to be had.
+constexpr uint64_t kPoolKeeps = 64ull << 20;  // bytes that the pool keeps between calls
+static void *pool_alloc(cuot_ctx *ctx, uint64_t bytes, cudaStream_t st) {
+  static std::mutex mu;
+  // other streams of the program may be under capture, which forbids a plain cudaMalloc
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  void *p = nullptr;
+  {
+    std::lock_guard<std::mutex> lk(mu);
+    if (!ctx->pool) {
+      cudaMemPoolProps props{};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location = {cudaMemLocationTypeDevice, ctx->device};
+      uint64_t keep = kPoolKeeps;
+      if (cudaMemPoolCreate(&ctx->pool, &props) != cudaSuccess) {
+        ctx->pool = nullptr;
+        cudaGetLastError();
+      } else {
+        cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+      }
+    }
+  }
+  if (ctx->pool && cudaMallocFromPoolAsync(&p, bytes, ctx->pool, st) != cudaSuccess) {
+    p = nullptr;
+    cudaGetLastError();
+  }
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  return p;
+}
+
 // Both roles, d = 10.  From kInterleaveRows rows on, kk and kk2 are first copied
-// side by side into the context's scratch (470,016 rows 66.8 -> 58.6 us with the
-// copy, 10,485,760 rows 1197 -> 927; at 131,072 rows the 3 us that the gathers
-// would save are the copy's launch).  Not while `st` is captured: the arena may
-// neither grow then nor, as far as this call goes, stay where it is until the
-// graph runs.  Nor if an arena is there and would have to grow for it (a caller's
-// graph may hold the old one), or none can be had: the plain form needs no scratch.
-constexpr int64_t kInterleaveRows = 1 << 18;
+// side by side (470,016 rows 66.8 -> 58.6 us with the copy, 10,485,760 rows 1197 ->
+// 927; at 131,072 rows the 3 us that the gathers would save are the copy's launch),
+// unless `st` is captured or there is no memory.  Without the copy two arrays of
+// more than about 32 MB each fall out of L2 together: one role after the other
+// is then faster (10,485,760 rows, k = 1.6 / 2 / 2.6 / 4 million: 1,227 / 1,623 / 2,128 /
+// 2,762 us together, 1,602 / 1,602 / 1,603 / 1,758 in turn; copied 950 / 1,058 / 1,224).
+constexpr int64_t kInterleaveRows = 1 << 18, kTogether = 2000000;
 int launch_dual(cuot_ctx *ctx, LpnArgs a, cudaStream_t st) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  const uint64_t bytes = uint64_t(a.k) * 32;
-  void *scr = nullptr;
-  if (a.ngroups * 4 < kInterleaveRows || a.k > a.ngroups || cudaStreamIsCapturing(st, &cap) != cudaSuccess ||
-      cap != cudaStreamCaptureStatusNone || (ctx->scratch && ctx->scratch_bytes < bytes) ||
-      scratch(ctx, bytes, &scr) != CUOT_OK) {
-    cudaGetLastError();
-    return launch_split<kTwoRoles>(ctx, a, st);
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) return launch_status(0);
+  if (a.ngroups * 4 >= kInterleaveRows && a.k <= a.ngroups && cap == cudaStreamCaptureStatusNone)
+    a.kk12 = static_cast<Blk *>(pool_alloc(ctx, uint64_t(a.k) * 32, st));
+  if (a.kk12) {
+    const int64_t grid = (a.k + 255) / 256;
+    lpn_interleave_kernel<<<unsigned(grid < 148 * 8 ? grid : 148 * 8), 256, 0, st>>>(a);
+    int rc = launch_status();
+    if (rc == CUOT_OK) rc = launch_split<kInterleaved>(ctx, a, st);
+    if (cudaFreeAsync(a.kk12, st) != cudaSuccess && rc == CUOT_OK) rc = launch_status(0);
+    return rc;
   }
-  a.kk12 = static_cast<Blk *>(scr);
-  const int64_t grid = (a.k + 255) / 256;
-  lpn_interleave_kernel<<<unsigned(grid < 148 * 8 ? grid : 148 * 8), 256, 0, st>>>(a);
-  CUOT_TRY(launch_status());
-  return launch_split<kInterleaved>(ctx, a, st);
+  if (a.k <= kTogether) return launch_split<kTwoRoles>(ctx, a, st);
+  LpnArgs b = a;
+  a.kk2 = nullptr;
+  a.e2 = nullptr;
+  b.kk = b.kk2;
+  b.e = b.e2;
+  b.kk2 = nullptr;
+  b.e2 = nullptr;
+  CUOT_TRY(launch_split<kOneRole>(ctx, a, st));
+  return launch_split<kOneRole>(ctx, b, st);
 }
 
 // Rows [row_lo, row_hi) of one task over [0, n) (lpn_f2.h:72-79), for one

@@ -206,7 +206,12 @@ int cuot_lpn_primal_range(cuot_ctx *ctx, const uint8_t seed[16],
  * BOB (lpn_f2.h:81-101), share the public index matrix, so it is generated
  * once and each index gathers from both kk_send_d and kk_recv_d.  Equal to
  * cuot_lpn_primal on (kk_send_d, e_send_io_d) and on (kk_recv_d,
- * e_recv_io_d); the two row arrays must not alias. */
+ * e_recv_io_d); the two row arrays must not alias.  With d = 10, 2^18 rows or
+ * more and k <= n/4 both kk are copied side by side first, into 32k bytes of
+ * stream-ordered memory from a pool of the context (at most 64 MiB of it is kept
+ * between calls, until the context is destroyed; the scratch arena is not
+ * touched).  Captured calls, and those for which there is no memory, gather
+ * from the two arrays as they are (10.5 M rows: 1.2 ms instead of 0.93). */
 int cuot_lpn_primal_dual(cuot_ctx *ctx, const uint8_t seed[16],
                          const cuot_block *kk_send_d, const cuot_block *kk_recv_d,
                          int64_t k, int d, cuot_block *e_send_io_d,
