@@ -19,6 +19,8 @@ struct cuot_ctx {
 };
 
 namespace cuot {
+// Bytes that a context's pool keeps between calls.
+constexpr uint64_t kPoolKeeps = 64ull << 20;
 // Records a failure message for cuot_last_error() and returns `status`.
 int fail(int status, const char *fmt, ...);
 // Makes ctx's device current for the lifetime of the guard.

@@ -123,7 +123,6 @@ int launch_split(cuot_ctx *ctx, const LpnArgs &a, cudaStream_t st) {
 // Memory of its own for one call on `st`, given back to the context's pool in stream
 // order: no other call's arena, captured graph or stream holds it.  Null if there is
 // none to be had.
-constexpr uint64_t kPoolKeeps = 64ull << 20;  // bytes that the pool keeps between calls
 static void *pool_alloc(cuot_ctx *ctx, uint64_t bytes, cudaStream_t st) {
   static std::mutex mu;
   // other streams of the program may be under capture, which forbids a plain cudaMalloc

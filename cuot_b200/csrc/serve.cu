@@ -69,7 +69,7 @@ uint64_t footprint(const cuot_request &r) {
   const uint64_t n = req_n(r), t = r.t, h = uint64_t(r.h);
   uint64_t b = 2 * 16 * n + 16 * t + t * h;
   if (r.kind == CUOT_KIND_FERRET)
-    b += 2 * 16 * uint64_t(r.k) + 4 * 16 * t * h + 16 * t;
+    b += 2 * 16 * uint64_t(r.k) + 4 * 16 * t * h + 16 * t + (32 * uint64_t(r.k) > kPoolKeeps ? 32 * uint64_t(r.k) - kPoolKeeps : 0);
   else
     b += 3 * 16 * h * t + 2 * 16 * (h + 1) * t + n / 8 + n / 8 + 8 * t;
   return b;
@@ -266,10 +266,13 @@ int cuot_server_create(int device, const cuot_server_config *cfg, cuot_server **
   const uint64_t nmax = 1ull << max_log_n;
   // per slot: PPRF levels (16n) or the one-shot dual LPN of any size up to
   // nmax (transform of `a`, blocks or tile words, pass intermediate; the
-  // library's own sizing), plus the QC twiddle tables of every size
+  // library's own sizing), plus the twiddle tables of the sizes that have some
+  // (not the ternary ones; 2^23 and 2^24 also those of their 2^22 leaves) and
+  // what the context's pool keeps
   uint64_t scratch = 24 * nmax + std::max<uint64_t>(4 * nmax, 512ull << 20) + (64ull << 20);
-  uint64_t tables = 0;
-  for (int e = 10; e <= max_log_n; e++) tables += 16 * (1ull << e) + 32 * (1ull << (e / 2 + 1));
+  uint64_t tables = kPoolKeeps + (max_log_n > kQcfMaxE ? 1ull << 20 : 0);
+  for (int e = 10; e <= max_log_n; e++)
+    if (!tern_supported(e)) tables += 16 * (1ull << e) + 32 * (1ull << (e / 2 + 1));
   int lo_prio = 0, hi_prio = 0;
   cudaSetDevice(device);
   cudaDeviceGetStreamPriorityRange(&lo_prio, &hi_prio);
@@ -280,6 +283,15 @@ int cuot_server_create(int device, const cuot_server_config *cfg, cuot_server **
     cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr);
   }
   int st = CUOT_OK;
+  void *warm_io = nullptr;  // nmax blocks, then as many bits
+  if (cudaMalloc(&warm_io, 16 * nmax + nmax / 8) != cudaSuccess ||
+      cudaMemset(warm_io, 0, 16 * nmax + nmax / 8) != cudaSuccess) {
+    const int rc = cuda_fail(cudaGetLastError(), "QC warm-up allocation");
+    cudaFree(warm_io);
+    cuot_server_destroy(sv);
+    return rc;
+  }
+  uint64_t *warm_a = reinterpret_cast<uint64_t *>(static_cast<uint8_t *>(warm_io) + 16 * nmax);
   for (auto &s : sv->slots) {
     if ((st = cuot_ctx_create(device, &s.ctx))) break;
     // the slots already overlap their requests: one stream per FFT encode
@@ -292,24 +304,14 @@ int cuot_server_create(int device, const cuot_server_config *cfg, cuot_server **
       st = cuda_fail(cudaGetLastError(), "stream/event creation");
       break;
     }
-    // build the QC tables of every size now (the first use of a size synchronises)
-    for (int e = 10; e <= max_log_n && !st; e++) {
-      const uint64_t n = 1ull << e;
-      void *a = nullptr, *pl = nullptr;
-      if (cudaMalloc(&a, n / 8) != cudaSuccess || cudaMalloc(&pl, n / 8) != cudaSuccess) {
-        if (a) cudaFree(a);
-        st = cuda_fail(cudaGetLastError(), "QC warm-up allocation");
-        break;
-      }
-      cudaMemset(a, 0, n / 8);
-      cudaMemset(pl, 0, n / 8);
-      st = cuot_qc_encode(s.ctx, static_cast<uint64_t *>(a), static_cast<uint64_t *>(pl), n, 1, s.lo);
-      cudaStreamSynchronize(s.lo);
-      cudaFree(a);
-      cudaFree(pl);
-    }
+    // every size's encode once, as requests call it: it builds the tables and
+    // loads the kernels, both of which synchronise
+    for (int e = 10; e <= max_log_n && !st; e++)
+      st = cuot_sot_dual_lpn(s.ctx, warm_a, static_cast<cuot_block *>(warm_io), 1ull << e, s.lo);
+    if (!st && cudaStreamSynchronize(s.lo) != cudaSuccess) st = cuda_fail(cudaGetLastError(), "QC warm-up");
     if (st) break;
   }
+  cudaFree(warm_io);
   if (st) {
     cuot_server_destroy(sv);
     return st;

@@ -520,8 +520,10 @@ typedef struct {
   double max_used_bytes;  /* peak footprint of admitted requests */
 } cuot_server_stats;
 typedef struct cuot_server cuot_server;
-/* Creates the slots' contexts and streams, reserves their scratch and builds
- * the QC tables of every size up to 2^max_log_n (synchronises). */
+/* Creates the slots' contexts and streams, reserves their scratch and runs
+ * every size's encode up to 2^max_log_n once, so that no request waits for
+ * tables or kernels to be loaded (synchronises; 16 * 2^max_log_n bytes more
+ * while it runs). */
 int cuot_server_create(int device, const cuot_server_config *cfg,
                        cuot_server **out);
 /* Device bytes reserved by the slots (taken from the budget). */
