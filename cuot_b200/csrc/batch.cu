@@ -555,8 +555,14 @@ int cuot_batch_create(cuot_ctx *ctx, const cuot_batch_item *items, int count,
       leaves += 1ull << items[tk.item].h;
     }
     const uint64_t ctas = uint64_t(sms) * per_sm;
-    b->pprf_group[br] =
-        b->cfg.pprf_threads == 128 ? 128 : pprf_group_size(leaves >> deepest, deepest, ctas);
+    // Smaller groups mean more slots of 2^hmax blocks per CTA; above depth 14 (116 MB
+    // of slots with one per CTA) there is nothing to gain for that (PPRF of 480 trees of
+    // depth 16: one per CTA 465 MB and 1,532 us, two 931 MB and 2,308; of 1,200 of depth
+    // 15 1,707 and 1,711)
+    constexpr int kDeep = 14;
+    b->pprf_group[br] = b->cfg.pprf_threads == 128 ? 128
+                        : hmax[br] > kDeep         ? kPprfThreads
+                                                   : pprf_group_size(leaves >> deepest, deepest, ctas);
     b->pprf_grid[br] = int(std::min<uint64_t>(ctas, tasks.size()));
     const uint64_t slots =
         uint64_t(b->pprf_grid[br]) * ((b->cfg.pprf_threads == 128 ? 128 : kPprfThreads) / b->pprf_group[br]);
