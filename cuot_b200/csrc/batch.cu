@@ -64,14 +64,18 @@ __global__ void __launch_bounds__(kPprfThreads, 3) pprf_batch_kernel(PprfBatchAr
   __syncthreads();
   const int group = threadIdx.x / G, tid = threadIdx.x % G;
   Blk *slot = b.scratch + ((uint64_t(blockIdx.x) * (blockDim.x / G) + group) << b.hmax);
-  for (;;) {
-    group_sync<G>(group);  // previous task finished with s_task and the shared state
-    if (tid == 0) s_task[group] = atomicAdd(b.counter, 1u);
-    group_sync<G>(group);
-    const uint32_t task = s_task[group];
+  // The first trees are dealt out, one to every CTA before any gets its second: from
+  // the queue alone the first CTAs to start would take several each, and a batch of
+  // few trees would leave the others' SMs idle.
+  uint32_t task = group * gridDim.x + blockIdx.x;
+  const uint32_t groups = gridDim.x * (blockDim.x / G);
+  for (;; task = s_task[group]) {
     if (task >= b.ntasks) break;
     const PprfTask tk = b.tasks[task];
     pprf_tree<SEND, G>(b.items[tk.item], b.sot[tk.item] != 0, tk.tree, slot, group, tid);
+    group_sync<G>(group);  // done with the shared state and the task before
+    if (tid == 0) s_task[group] = groups + atomicAdd(b.counter, 1u);
+    group_sync<G>(group);
   }
 }
 

@@ -61,8 +61,9 @@ template <int MODE, int G, bool CHAINED>
 static int launch_on(cuot_ctx *ctx, PprfArgs &a, int threads, cudaStream_t st) {
   uint64_t cap = 0;
   CUOT_TRY((pprf_capacity<MODE, G, CHAINED>(ctx, &cap)));
-  // fewer trees than groups: one tree per CTA as far as the CTAs go
-  const uint64_t grid = a.t < cap ? a.t : cap, groups = grid * (threads / G);
+  // one tree per CTA of 256 threads (pprf_group_size); smaller groups share
+  // resident CTAs, one tree per CTA as far as the CTAs go
+  const uint64_t grid = G == kPprfThreads || a.t < cap ? a.t : cap, groups = grid * (threads / G);
   a.t0 = ctx->t0_d;
   void *scr = nullptr;
   CUOT_TRY(scratch(ctx, ((a.t < groups ? a.t : groups) << a.h) * sizeof(Blk), &scr));
