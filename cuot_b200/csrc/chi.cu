@@ -19,12 +19,12 @@
 // times, once per group of four banks, and a lane reads the copy of its own
 // group: four wavefronts per lookup, where 256-entry byte tables (16 lookups,
 // also 64 KiB) met about eleven, and an eighth of the entries to compute.  The
-// 132 products of the fold are a warp's each: lane l holds c x^(4l + b), b < 4,
+// 128 products of the fold are a warp's each: lane l holds c x^(4l + b), b < 4,
 // for the multiplier c and adds those whose bits of x are set; four XOR
 // reductions over the warp give the product (bit-serial ones by single
 // threads, level by level, took as long as the leaves).
 // Bound by the lookups' wavefronts: 32 x 4 per 32 leaves and SM, 145 us for
-// 2,507 trees of depth 12.  Measured there 675 -> 196 us (64 trees of depth 10: 48 -> 13).
+// 2,507 trees of depth 12.  Measured there 675 -> 180 us (64 trees of depth 10: 45 -> 8).
 #include <atomic>
 
 #include "ctx.cuh"
@@ -45,7 +45,6 @@ __device__ __forceinline__ U128 u128(const uint4 v) {
 __device__ __forceinline__ uint4 to_u4(U128 a) {
   return make_uint4(uint32_t(a.lo), uint32_t(a.lo >> 32), uint32_t(a.hi), uint32_t(a.hi >> 32));
 }
-__device__ __forceinline__ U128 xor128(U128 a, U128 b) { return U128{a.lo ^ b.lo, a.hi ^ b.hi}; }
 // a * x, reduced (x^128 = x^7 + x^2 + x + 1)
 __device__ __forceinline__ U128 mulx(U128 a) {
   const uint64_t c = a.hi >> 63;
@@ -143,6 +142,14 @@ __global__ void __launch_bounds__(kChiThreads) chi_sum_kernel(const uint4 *__res
   const U128 s = u128(__ldg(&seeds[tree])), s4 = gsqr(gsqr(s));
   uint4 acc = make_uint4(0, 0, 0, 0);
   if (Q > 1) {
+    // Leaves are loaded four steps ahead, the first ones beside the table: one step
+    // covers L2's latency and not that of memory, which few deep trees have nothing
+    // else to hide behind (16 trees of depth 20 4,993 us so, 2,877 four ahead).
+    constexpr int kAhead = 4;
+    uint4 first[kAhead];
+#pragma unroll
+    for (int i = 0; i < kAhead; i++)
+      if (i < Q) first[i] = __ldg(&lv[j + kChiThreads * (Q - 1 - i)]);
     U128 u = s4;
 #pragma unroll 1
     for (int l = 0; l < 5; l++) u = gsqr(u);
@@ -163,10 +170,23 @@ __global__ void __launch_bounds__(kChiThreads) chi_sum_kernel(const uint4 *__res
     }
     __syncthreads();
     const char *mine = reinterpret_cast<const char *>(T + (lane & 7));
-    acc = __ldg(&lv[j + kChiThreads * (Q - 1)]);
-    for (int64_t q = Q - 2; q >= 0; q--) {
-      const uint4 next = __ldg(&lv[j + kChiThreads * q]);
-      acc = xor4(to_u4(tmul(mine, acc)), next);
+    if (Q == 2) {
+      acc = xor4(to_u4(tmul(mine, first[0])), first[1]);
+    } else {
+      acc = first[0];
+#pragma unroll 1
+      for (int64_t q = Q - kAhead; q >= 0; q -= kAhead) {  // leaves q + 3 .. q
+        uint4 x[kAhead];
+#pragma unroll
+        for (int i = 0; i < kAhead; i++) x[i] = first[i];
+        if (q) {
+#pragma unroll
+          for (int i = 0; i < kAhead; i++) first[i] = __ldg(&lv[j + kChiThreads * (q - 1 - i)]);
+        }
+        if (q != Q - kAhead) acc = xor4(to_u4(tmul(mine, acc)), x[0]);
+#pragma unroll
+        for (int i = 1; i < kAhead; i++) acc = xor4(to_u4(tmul(mine, acc)), x[i]);
+      }
     }
   } else if (j < L) {
     acc = __ldg(&lv[j]);

@@ -71,3 +71,13 @@ def test_chi_sum_table_edges(ctx, t, h):
         out = torch.empty((t, 16), dtype=torch.uint8, device="cuda")
         ctx.ferret_chi_sum(to_dev(leaves), h, to_dev(seeds), out)
         assert np.array_equal(to_host(out), oracle.ferret_chi_sum(leaves, h, seeds, threads=8))
+
+
+@pytest.mark.parametrize("t,h", [(3, 8), (2, 9), (3, 10), (2, 11), (1, 17)])
+def test_chi_sum_leaves_ahead(ctx, t, h):
+    """Fewer, as many and more steps per thread than are loaded ahead."""
+    rng = np.random.default_rng(t * 31 + h)
+    leaves, seeds = rng_blocks(rng, t << h), rng_blocks(rng, t)
+    out = torch.empty((t, 16), dtype=torch.uint8, device="cuda")
+    ctx.ferret_chi_sum(to_dev(leaves), h, to_dev(seeds), out)
+    assert np.array_equal(to_host(out), oracle.ferret_chi_sum(leaves, h, seeds, threads=8))
