@@ -570,8 +570,10 @@ template <int V, int NW, bool CHAINED>
 static int launch_sparse_as(const uint64_t *a_d, const uint64_t *pos_d, int weight, uint64_t n, uint64_t *out_d,
                             int r2, cudaStream_t st) {
   const uint64_t gx = (n / 64 + 32 * V - 1) / (32 * V);
-  // 64 positions per warp at least, and no more CTAs than fill the chip several times
-  const uint64_t most = (uint64_t(weight) + 1023) / 1024, fill = (2048 + gx - 1) / gx;
+  // A CTA's 32 NW positions of one step, and no more CTAs than fill the chip several
+  // times (a position costs its warp a latency of about 0.2 us: twice as many per CTA
+  // and 2,048 positions at n = 2^16 take 31 us instead of 21)
+  const uint64_t most = (uint64_t(weight) + 32 * NW - 1) / (32 * NW), fill = (2048 + gx - 1) / gx;
   const uint64_t gy = most < fill ? most : fill;
   if (gy > 1 && cudaMemsetAsync(out_d, 0, n / 8, st) != cudaSuccess) return launch_status(0);
   launch_as(CHAINED, r2 ? qc_sparse<true, V, NW, CHAINED> : qc_sparse<false, V, NW, CHAINED>,
@@ -589,6 +591,16 @@ static int launch_sparse(const uint64_t *a_d, const uint64_t *pos_d, int weight,
   // Few words: small tiles, or most SMs stay idle (n = 2^10 with 20,000 positions
   // 17 against 25 us).  From 2^16 on the wide tile is as fast or faster: it loads a
   // position's words independently (2^17 with 2^17 positions 189 against 490).
+  // Dense ones of few words by smaller CTAs (16 / 8 warps: 5,000 positions at 2^16
+  // 24.7 / 20.5 us, 20,000 43.2 / 34.0; one CTA's 256 positions 8.9 / 11.5, and 20,000
+  // at 2^22 831 / 856).
+  if (weight > 2048 && n <= 1ull << 18) {
+    if (n / 64 <= 512)
+      return chained ? launch_sparse_as<1, 8, true>(a_d, pos_d, weight, n, out_d, r2, st)
+                     : launch_sparse_as<1, 8, false>(a_d, pos_d, weight, n, out_d, r2, st);
+    return chained ? launch_sparse_as<4, 8, true>(a_d, pos_d, weight, n, out_d, r2, st)
+                   : launch_sparse_as<4, 8, false>(a_d, pos_d, weight, n, out_d, r2, st);
+  }
   if (n / 64 <= 512)
     return chained ? launch_sparse_as<1, 16, true>(a_d, pos_d, weight, n, out_d, r2, st)
                    : launch_sparse_as<1, 16, false>(a_d, pos_d, weight, n, out_d, r2, st);
