@@ -172,6 +172,13 @@ __global__ void __launch_bounds__(kTrThreads) tr_planes128_to_blocks(const uint4
   }
 }
 
+// The ragged kernels' CTAs of 1,024 blocks are too few below these sizes: a thread
+// of the byte-granular kernel per 64 bits is faster there (to planes and back, us in
+// a graph, that / ragged: 1,000 blocks 2.6 / 5.4 and 1.8 / 3.3, 16,392 2.6 / 3.4 and 1.8 /
+// 3.4, 20,488 3.9 / 3.4 and 2.3 / 3.4, 65,544 6.2 / 3.4 and 2.8 / 3.3, 81,928 7.2 / 3.4 and
+// 3.4 / 3.4, 262,152 17.2 / 4.2 and 5.7 / 4.1).
+constexpr uint64_t kRaggedRows = 18 << 10, kRaggedCols = 72 << 10;
+
 // blocks -> 128 planes, rows % 8 == 0.  out: 128 rows of rows / 8 bytes, any
 // alignment.  A warp writes a plane's 128 bytes of the CTA: lane j the aligned
 // word that holds bytes 4j - m .. 4j - m + 3 of them (m: the row's misalignment);
@@ -413,14 +420,14 @@ int transpose_launch(const void *in, uint64_t rows, uint64_t row_bytes, uint64_t
     return launch_status();
   }
   const bool all_planes = row_bytes == 16 && col_lo == 0 && ncols == 128 && aligned(in, 16);
-  if (all_planes && (rows % 32 || !aligned(out, 4))) {
+  if (all_planes && rows >= kRaggedRows && (rows % 32 || !aligned(out, 4))) {
     const uint64_t grid = (rows + 32 * kTrG - 1) / (32 * kTrG);
     if (grid > 0x7fffffffull) return fail(CUOT_EINVAL, "too many rows");
     tr_blocks_to_ragged<<<unsigned(grid), kTrThreads, 0, st>>>(static_cast<const uint4 *>(in), rows,
                                                                 static_cast<uint8_t *>(out));
     return launch_status();
   }
-  if (rows == 128 && col_lo == 0 && aligned(out, 16) && (ncols % 32 || row_bytes % 4 || !aligned(in, 4))) {
+  if (rows == 128 && ncols >= kRaggedCols && col_lo == 0 && aligned(out, 16) && (ncols % 32 || row_bytes % 4 || !aligned(in, 4))) {
     const uint64_t grid = (ncols + 32 * kTrG - 1) / (32 * kTrG);
     if (grid > 0x7fffffffull) return fail(CUOT_EINVAL, "too many columns");
     tr_ragged_to_blocks<<<unsigned(grid), kTrThreads, 0, st>>>(static_cast<const uint8_t *>(in), ncols, row_bytes,

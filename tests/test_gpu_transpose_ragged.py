@@ -45,3 +45,20 @@ def test_planes_to_blocks(ctx, n, offset, extra):
     ctx.bit_transpose(src, 128, rb, 0, n, out)
     assert np.array_equal(to_host(out), oracle.bit_transpose(x, 128, rb, 0, n).reshape(-1))
     assert untouched(buf, 16 * n, 16)
+
+
+# around the sizes from which tiles are used: below them, last tiles of 8, 40, 1,016 and
+# 1,024 rows, and whole words at odd addresses
+TILES = [18424, 18432, 18440, 73720, 73728, 73736, 73768, 74744, 74752, 131072]
+
+
+@pytest.mark.parametrize("offset", [0, 1, 2, 3])
+@pytest.mark.parametrize("n", TILES)
+def test_tiles_to_planes(ctx, n, offset):
+    test_blocks_to_planes(ctx, n, offset)
+
+
+@pytest.mark.parametrize("offset,extra", [(0, 0), (1, 0), (2, 3), (3, 1), (0, 5)])
+@pytest.mark.parametrize("n", TILES)
+def test_tiles_to_blocks(ctx, n, offset, extra):
+    test_planes_to_blocks(ctx, n, offset, extra)
