@@ -1202,6 +1202,35 @@ static int plane_ahat(cuot_qc_plan *pl, const QcEngine &g, void *scr, cudaStream
   return CUOT_OK;
 }
 
+// Captured launches are not chained, and the FFT's are fewer: smaller sizes than
+// this go to it under capture (a plan's dual LPN in a graph, FFT / ternary: 2^14 28.7 /
+// 32.8 us, 2^15 38.9 / 41.4, 2^16 55.3 / 47.2).
+constexpr int kTernCapturedMinE = 16;
+
+static int plan_dual(cuot_qc_plan *pl, const cuot_block *in_d, cuot_block *out_d, bool r2, cudaStream_t st) {
+  cuot_ctx *ctx = pl->ctx;
+  DeviceGuard dg(ctx);
+  const bool either = pl->kind == kQcTern && pl->e < kTernCapturedMinE && pl->planes_ready;
+  const int batch = pl->planes_per_pass(pl->kind, 128), fft_batch = pl->planes_per_pass(kQcFft, 128);
+  uint64_t bytes = dual_scratch_bytes(ctx, pl->kind, pl->e, batch, r2);
+  QcKind kind = pl->kind;
+  if (either) {  // room for both, so that a capture finds it; one that does not keeps to the ternary transform
+    const uint64_t fft = dual_scratch_bytes(ctx, kQcFft, pl->e, fft_batch, r2);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) return launch_status(0);
+    if (cap == cudaStreamCaptureStatusNone)
+      bytes = bytes > fft ? bytes : fft;
+    else if (ctx->scratch_bytes >= fft)
+      kind = kQcFft;
+  }
+  QcEngine g;
+  CUOT_TRY(engine(ctx, pl->e, kind, false, &g));
+  void *scr;
+  CUOT_TRY(scratch(ctx, kind == pl->kind ? bytes : dual_scratch_bytes(ctx, kind, pl->e, fft_batch, r2), &scr));
+  return eng_dual(ctx, g, pl->e, kind == pl->kind ? pl->ahat : pl->plane_ahat, in_d, out_d, r2,
+                  static_cast<uint8_t *>(scr), kind == pl->kind ? batch : fft_batch, st);
+}
+
 extern "C" {
 
 int cuot_qc_gen_a(cuot_ctx *ctx, const uint8_t key[16], uint64_t n, uint64_t *a_d, void *stream) {
@@ -1241,8 +1270,11 @@ int cuot_qc_plan_create(cuot_ctx *ctx, const uint64_t *a_d, uint64_t n, void *st
   void *scr = nullptr;
   if (st == CUOT_OK) st = scratch(ctx, ahat_scratch_bytes(pl->kind, e), &scr);
   if (st == CUOT_OK) st = eng_ahat(g, e, a_d, scr, pl->ahat, true, static_cast<cudaStream_t>(stream));
+  const void *planes;
+  if (st == CUOT_OK && e < kTernCapturedMinE) st = plane_ahat(pl, g, scr, static_cast<cudaStream_t>(stream), &planes);
   if (st != CUOT_OK) {
     if (pl->ahat) cudaFree(pl->ahat);
+    if (pl->plane_ahat) cudaFree(pl->plane_ahat);
     delete pl;
     return st;
   }
@@ -1286,28 +1318,12 @@ int cuot_qc_plan_encode(cuot_qc_plan *pl, uint64_t *planes_io_d, int nplanes, vo
 
 int cuot_qc_plan_dual_lpn(cuot_qc_plan *pl, cuot_block *io_d, void *stream) {
   if (!pl || !io_d) return fail(CUOT_EINVAL, "bad argument");
-  cuot_ctx *ctx = pl->ctx;
-  DeviceGuard dg(ctx);
-  QcEngine g;
-  CUOT_TRY(engine(ctx, pl->e, pl->kind, false, &g));
-  const int batch = pl->planes_per_pass(pl->kind, 128);
-  void *scr;
-  CUOT_TRY(scratch(ctx, dual_scratch_bytes(ctx, pl->kind, pl->e, batch, false), &scr));
-  return eng_dual(ctx, g, pl->e, pl->ahat, io_d, io_d, false, static_cast<uint8_t *>(scr), batch,
-                  static_cast<cudaStream_t>(stream));
+  return plan_dual(pl, io_d, io_d, false, static_cast<cudaStream_t>(stream));
 }
 
 int cuot_qc_plan_dual_lpn_r2(cuot_qc_plan *pl, const cuot_block *in_d, cuot_block *out_d, void *stream) {
   if (!pl || !in_d || !out_d) return fail(CUOT_EINVAL, "bad argument");
-  cuot_ctx *ctx = pl->ctx;
-  DeviceGuard dg(ctx);
-  QcEngine g;
-  CUOT_TRY(engine(ctx, pl->e, pl->kind, false, &g));
-  const int batch = pl->planes_per_pass(pl->kind, 128);
-  void *scr;
-  CUOT_TRY(scratch(ctx, dual_scratch_bytes(ctx, pl->kind, pl->e, batch, true), &scr));
-  return eng_dual(ctx, g, pl->e, pl->ahat, in_d, out_d, true, static_cast<uint8_t *>(scr), batch,
-                  static_cast<cudaStream_t>(stream));
+  return plan_dual(pl, in_d, out_d, true, static_cast<cudaStream_t>(stream));
 }
 
 int cuot_qc_encode(cuot_ctx *ctx, const uint64_t *a_d, uint64_t *planes_io_d, uint64_t n,
