@@ -1150,12 +1150,25 @@ static int one_shot_batch(const cuot_ctx *ctx, QcKind kind, uint64_t n) {
   return batch > 128 ? 128 : batch;
 }
 
-// Scratch of cuot_sot_dual_lpn (r2: cuot_sot_dual_lpn_r2) at n = 2^e on ctx.
-uint64_t qc_one_shot_dual_bytes(const cuot_ctx *ctx, int e, bool r2) {
-  const QcKind kind = dual_kind(ctx, e, ctx->qc_planes_per_pass);
+static uint64_t one_shot_bytes(const cuot_ctx *ctx, QcKind kind, int e, bool r2) {
   const uint64_t ds = dual_scratch_bytes(ctx, kind, e, one_shot_batch(ctx, kind, 1ull << e), r2);
   const uint64_t as = ahat_scratch_bytes(kind, e);
   return ahat_bytes(kind, e, false) + (ds > as ? ds : as);
+}
+
+// Captured launches are not chained, and the FFT's are fewer: smaller sizes than
+// these go to it under capture (in a graph, FFT / ternary: a plan's dual LPN of 2^14 28.7 /
+// 32.8 us, 2^15 38.9 / 41.4, 2^16 55.3 / 47.2; a one-shot one 34.0 / 45.1, 44.8 / 57.4,
+// 62.2 / 65.6, 2^17 105.0 / 92.2).  Calls that are not captured make room for it too.
+constexpr int kTernCapturedMinE = 16, kTernCapturedOneShotMinE = 17;
+
+// Scratch of cuot_sot_dual_lpn (r2: cuot_sot_dual_lpn_r2) at n = 2^e on ctx.
+uint64_t qc_one_shot_dual_bytes(const cuot_ctx *ctx, int e, bool r2) {
+  const QcKind kind = dual_kind(ctx, e, ctx->qc_planes_per_pass);
+  const uint64_t bytes = one_shot_bytes(ctx, kind, e, r2);
+  if (kind != kQcTern || e >= kTernCapturedOneShotMinE) return bytes;
+  const uint64_t fft = one_shot_bytes(ctx, kQcFft, e, r2);
+  return bytes > fft ? bytes : fft;
 }
 
 }  // namespace cuot
@@ -1201,11 +1214,6 @@ static int plane_ahat(cuot_qc_plan *pl, const QcEngine &g, void *scr, cudaStream
   pl->planes_ready = cap == cudaStreamCaptureStatusNone;
   return CUOT_OK;
 }
-
-// Captured launches are not chained, and the FFT's are fewer: smaller sizes than
-// this go to it under capture (a plan's dual LPN in a graph, FFT / ternary: 2^14 28.7 /
-// 32.8 us, 2^15 38.9 / 41.4, 2^16 55.3 / 47.2).
-constexpr int kTernCapturedMinE = 16;
 
 static int plan_dual(cuot_qc_plan *pl, const cuot_block *in_d, cuot_block *out_d, bool r2, cudaStream_t st) {
   cuot_ctx *ctx = pl->ctx;
@@ -1354,14 +1362,23 @@ static int one_shot_dual(cuot_ctx *ctx, const uint64_t *a_d, const cuot_block *i
   CUOT_TRY(check_n(n, &e));
   DeviceGuard dg(ctx);
   QcEngine g;
-  const QcKind kind = dual_kind(ctx, e, ctx->qc_planes_per_pass);
+  QcKind kind = dual_kind(ctx, e, ctx->qc_planes_per_pass);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  uint64_t bytes = qc_one_shot_dual_bytes(ctx, e, r2);
+  if (kind == kQcTern && e < kTernCapturedOneShotMinE) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) return launch_status(0);
+    if (cap != cudaStreamCaptureStatusNone) {
+      if (ctx->scratch_bytes >= one_shot_bytes(ctx, kQcFft, e, r2)) kind = kQcFft;
+      bytes = one_shot_bytes(ctx, kind, e, r2);
+    }
+  }
   CUOT_TRY(engine(ctx, e, kind, false, &g));
   const int batch = one_shot_batch(ctx, kind, n);
   const uint64_t ab = ahat_bytes(kind, e, false);
   void *scr;
-  CUOT_TRY(scratch(ctx, qc_one_shot_dual_bytes(ctx, e, r2), &scr));
+  CUOT_TRY(scratch(ctx, bytes, &scr));
   uint8_t *work = static_cast<uint8_t *>(scr) + ab;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
   CUOT_TRY(eng_ahat(g, e, a_d, work, scr, false, st));
   return eng_dual(ctx, g, e, scr, in_d, out_d, r2, work, batch, st);
 }

@@ -963,6 +963,9 @@ void launch_col_inv(const QcfTables *t, int ntr, cudaStream_t st, const double2 
 
 bool qcf_supported(int e) { return e >= 10 && e <= kQcfMaxE; }
 
+// Builds a size's tables on its own stream, outside any capture of the caller's.
+static int make_tables(cuot_ctx *ctx, int e, QcfTables **out);
+
 int qcf_get_tables(cuot_ctx *ctx, int e, QcfTables **out) {
   if (!qcf_supported(e)) return fail(CUOT_ENOTSUP, "QC FFT backend: n = 2^%d outside [2^10, 2^%d]", e, kQcfMaxE);
   if (ctx->qcf_tables[e]) {
@@ -970,6 +973,14 @@ int qcf_get_tables(cuot_ctx *ctx, int e, QcfTables **out) {
     return CUOT_OK;
   }
   CUOT_TRY(set_attrs());
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  const int st = make_tables(ctx, e, out);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  return st;
+}
+
+static int make_tables(cuot_ctx *ctx, int e, QcfTables **out) {
   QcfTables *t = new QcfTables{};
   t->e = e;
   t->owner = ctx;
@@ -990,10 +1001,10 @@ int qcf_get_tables(cuot_ctx *ctx, int e, QcfTables **out) {
     qcf_free(t);
     return fail(CUOT_ECUDA, "QC FFT stream / event creation failed");
   }
-  qcf_gen_roots<<<8, 256>>>(t->e1, t->T1);
-  qcf_gen_roots<<<8, 256>>>(t->e2, t->T2);
-  qcf_gen_fourstep<<<256, 256>>>(t->e1, t->e2, t->fs);
-  if (cudaDeviceSynchronize() != cudaSuccess || cudaGetLastError() != cudaSuccess) {
+  qcf_gen_roots<<<8, 256, 0, t->aux>>>(t->e1, t->T1);
+  qcf_gen_roots<<<8, 256, 0, t->aux>>>(t->e2, t->T2);
+  qcf_gen_fourstep<<<256, 256, 0, t->aux>>>(t->e1, t->e2, t->fs);
+  if (cudaStreamSynchronize(t->aux) != cudaSuccess || cudaGetLastError() != cudaSuccess) {
     qcf_free(t);
     return fail(CUOT_ECUDA, "QC FFT table generation failed");
   }
