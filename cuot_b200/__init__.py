@@ -112,6 +112,7 @@ class Context:
     def __init__(self, device: int = 0):
         self.lib = load()
         self.device = device
+        self.tuning: dict[int, int] = {}  # what set_tuning set
         h = ctypes.c_void_p()
         _check(self.lib.cuot_ctx_create(C.c_int(device), C.byref(h)), "cuot_ctx_create")
         self.h = h
@@ -138,6 +139,7 @@ class Context:
 
     def set_tuning(self, key: int, value: int):
         _check(self.lib.cuot_ctx_set_tuning(self.h, C.c_int(key), C.c_int64(value)), "cuot_ctx_set_tuning")
+        self.tuning[key] = value
 
     def qc_fft_margin(self, reset: bool = True) -> float:
         """Largest |v - round(v)| rounded by this context's fp64 FFT encodes

@@ -122,7 +122,10 @@ def tune_single(ctx, inst, table: TuningTable | None = None, reps: int = 3):
             res[thr] = _time(lambda st: ctx.ferret_pprf_sender(inst.d_roots, h, inst.delta, inst.v, lsum, rsum, ss,
                                                                stream=st), stream, reps)
         hit = {"pprf_threads": min(res, key=res.get), "pprf_ms": res}
-        if inst.kind == 1:
+        # (a pass's planes bound the scratch of a ternary dual LPN, whose fastest is the default)
+        ternary = 1 << 14 <= inst.n <= 1 << 22 and not (ctx.tuning.get(ctx.TUNE_QC_BACKEND)
+                                                        or ctx.tuning.get(ctx.TUNE_QC_RECORD_MARGIN))
+        if inst.kind == 1 and not ternary:
             base = max(1, (512 << 20) // (4 * inst.n))  # the library's default batch
             qres = {}
             for planes in sorted({max(1, base // 4), max(1, min(128, base // 2)), min(128, base)}):

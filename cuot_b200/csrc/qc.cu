@@ -909,10 +909,11 @@ static int tern_aux(cuot_ctx *ctx, int e, int njobs, cudaStream_t st, TernAux **
   if (ctx->qc_streams != 2 || (uint64_t(njobs) << e) < (1ull << kTernAuxMinE)) return CUOT_OK;
   if (!ctx->tern_aux[e]) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
       cudaGetLastError();
       return CUOT_OK;
     }
+    if (cap != cudaStreamCaptureStatusNone) return CUOT_OK;
     TernAux *a = new TernAux{};
     if (cudaStreamCreateWithFlags(&a->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&a->ev[0], cudaEventDisableTiming) != cudaSuccess ||

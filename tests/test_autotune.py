@@ -55,3 +55,35 @@ def test_winners_of_earlier_launch_rules_are_measured_again(fakes, tmp_path):
     best, _ = autotune.tune_batch(None, [i], table=table)
     assert best["pprf_threads"] == 256 and table.get(autotune.batch_key([i]))["config"] == best
     assert table.get(autotune.shape_key(i.kind, i.n, i.h)) is None
+
+
+class FakeContext:
+    TUNE_PPRF_THREADS, TUNE_QC_PLANES, TUNE_QC_BACKEND, TUNE_QC_RECORD_MARGIN = 1, 2, 3, 5
+
+    def __init__(self, **tuning):
+        self.tuning, self.calls = {getattr(self, k): v for k, v in tuning.items()}, []
+
+    def set_tuning(self, key, value):
+        self.tuning[key] = value
+
+    def ferret_pprf_sender(self, *a, **kw):
+        pass
+
+    def sot_dual_lpn(self, *a, **kw):
+        self.calls.append(self.tuning.get(self.TUNE_QC_PLANES))
+
+
+@pytest.mark.parametrize("log_n,tuning,swept", [(13, {}, True), (14, {}, False), (22, {}, False), (23, {}, True),
+                                                (20, dict(TUNE_QC_BACKEND=2), True), (20, dict(TUNE_QC_BACKEND=1), True),
+                                                (20, dict(TUNE_QC_RECORD_MARGIN=1), True)])
+def test_planes_are_tuned_where_a_pass_depends_on_them(fakes, monkeypatch, tmp_path, log_n, tuning, swept):
+    """The ternary dual LPN takes all its planes at once unless the caller bounds its scratch."""
+    fakes(lambda ret: 1.0)
+    monkeypatch.setattr(torch, "empty", lambda *a, **kw: None)
+    monkeypatch.setattr(autotune, "_time", lambda fn, stream, reps: fn(None) or 1.0)
+    i = inst(kind=1, n=1 << log_n)
+    i.a = i.v = i.d_roots = i.delta = None
+    ctx = FakeContext(**tuning)
+    hit = autotune.tune_single(ctx, i, table=autotune.TuningTable(str(tmp_path / "t.json")))
+    assert ("qc_planes_per_pass" in hit) == swept == bool(ctx.calls)
+    assert (ctx.TUNE_QC_PLANES in ctx.tuning) == swept
