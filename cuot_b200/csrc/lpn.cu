@@ -155,7 +155,8 @@ static void *pool_alloc(cuot_ctx *ctx, uint64_t bytes, cudaStream_t st) {
 // Both roles, d = 10.  From kInterleaveRows rows on, kk and kk2 are first copied
 // side by side (470,016 rows 66.8 -> 58.6 us with the copy, 10,485,760 rows 1197 ->
 // 927; at 131,072 rows the 3 us that the gathers would save are the copy's launch),
-// unless `st` is captured or there is no memory.  Without the copy two arrays of
+// unless `st` is captured, kk has more than half as many blocks as there are rows
+// (262,144 of both: nothing gained), or there is no memory.  Without the copy two arrays of
 // more than about 32 MB each fall out of L2 together: one role after the other
 // is then faster (10,485,760 rows, k = 1.6 / 2 / 2.6 / 4 million: 1,227 / 1,623 / 2,128 /
 // 2,762 us together, 1,602 / 1,602 / 1,603 / 1,758 in turn; copied 950 / 1,058 / 1,224).
@@ -163,7 +164,7 @@ constexpr int64_t kInterleaveRows = 1 << 18, kTogether = 2000000;
 int launch_dual(cuot_ctx *ctx, LpnArgs a, cudaStream_t st) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) return launch_status(0);
-  if (a.ngroups * 4 >= kInterleaveRows && a.k <= a.ngroups && cap == cudaStreamCaptureStatusNone)
+  if (a.ngroups * 4 >= kInterleaveRows && a.k <= 2 * a.ngroups && cap == cudaStreamCaptureStatusNone)
     a.kk12 = static_cast<Blk *>(pool_alloc(ctx, uint64_t(a.k) * 32, st));
   if (a.kk12) {
     const int64_t grid = (a.k + 255) / 256;

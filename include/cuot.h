@@ -207,7 +207,7 @@ int cuot_lpn_primal_range(cuot_ctx *ctx, const uint8_t seed[16],
  * once and each index gathers from both kk_send_d and kk_recv_d.  Equal to
  * cuot_lpn_primal on (kk_send_d, e_send_io_d) and on (kk_recv_d,
  * e_recv_io_d); the two row arrays must not alias.  With d = 10, 2^18 rows or
- * more and k <= n/4 both kk are copied side by side first, into 32k bytes of
+ * more and k < n/2 both kk are copied side by side first, into 32k bytes of
  * stream-ordered memory from a pool of the context (at most 64 MiB of it is kept
  * between calls, until the context is destroyed; the scratch arena is not
  * touched).  Captured calls, and those for which there is no memory, gather

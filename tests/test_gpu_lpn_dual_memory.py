@@ -66,6 +66,23 @@ def test_beside_a_capture_and_on_two_streams():
     ctx.close()
 
 
+@pytest.mark.parametrize("n,k,launches", [((1 << 18) - 4, 65536, 1), (1 << 18, 65536, 2), (1 << 18, 131072, 2),
+                                          (1 << 18, 131073, 1)])
+def test_where_the_copy_is_made(n, k, launches):
+    """n: rows in groups of four (the last four are not)."""
+    import cuot_b200
+    ctx = cuot_b200.Context(0)
+    n += 4
+    s, kk, e, want = _case(n, k)
+    torch.cuda.synchronize()
+    before = _launches()
+    ctx.lpn_primal_dual(s, kk[0], kk[1], e[0], e[1])
+    assert _launches() - before == launches
+    for r in range(2):
+        assert np.array_equal(to_host(e[r]), want[r]), r
+    ctx.close()
+
+
 @pytest.mark.parametrize("n,k", [((1 << 18) + 5, 2000000), ((1 << 18) + 5, 2000001), (29, 2000001)])
 def test_large_k_in_turn(n, k):
     import cuot_b200
