@@ -273,14 +273,14 @@ class Instance:
 # stage's kernels per step, from ncu captures of the same bench command, one
 # kernel and one to three launches per capture (ncu starts every launch with
 # cold caches, so intermediate that steady state keeps in L2 is counted):
-# ferret_b13: the dual-role LPN launch (profiles/pprf_lpn_ferret_b13.md);
+# ferret_b13: both roles' LPN and the copy of their kk (profiles/pprf_lpn_ferret_b13.md);
 # sot_n20_fft: gather, 16 launches of each transform pass and scatter per role
 # (profiles/qc_fft_sot_n20.md); sot_n20_ntt: the same workload on the NTT
 # backend, which scales the SOT encodes of NTT sizes (profiles/qc_ntt_sot_n20.md);
 # sot_n22_fft: 32 transforms of 251.8 MB per role plus gather and scatter
 # (profiles/qc_fft_sot_n22.md).
 NCU_TRAFFIC_PER_STEP = {
-    "ferret_b13:lpn": 631.83e6,
+    "ferret_b13:lpn": 350.3e6 + 283.1e6 + 14.5e6,
     "sot_n20_fft:dual_lpn": 2 * (16.79e6 + 16 * 88.24e6 + 16.86e6),
     "sot_n20_ntt:dual_lpn": 2 * (509.60e6 + 1024.36e6 + 563.98e6 + 33.58e6),
     "sot_n22_fft:dual_lpn": 2 * (32 * 251.75e6 + 84.17e6 + 82.25e6),
@@ -381,6 +381,35 @@ def fp64_roofline(qct: dict) -> dict | None:
             "work": "fft_fp64_flops of qc_transform per step"}
 
 
+def bound_by_pipe(roofline: dict, qct: dict, clocks: dict, props) -> None:
+    """Adds the encode's own bound (fp64 of FFTs, ALU of ternary transforms) to
+    its stage's HBM object, and names the nearest bound of them."""
+    roofline["nearest_bound"] = roofline["bound"]
+    nearest = roofline["frac"]
+    for pipe, r in (("fp64", fp64_roofline(qct)), ("alu", alu_roofline(qct, clocks, props))):
+        if r:
+            roofline[pipe] = r
+            if r["frac"] > nearest:
+                roofline["nearest_bound"], nearest = pipe, r["frac"]
+
+
+TERN_OPS_PER_WORD = 600  # ALU operations of the ternary transform per coefficient and 32 planes
+
+
+def alu_roofline(qct: dict, clocks: dict, props) -> dict | None:
+    """A purely ternary encode stage against the integer ALU pipe (64 lanes
+    per SM and clock): the bound of its logic operations, reported beside the
+    stage's HBM fraction."""
+    if not qct.get("ternary_coefficients") or qct["fft_fp64_flops"] or qct["ntt_butterflies"]:
+        return None
+    mhz = clocks.get("sm_mhz") or clocks.get("sm_max_mhz") or 1965.0
+    peak = props.multi_processor_count * 64 * mhz * 1e6 / 1e12
+    achieved = 4 * qct["ternary_coefficients"] * TERN_OPS_PER_WORD / (qct["stage_ms"] / 1e3) / 1e12
+    return {"achieved": achieved, "peak": peak, "unit": "TOP/s", "frac": achieved / peak,
+            "model": f"{TERN_OPS_PER_WORD} ALU operations per coefficient and 32 planes (this transform's own count, "
+                     "three quarters of them in the inner products); peak = SMs x 64 lanes x median SM clock"}
+
+
 AES_PEAK_MODEL = ("T-table AES: 160 shared-memory lookups per block (10 rounds x 16), one conflict-free "
                   "32-lane lookup wavefront per clock per SM; peak = SMs x 32 x median SM clock / 160")
 
@@ -388,16 +417,17 @@ AES_PEAK_MODEL = ("T-table AES: 160 shared-memory lookups per block (10 rounds x
 LPN_L1_MODEL = ("L1 wavefronts per LPN row pair (the dual-role kernel: one index computation for the two "
                 "parties' rows): index-AES table lookups (145 per block for d = 10 blocks of a 4-row group "
                 "plus 15 shared round-1 lookups, i.e. (145 d + 15) / 4 per row, 32 lanes per wavefront) + 2d "
-                "random 16-byte kk gathers (one line, one wavefront each) + both rows' 16-byte read and write "
+                "random 16-byte kk gathers, or d 32-byte ones where both parties' kk lie side by side (one line, one "
+                "wavefront each) + both rows' 16-byte read and write "
                 "(1/8 wavefront each); rows counted per role, peak rows/s = SMs x median SM clock / "
                 "wavefronts per role row")
 
 
-def lpn_l1_roofline(rows: int, d: int, ms: float, clocks: dict, props) -> dict:
+def lpn_l1_roofline(rows: int, d: int, ms: float, clocks: dict, props, side_by_side: bool = False) -> dict:
     """LPN rows per second against the L1 wavefront bound the index AES and
     the kk gathers share (both go through the L1/shared data pipe)."""
     mhz = clocks.get("sm_mhz") or clocks.get("sm_max_mhz") or 1965.0
-    per_row = ((145 * d + 15) / 4 / 32 + 2 * d + 0.5) / 2  # per role row
+    per_row = ((145 * d + 15) / 4 / 32 + (1 if side_by_side else 2) * d + 0.5) / 2  # per role row
     peak = props.multi_processor_count * mhz * 1e6 / per_row
     achieved = rows / (ms / 1e3)
     return {"rows_per_step": rows, "rows_per_s": achieved, "peak_rows_per_s": peak, "frac": achieved / peak,
@@ -455,7 +485,8 @@ def aes_roofline(inst: Instance, stages: dict, clocks: dict, props) -> dict:
         a = cnt / (stages[k][0] / 1e3)
         res[k] = {"aes_per_step": cnt, "aes_per_s": a, "frac": a / peak}
     if "lpn" in counts and inst.d == 10:
-        res["lpn_l1_roofline"] = lpn_l1_roofline(2 * inst.n, inst.d, stages["lpn"][0], clocks, props)
+        res["lpn_l1_roofline"] = lpn_l1_roofline(2 * inst.n, inst.d, stages["lpn"][0], clocks, props,
+                                                 side_by_side=inst.n > 1 << 18 and 2 * inst.k < inst.n)
     return res
 
 
@@ -1013,7 +1044,7 @@ def run_batch(args):
         aes[k] = {"aes_per_step": cnt, "aes_per_s": a, "frac": a / aes_peak}
     fer_rows = sum(2 * i.n for i in insts if i.kind == KIND_FERRET and i.d == 10)
     if fer_rows and stages.get("lpn"):
-        aes["lpn_l1_roofline"] = lpn_l1_roofline(fer_rows, 10, stages["lpn"], clocks, props)
+        aes["lpn_l1_roofline"] = lpn_l1_roofline(fer_rows, 10, stages["lpn"], clocks, props, side_by_side=True)
     out = {
         "metric": metric_name(args.workload),
         "value": world * cots / (ms / 1e3), "unit": "COTs/s", "n_gpus": world, "steps": args.steps,
@@ -1050,8 +1081,8 @@ def run_batch(args):
         "gpu_launches": launches * args.steps,
         "clocks": clocks,
     }
-    if dom == "sot_encode" and fp64_roofline(out["qc_transform"]):
-        out["roofline"]["fp64"] = fp64_roofline(out["qc_transform"])
+    if dom == "sot_encode":
+        bound_by_pipe(out["roofline"], out["qc_transform"], clocks, props)
     batch.close()
     batch2.close()
     if args.serve_requests > 0:
@@ -1428,8 +1459,8 @@ def run_ours(args):
         out["transpose"] = transpose_roofline(inst, flush, peaks, peak_kind)
     if inst.spec["kind"] == "sot":
         out["qc_transform"] = qc_report([inst.n], lpn_ms, inst.sctx.measure_fp64_tflops)
-        if dom == "dual_lpn" and fp64_roofline(out["qc_transform"]):
-            out["roofline"]["fp64"] = fp64_roofline(out["qc_transform"])
+        if dom == "dual_lpn":
+            bound_by_pipe(out["roofline"], out["qc_transform"], clocks, torch.cuda.get_device_properties(local))
     if rank == 0 and world == 1:
         rg = reference_gpu_context(args.workload, pprf_ms, lpn_ms)
         if rg:

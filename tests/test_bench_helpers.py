@@ -43,3 +43,31 @@ def test_lpn_l1_roofline_model():
     assert abs(r["wavefronts_per_row"] - ((145 * 10 + 15) / 4 / 32 + 2 * 10 + 0.5) / 2) < 1e-12
     assert abs(r["peak_rows_per_s"] - 148 * 1965e6 / r["wavefronts_per_row"]) < 1.0
     assert 0.85 < r["frac"] < 0.95
+
+
+class Props:
+    multi_processor_count = 148
+
+
+def test_lpn_l1_roofline_of_kk_side_by_side():
+    r = bench.lpn_l1_roofline(2 * 10485760, 10, 0.9425, {"sm_mhz": 1965.0}, Props(), side_by_side=True)
+    assert abs(r["wavefronts_per_row"] - ((145 * 10 + 15) / 4 / 32 + 10 + 0.5) / 2) < 1e-12
+    assert 0.8 < r["frac"] < 0.9
+
+
+def test_encode_is_bound_by_its_pipe():
+    clocks, n = {"sm_mhz": 1965.0}, 1 << 20
+    tern = bench.qc_report([n], 0.765, None)
+    r = bench.alu_roofline(tern, clocks, Props())
+    assert abs(r["achieved"] * 1e12 * 0.765e-3 - 2 * n * 4 * bench.TERN_OPS_PER_WORD) < 1.0
+    assert abs(r["peak"] - 148 * 64 * 1.965e-3) < 1e-9 and abs(r["frac"] - r["achieved"] / r["peak"]) < 1e-12
+    mixed = bench.qc_report([n, 1 << 23], 20.0, None)
+    assert bench.alu_roofline(mixed, clocks, Props()) is None
+    out = {"bound": "hbm", "frac": 0.03}
+    bench.bound_by_pipe(out, tern, clocks, Props())
+    assert out["alu"]["frac"] == r["frac"] and out["nearest_bound"] == "alu" and "fp64" not in out
+    out = {"bound": "hbm", "frac": 0.9}
+    bench.bound_by_pipe(out, bench.qc_transform_report([n], 1.5, fp64_peak=37.0), clocks, Props())
+    assert out["nearest_bound"] == "hbm" and out["fp64"]["frac"] < 0.9
+    bench.bound_by_pipe(out, mixed, clocks, Props())
+    assert "alu" not in out
