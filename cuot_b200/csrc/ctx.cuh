@@ -52,8 +52,8 @@ uint64_t qc_one_shot_dual_bytes(const cuot_ctx *ctx, int e, bool r2);
 int qc_kind(const cuot_ctx *ctx, int e);
 int qc_prepare(cuot_ctx *ctx, int kind, int e);
 uint64_t qc_ahat_bytes(int kind, int e);
-// Encodes of two sizes with the same lane share per-size FFT state (the
-// tables' second stream, events and plane-parity words) and must not run at
+// Encodes of two sizes with the same lane share per-size state (second
+// stream and events; the FFT's plane-parity words) and must not run at
 // the same time; different lanes may.
 int qc_lane(int kind, int e);
 uint64_t qc_y_bytes(const cuot_ctx *ctx, int kind, int e, int batch);

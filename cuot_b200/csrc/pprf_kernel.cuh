@@ -53,14 +53,12 @@ __device__ __forceinline__ Blk mask_lsb(Blk b) {
   return b;
 }
 
-// Shared-memory state of a group of G threads (256, 128 or 64): the levels of up to G nodes, the
-// warps' level sums (left, right), double-buffered by level parity, and the
-// receiver's path.
+// Shared-memory state of a group of G threads (256, 128 or 64): the levels of up to G nodes and the
+// warps' level sums (left, right), double-buffered by level parity.
 template <int G>
 struct PprfSmem {
   Blk lev[G + G / 2];
   Blk red[2][2][G / 32];
-  unsigned long long ap;
   // Level of 2^k <= G nodes: levels alternate between the two parts.
   __device__ Blk *level(int k) {
     constexpr int kLog = G == 256 ? 8 : G == 128 ? 7 : 6;

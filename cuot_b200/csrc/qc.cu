@@ -1,8 +1,9 @@
 // qc.cu -- exact quasi-cyclic encode over GF(2)[x]/(x^n - 1) (SOT dual LPN):
-// the entry points, the choice of transform per size (the fp64 FFT of
-// qc_fft.cu up to 2^22, GF(2) Karatsuba over it in qc_kara.cu for dual LPNs
-// at 2^23 and 2^24, the number-theoretic transform below otherwise), the
-// sparse encode and the AES-CTR helpers.
+// the entry points, the choice of transform per call and size (the ternary
+// GF(2) transform of qc_tern.cu for dual LPNs of 2^14 to 2^22, the fp64 FFT of
+// qc_fft.cu for others and for plane encodes up to 2^22, GF(2) Karatsuba over it
+// in qc_kara.cu for dual LPNs at 2^23 and 2^24, the number-theoretic transform
+// below otherwise), the sparse encode and the AES-CTR helpers.
 //
 // The reference multiplies with float32 cuFFT and recovers bits by truncating
 // the unnormalised result (silent/quasi_cyclic.cu:34-49, 118-128), which is
@@ -1035,7 +1036,7 @@ uint64_t qc_ahat_bytes(int kind, int e) { return ahat_bytes(QcKind(kind), e, fal
 int qc_lane(int kind, int e) {
   if (kind == kQcFft) return e;
   if (kind == kQcKara) return kQcfMaxE;  // its leaves run on the 2^22 FFT tables
-  return 64 + e;                         // the NTT and the ternary transform keep no per-call state in the context
+  return 64 + e;  // the NTT keeps no per-call state in the context, the ternary transform only its size's second stream
 }
 
 uint64_t qc_layout_bytes(int kind, int e, int njobs) {

@@ -77,7 +77,8 @@ constexpr int kTrCpw = kTrCh / (kTrThreads / 32);  // chunks per warp
 static_assert(kTrCpw >= 1 && kTrCh >= 8, "tile shape");
 // The 128-plane kernels are chained up to 16 times the general limit, 2^22 blocks:
 // their few waves of CTAs then start while the kernel before drains (to planes and
-// back, 2^21 blocks: 27.1 -> 25.0 us, 2^22 47.7 -> 46.4, 2^24 no difference).
+// back, one buffer over and over, 2^21 blocks: 27.1 -> 25.0 us, 2^22 47.7 -> 46.4, 2^24
+// no difference; 2^21 of new buffers 32.7 -> 29.0).
 // Bound by the two trips through memory, and by the last wave (8 CTAs per SM, 1.7
 // waves at 2^21).
 constexpr uint64_t kTrChain = 16;
