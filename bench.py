@@ -273,13 +273,15 @@ class Instance:
 # stage's kernels per step, from ncu captures of the same bench command, one
 # kernel and one to three launches per capture (ncu starts every launch with
 # cold caches, so intermediate that steady state keeps in L2 is counted):
-# ferret_b13: both roles' LPN and the copy of their kk (profiles/pprf_lpn_ferret_b13.md);
+# ferret_b13: the sender's and the receiver's PPRF; both roles' LPN and the copy of
+# their kk (profiles/pprf_lpn_ferret_b13.md);
 # sot_n20_fft: gather, 16 launches of each transform pass and scatter per role
 # (profiles/qc_fft_sot_n20.md); sot_n20_ntt: the same workload on the NTT
 # backend, which scales the SOT encodes of NTT sizes (profiles/qc_ntt_sot_n20.md);
 # sot_n22_fft: 32 transforms of 251.8 MB per role plus gather and scatter
 # (profiles/qc_fft_sot_n22.md).
 NCU_TRAFFIC_PER_STEP = {
+    "ferret_b13:pprf": 0.1e6 + 178.7e6 + 0.4e6 + 180.1e6,
     "ferret_b13:lpn": 350.3e6 + 283.1e6 + 14.5e6,
     "sot_n20_fft:dual_lpn": 2 * (16.79e6 + 16 * 88.24e6 + 16.86e6),
     "sot_n20_ntt:dual_lpn": 2 * (509.60e6 + 1024.36e6 + 563.98e6 + 33.58e6),
