@@ -21,8 +21,8 @@
 // stream of its own beside the SOT branch; CUOT_BATCH_FORK_SIZES also puts
 // each transform size on its own stream (sizes that share per-size FFT
 // state, qc_lane, on one).  Measured on B200 (the 64-instance mix of
-// log2 n in [16, 22], 10 graph replays each): one chain 48.5 ms, Ferret
-// beside SOT 48.3 ms, sizes side by side 48.9 ms (86.1, 88.7 and 97.3 ms when
+// log2 n in [16, 22], 10 graph replays each): one chain 48.2 ms, Ferret
+// beside SOT 48.3 ms, sizes side by side 48.7 ms (86.1, 88.7 and 97.3 ms when
 // the encodes were FFTs, whose intermediates evicted each other from L2).  Every
 // part already fills the GPU.
 // The whole program is captured into a CUDA graph on the first run.
