@@ -24,7 +24,7 @@
 // reductions over the warp give the product (bit-serial ones by single
 // threads, level by level, took as long as the leaves).
 // Bound by the lookups' wavefronts: 32 x 4 per 32 leaves and SM, 145 us for
-// 2,507 trees of depth 12.  Measured there 675 -> 180 us (64 trees of depth 10: 45 -> 8).
+// 2,507 trees of depth 12.  Measured there 675 -> 178 us (64 trees of depth 10: 45 -> 8).
 #include <atomic>
 
 #include "ctx.cuh"
@@ -144,12 +144,14 @@ __global__ void __launch_bounds__(kChiThreads) chi_sum_kernel(const uint4 *__res
   if (Q > 1) {
     // Leaves are loaded four steps ahead, the first ones beside the table: one step
     // covers L2's latency and not that of memory, which few deep trees have nothing
-    // else to hide behind (16 trees of depth 20 4,993 us so, 2,877 four ahead).
-    constexpr int kAhead = 4;
+    // else to hide behind (16 trees of depth 20 4,978 us so, 2,673 four ahead).
+    // Chained calls' leaves fit L2: two (one tree of depth 16 162 us, four 184).
+    constexpr int kAhead = CHAINED ? 2 : 4;
     uint4 first[kAhead];
+    const uint4 *p = lv + j + kChiThreads * (Q - 1);
 #pragma unroll
     for (int i = 0; i < kAhead; i++)
-      if (i < Q) first[i] = __ldg(&lv[j + kChiThreads * (Q - 1 - i)]);
+      if (i < Q) first[i] = __ldg(p - kChiThreads * i);
     U128 u = s4;
 #pragma unroll 1
     for (int l = 0; l < 5; l++) u = gsqr(u);
@@ -170,18 +172,19 @@ __global__ void __launch_bounds__(kChiThreads) chi_sum_kernel(const uint4 *__res
     }
     __syncthreads();
     const char *mine = reinterpret_cast<const char *>(T + (lane & 7));
-    if (Q == 2) {
+    if (Q < kAhead) {  // Q = 2
       acc = xor4(to_u4(tmul(mine, first[0])), first[1]);
     } else {
       acc = first[0];
 #pragma unroll 1
-      for (int64_t q = Q - kAhead; q >= 0; q -= kAhead) {  // leaves q + 3 .. q
+      for (int64_t q = Q - kAhead; q >= 0; q -= kAhead) {  // leaves q + kAhead - 1 .. q
         uint4 x[kAhead];
 #pragma unroll
         for (int i = 0; i < kAhead; i++) x[i] = first[i];
+        p -= kChiThreads * kAhead;
         if (q) {
 #pragma unroll
-          for (int i = 0; i < kAhead; i++) first[i] = __ldg(&lv[j + kChiThreads * (q - 1 - i)]);
+          for (int i = 0; i < kAhead; i++) first[i] = __ldg(p - kChiThreads * i);
         }
         if (q != Q - kAhead) acc = xor4(to_u4(tmul(mine, acc)), x[0]);
 #pragma unroll
