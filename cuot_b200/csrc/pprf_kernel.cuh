@@ -297,14 +297,15 @@ __global__ void __launch_bounds__(kPprfThreads, 3) pprf_tree_kernel(PprfArgs a) 
 // 24.6 us, 300 33.5 / 32.9 / 39.2, 918 of depth 9 45 / 41 / 41, 1,280 of depth 13
 // 463 / 468 / 485, 1,500 of depth 10 102 / 99 / 90, 4,971 of depth 11 519 / 490 /
 // 458, 5,000 of depth 9 203 / 194 / 148 (one CTA per tree and launch before: 277).
-// Deep trees from one to 8 / 3 of the CTAs (four to eight per SM) go one by one to
-// CTAs as these get free: dealt out beforehand to groups they leave SMs waiting for
-// the fullest one (one by one / two groups per CTA: 592 trees of depth 13 209 / 260
-// us, 740 258 / 302, 1,036 359 / 396, 1,184 408 / 464), except where every SM has six
-// groups of 128 for six trees (888: 322 / 302).
+// Deep trees that two groups per CTA would share out badly (more than 1.2 times the
+// CTAs, but not two per CTA; more than 13 / 6, but not 8 / 3) go one by one to CTAs as
+// these get free: dealt out beforehand they leave SMs waiting for the fullest one
+// (one by one / dealt out: 500 trees of depth 13 209 / 208 us, 592 209 / 260, 740 258 /
+// 302, 888 322 / 302, 950 359 / 350, 1,036 359 / 396, 1,184 408 / 464, 1,280 468 / 465).
 inline int pprf_group_size(uint64_t trees, int h, uint64_t ctas) {
   if (trees <= ctas) return 256;
-  if (h >= 12 && 3 * trees <= 8 * ctas && (3 * trees <= 5 * ctas || trees > 2 * ctas)) return 256;
+  const bool uneven = (5 * trees > 6 * ctas && 3 * trees <= 5 * ctas) || (6 * trees > 13 * ctas && 3 * trees <= 8 * ctas);
+  if (h >= 12 && uneven) return 256;
   return trees <= 3 * ctas || h > 12 ? 128 : 64;
 }
 

@@ -31,10 +31,10 @@ def test_no_more_than_a_tree_per_cta(rule, h):
 
 @pytest.mark.parametrize("h", [12, 13, 14, 20])
 def test_deep_trees_of_a_few_waves(rule, h):
-    """Up to eight trees per SM: one by one, except where six groups of 128 hold an SM's six."""
-    for t in (445, 592, 740, 889, 1036, 1184):
+    """One by one where two groups per CTA would share them out badly."""
+    for t in (533, 592, 740, 963, 1036, 1184):
         assert rule(t, h) == 256, t
-    for t in (741, 888, 1185, 1332):
+    for t in (445, 532, 741, 888, 962, 1185, 1332):
         assert rule(t, h) == 128, t
 
 
