@@ -594,8 +594,8 @@ static int launch_sparse(const uint64_t *a_d, const uint64_t *pos_d, int weight,
   // position's words independently (2^17 with 2^17 positions 189 against 490).
   // Dense ones of few words by smaller CTAs (16 / 8 warps: 5,000 positions at 2^16
   // 24.7 / 20.5 us, 20,000 43.2 / 34.0; one CTA's 256 positions 8.9 / 11.5, and 20,000
-  // at 2^22 831 / 856).
-  if (weight > 2048 && n <= 1ull << 18) {
+  // at 2^22 831 / 856, 100,000 at 2^18 296 / 303).
+  if (weight > 2048 && weight <= 1 << 15 && n <= 1ull << 18) {
     if (n / 64 <= 512)
       return chained ? launch_sparse_as<1, 8, true>(a_d, pos_d, weight, n, out_d, r2, st)
                      : launch_sparse_as<1, 8, false>(a_d, pos_d, weight, n, out_d, r2, st);
