@@ -963,7 +963,7 @@ void launch_col_inv(const QcfTables *t, int ntr, cudaStream_t st, const double2 
 
 bool qcf_supported(int e) { return e >= 10 && e <= kQcfMaxE; }
 
-// Builds a size's tables on its own stream, outside any capture of the caller's.
+// Builds a size's tables outside any capture of the caller's.
 static int make_tables(cuot_ctx *ctx, int e, QcfTables **out);
 
 int qcf_get_tables(cuot_ctx *ctx, int e, QcfTables **out) {
@@ -1001,10 +1001,19 @@ static int make_tables(cuot_ctx *ctx, int e, QcfTables **out) {
     qcf_free(t);
     return fail(CUOT_ECUDA, "QC FFT stream / event creation failed");
   }
-  qcf_gen_roots<<<8, 256, 0, t->aux>>>(t->e1, t->T1);
-  qcf_gen_roots<<<8, 256, 0, t->aux>>>(t->e2, t->T2);
-  qcf_gen_fourstep<<<256, 256, 0, t->aux>>>(t->e1, t->e2, t->fs);
-  if (cudaStreamSynchronize(t->aux) != cudaSuccess || cudaGetLastError() != cudaSuccess) {
+  // On the default stream: once the tables' own stream has been used, every graph launch
+  // of a program that never needs it is slower (a batch of 12 small instances 529 ->
+  // 540 us).  Beside a capture that the default stream would break, on their own.
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  cudaStream_t st_gen = nullptr;
+  if (cudaStreamIsCapturing(cudaStreamLegacy, &cap) != cudaSuccess) {
+    cudaGetLastError();
+    st_gen = t->aux;
+  }
+  qcf_gen_roots<<<8, 256, 0, st_gen>>>(t->e1, t->T1);
+  qcf_gen_roots<<<8, 256, 0, st_gen>>>(t->e2, t->T2);
+  qcf_gen_fourstep<<<256, 256, 0, st_gen>>>(t->e1, t->e2, t->fs);
+  if (cudaStreamSynchronize(st_gen) != cudaSuccess || cudaGetLastError() != cudaSuccess) {
     qcf_free(t);
     return fail(CUOT_ECUDA, "QC FFT table generation failed");
   }
